@@ -1,6 +1,6 @@
 // cpa5i.cuh — the tcgen05 IND-CPA kernel specialised per parameter set: one
-// CTA of 256 threads per instance, with every width, count and offset a
-// compile-time constant.
+// CTA of 256 threads per instance (a resident CTA takes further ones), with
+// every width, count and offset a compile-time constant.
 //
 // Per instance:
 //   1. the packed inputs arrive by TMA bulk copies (cp.async.bulk) issued by
@@ -115,16 +115,23 @@ struct LayoutC {
   static constexpr int BM = H + C::L * kHankelBytes5;
   static constexpr int EXT = BM + C::L * BJ;
   static constexpr int ENG_END_OPS = EXT + C::L * 512;
-  static constexpr int ENG_BYTES = ENG_END_OPS;  // also holds the epilogue's 16-bit values (R x 512 bytes)
-  static_assert(S::R * 512 <= ENG_END_OPS, "epilogue values fit the operand region");
+  static constexpr int ENG_BYTES = ENG_END_OPS;
+  // the output ops' 16-bit values (R x 512 bytes), over the digit columns
+  // (the next instance's inputs are landing in H)
+  static constexpr int VALS = BM;
+  static_assert(HAS_CT || HAS_MV || S::R * 512 <= C::L * BJ, "epilogue values fit the digit columns");
+  // ciphertext and message, read until the end of an instance: two buffers of
+  // CTB bytes, so that the next instance's copies land beside them
   static constexpr int CTO = al16c(ENG + ENG_BYTES);
   static constexpr int MSG = HAS_CT ? al16c(CTO + NCT * CTS) : CTO;
-  static constexpr int SEC8 = HAS_B ? al16c(MSG + 32 + 16) : MSG;
+  static constexpr int CTB = (HAS_B ? al16c(MSG + 32 + 16) : MSG) - CTO;
+  static constexpr int SEC8 = CTO + 2 * CTB;
   static constexpr int OUT = OP == kKeygen ? al16c(SEC8 + C::L * 256) : SEC8;
   static constexpr int OUT_BYTES = OP == kEncrypt ? C::CT + 16
                                    : (OP == kKeygen ? C::L * C::POLYCOMP + C::INDCPA_SK + 16 : 0);
-  static constexpr int BAR = al16c(OUT + OUT_BYTES);  // mbarriers in, mma; TMEM base
-  static constexpr int TOTAL = BAR + 32;
+  // mbarriers in, mma, clc; TMEM base; the next instance; two CLC responses
+  static constexpr int BAR = al16c(OUT + OUT_BYTES);
+  static constexpr int TOTAL = BAR + 64;
   static constexpr int IN_BYTES = (HAS_AS ? C::GM + C::GS : 0) + (HAS_B ? C::L * C::POLYCOMP + 32 : 0) +
                                   (HAS_CT ? C::CT : 0) + (HAS_SK ? C::INDCPA_SK : 0) + (HAS_MV ? MV_A + MV_S : 0);
   static_assert(!HAS_AS || B + (HAS_B ? C::L * C::POLYCOMP + 16 : 0) <= BM, "streams fit inside H");
@@ -235,62 +242,124 @@ __device__ __forceinline__ void stage_digits32(const uint8_t *sm, int src, uint3
   }
 }
 
-// One instance (CTA of kI5Threads threads; sm: its dynamic shared memory).
+// Cluster launch control: asks for a CTA of this grid that has not been
+// launched yet, to run its work here instead.  The 16-byte answer lands at
+// resp and counts on mbar.
+__device__ __forceinline__ void clc_try_cancel(uint32_t resp, uint32_t mbar) {
+  asm volatile(
+      "clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(resp),
+      "r"(mbar)
+      : "memory");
+}
+// The answer: the taken CTA's blockIdx.x, or ~0u when none was left to take.
+__device__ __forceinline__ uint32_t clc_answer(uint32_t resp) {
+  uint32_t x;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b128 h;\n\t"
+      "ld.shared.b128 h, [%1];\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, h;\n\t"
+      "mov.u32 %0, 0xffffffff;\n\t"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %0, h;\n\t}\n"
+      : "=r"(x)
+      : "r"(resp)
+      : "memory");
+  return x;
+}
+
+// The input copies of instance inst into ciphertext / message buffer cb
+// (0 or CTB), counted on mbar (one thread).  kDecryptK: ciphertexts
+// inst * NCT .. of the one key.
 template <int OP, int SET>
-__device__ __forceinline__ void cpa5i_body(const CpaArgs &a, const unsigned inst, uint8_t *sm) {
+__device__ __forceinline__ void cpa5i_load(const CpaArgs &a, const unsigned inst, uint32_t d, uint32_t cb,
+                                           uint32_t mbar) {
+  using C = SetC<SET>;
+  using LO = LayoutC<OP, SET>;
+  constexpr bool DECK = OP == kDecryptK;
+  const size_t inst0 = DECK ? (size_t)inst * LO::NCT : (size_t)inst;
+  const int nvalid = DECK ? min(LO::NCT, a.n - (int)inst0) : 1;
+  const uint32_t in_bytes = DECK ? (uint32_t)(C::INDCPA_SK + nvalid * C::CT) : (uint32_t)LO::IN_BYTES;
+  mbar_expect_tx(mbar, in_bytes + (a.stall_inputs ? 16 : 0));
+  if (LO::HAS_AS) {
+    bulk_g2s(d + LO::A, a.a_stream + (a.key_shared ? 0 : (size_t)inst * C::GM), C::GM, mbar);
+    bulk_g2s(d + LO::SS, a.s_stream + (size_t)inst * C::GS, C::GS, mbar);
+  }
+  if (LO::HAS_B) {
+    bulk_g2s(d + LO::B, a.pk + (size_t)inst * a.pk_stride + a.pk_off, C::L * C::POLYCOMP, mbar);
+    bulk_g2s(d + LO::MSG + cb, a.msg + (size_t)inst * a.msg_stride, 32, mbar);
+  }
+  if (DECK) {
+    for (int r = 0; r < nvalid; r++)
+      bulk_g2s(d + LO::CTO + cb + r * LO::CTS, a.ct + (inst0 + r) * C::CT, C::CT, mbar);
+  } else if (LO::HAS_CT) {
+    bulk_g2s(d + LO::CTO + cb, a.ct + (size_t)inst * C::CT, C::CT, mbar);
+  }
+  if (LO::HAS_SK)
+    bulk_g2s(d + LO::SKO, a.sk + ((a.key_shared || DECK) ? 0 : (size_t)inst * C::SK), C::INDCPA_SK, mbar);
+  if (LO::HAS_MV) {
+    bulk_g2s(d + LO::A, reinterpret_cast<const uint8_t *>(a.mv_A) + (size_t)inst * LO::MV_A, LO::MV_A, mbar);
+    bulk_g2s(d + LO::SS, reinterpret_cast<const uint8_t *>(a.mv_s) + (size_t)inst * LO::MV_S, LO::MV_S, mbar);
+  }
+}
+
+// The instances of a launch, from the CTA of kI5Threads threads that runs
+// blockIdx.x (sm: its dynamic shared memory).  at(gi) names the arguments and
+// the instance of CTA gi: a pair-like struct {const CpaArgs &a; unsigned inst}.
+//
+// The grid has one CTA per instance, but a resident CTA goes on to the next
+// one that has not started (cluster launch control) instead of exiting: tensor
+// memory and barriers are set up once, and the next instance's input copies
+// run beside the epilogue of this one.  Without that, an empty instance (no
+// staging, no MMAs) took 0.207 of the decryption's 0.273 ms at 65536; with it
+// 0.090 of 0.246 (re-encryption 0.353 -> 0.342), and what bounds the kernel is
+// its MMAs (0.217 ms for the decryption's 24 alone).
+template <int OP, int SET, class AT>
+__device__ __forceinline__ void cpa5i_run(const AT &at, uint8_t *sm) {
   using C = SetC<SET>;
   using S = ShapeC<OP, SET>;
   using LO = LayoutC<OP, SET>;
   constexpr int L = C::L, NU = S::NU, NT = kI5Threads;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const uint32_t mbar_in = smem_u32(sm + LO::BAR), mbar_mma = mbar_in + 8;
-  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(sm + LO::BAR + 16);
-  // kDecryptK: this CTA's ciphertexts inst0 .. inst0 + nvalid - 1 (one key)
+  const uint32_t mbar_in = smem_u32(sm + LO::BAR), mbar_mma = mbar_in + 8, mbar_clc = mbar_in + 16;
+  const uint32_t clc_resp = mbar_in + 32;
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(sm + LO::BAR + 24);
+  volatile uint32_t *next_slot = reinterpret_cast<volatile uint32_t *>(sm + LO::BAR + 28);
   constexpr bool DECK = OP == kDecryptK, IS_DEC = OP == kDecrypt || DECK;
-  const size_t inst0 = DECK ? (size_t)inst * LO::NCT : (size_t)inst;
-  const int nvalid = DECK ? min(LO::NCT, a.n - (int)inst0) : 1;
 
-  // 0. tensor memory, barriers, and the input copies (one thread)
-  if (warp == 0) tmem_alloc(smem_u32(tmem_slot), S::TMEM_COLS);
-  if (tid == 0) {
+  // 0. tensor memory, barriers, and the first input copies (one thread)
+  if (threadIdx.x < 32) tmem_alloc(smem_u32(tmem_slot), S::TMEM_COLS);
+  if (threadIdx.x == 0) {
     mbar_init(mbar_in, 1);
     mbar_init(mbar_mma, 1);
+    mbar_init(mbar_clc, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    const uint32_t d = smem_u32(sm);
-    const uint32_t in_bytes = DECK ? (uint32_t)(C::INDCPA_SK + nvalid * C::CT) : (uint32_t)LO::IN_BYTES;
-    mbar_expect_tx(mbar_in, in_bytes + (a.stall_inputs ? 16 : 0));
-    if (LO::HAS_AS) {
-      bulk_g2s(d + LO::A, a.a_stream + (a.key_shared ? 0 : (size_t)inst * C::GM), C::GM, mbar_in);
-      bulk_g2s(d + LO::SS, a.s_stream + (size_t)inst * C::GS, C::GS, mbar_in);
-    }
-    if (LO::HAS_B) {
-      bulk_g2s(d + LO::B, a.pk + (size_t)inst * a.pk_stride + a.pk_off, C::L * C::POLYCOMP, mbar_in);
-      bulk_g2s(d + LO::MSG, a.msg + (size_t)inst * a.msg_stride, 32, mbar_in);
-    }
-    if (DECK) {
-      for (int r = 0; r < nvalid; r++) bulk_g2s(d + LO::CTO + r * LO::CTS, a.ct + (inst0 + r) * C::CT, C::CT, mbar_in);
-    } else if (LO::HAS_CT) {
-      bulk_g2s(d + LO::CTO, a.ct + (size_t)inst * C::CT, C::CT, mbar_in);
-    }
-    if (LO::HAS_SK)
-      bulk_g2s(d + LO::SKO, a.sk + ((a.key_shared || DECK) ? 0 : (size_t)inst * C::SK), C::INDCPA_SK, mbar_in);
-    if (LO::HAS_MV) {
-      bulk_g2s(d + LO::A, reinterpret_cast<const uint8_t *>(a.mv_A) + (size_t)inst * LO::MV_A, LO::MV_A, mbar_in);
-      bulk_g2s(d + LO::SS, reinterpret_cast<const uint8_t *>(a.mv_s) + (size_t)inst * LO::MV_S, LO::MV_S, mbar_in);
-    }
+    const auto w = at(blockIdx.x);
+    cpa5i_load<OP, SET>(w.a, w.inst, smem_u32(sm), 0, mbar_in);
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *reinterpret_cast<volatile uint32_t *>(tmem_slot);
-  bool ready = true;
-  if (warp == 0) ready = mbar_wait_bounded(mbar_in, 0);
-  ready = __syncthreads_and(ready) != 0;
-
   uint32_t *sec8w = reinterpret_cast<uint32_t *>(sm + LO::SEC8);
   uint8_t *H = sm + LO::H, *Bm = sm + LO::BM;
   const uint32_t ext32 = smem_u32(sm + LO::EXT);
-  bool ok = true, done = false;
+  unsigned gi = blockIdx.x;
+  for (uint32_t it = 0;; it++) {
+  // per-thread values are made afresh for every instance (not kept across the
+  // loop in registers, which bound the CTAs per SM)
+  int tid = threadIdx.x;
+  asm volatile("" : "+r"(tid));
+  const int warp = tid >> 5, lane = tid & 31;
+  const uint32_t par = it & 1u, cbuf = par ? (uint32_t)LO::CTB : 0u;
+  const auto here = at(gi);
+  const CpaArgs &a = here.a;
+  const unsigned inst = here.inst;
+  const size_t inst0 = DECK ? (size_t)inst * LO::NCT : (size_t)inst;
+  const int nvalid = DECK ? min(LO::NCT, a.n - (int)inst0) : 1;
+  if (tid == 0) {  // ask for the next instance; answer buffer par was read before this instance's predecessor's barriers
+    mbar_expect_tx(mbar_clc, 16);
+    clc_try_cancel(clc_resp + 16 * par, mbar_clc);
+  }
+  bool ready = mbar_wait_bounded(mbar_in, par);
+  bool ok = true;
   if (ready) {
     // 1. secrets, straight into s_ext (s_ext[d] = -s[d + 1] for d < 255,
     // s[d - 255] for 255 <= d <= 510, 0 at 511; 128 words per j).  Warp
@@ -407,7 +476,7 @@ __device__ __forceinline__ void cpa5i_body(const CpaArgs &a, const unsigned inst
 #pragma unroll
         for (int j = 0; j < L; j++) {
           if (warp < nvalid) {
-            item(std::integral_constant<int, S::WB>{}, LO::CTO + warp * LO::CTS + 32 * j * S::WB, warp * S::DB, j);
+            item(std::integral_constant<int, S::WB>{}, (int)cbuf + LO::CTO + warp * LO::CTS + 32 * j * S::WB, warp * S::DB, j);
           } else {
 #pragma unroll
             for (int d0 = 0; d0 < S::DB; d0++) {
@@ -418,7 +487,7 @@ __device__ __forceinline__ void cpa5i_body(const CpaArgs &a, const unsigned inst
         }
       }
     } else if constexpr (S::R == 1) {
-      if (warp < L) item(std::integral_constant<int, S::WB>{}, LO::CTO + 32 * warp * S::WB, 0, warp);
+      if (warp < L) item(std::integral_constant<int, S::WB>{}, (int)cbuf + LO::CTO + 32 * warp * S::WB, 0, warp);
     } else {
       // public matrix A (RA x L polynomials), then b (encryption, re-encryption):
       // four polynomials per warp, eight lanes each
@@ -443,8 +512,17 @@ __device__ __forceinline__ void cpa5i_body(const CpaArgs &a, const unsigned inst
       }
     }
   }
-  __syncthreads();  // s_ext complete, and the streams inside H read, before H is written
-  if (ready) stage_hankel_ct<L, NT, kHankelCores5>(smem_u32(H), ext32, tid);
+  // s_ext complete, and the streams inside H read, before H is written
+  ready = __syncthreads_and(ready) != 0;
+  if (!ready) {  // the input copies did not complete in time: report, leave
+    if (tid == 0 && a.err) atomicOr(a.err, 2);
+    if (warp == 0) {
+      mbar_wait_bounded(mbar_in, par);
+      mbar_wait_bounded(mbar_clc, par);
+    }
+    break;
+  }
+  stage_hankel_ct<L, NT, kHankelCores5>(smem_u32(H), ext32, tid);
   fence_async_smem();  // generic-proxy writes -> visible to the tensor core
   ok = __syncthreads_and(ok) != 0;
   if (!ok && tid == 0 && a.err) atomicOr(a.err, 1);
@@ -456,7 +534,8 @@ __device__ __forceinline__ void cpa5i_body(const CpaArgs &a, const unsigned inst
   // r, so window r + 4 gives (top, step r + 4 | bottom, step r) in region 0
   // and window r gives (-bottom, step r + 4 | top, step r) in region 1:
   // 8 MMAs per j, top = region0[0] + region1[1], bottom = region0[1] - region1[0].
-  if (ready && tid == 0) {
+  if (tid == 0) {
+    tc_fence_after();  // the previous instance's accumulator loads come before these MMAs
     constexpr uint32_t idesc = umma_idesc_e4m3(NU);
     const uint64_t ad0 = umma_desc(smem_u32(H), 256, 128);
     const uint32_t b0 = smem_u32(Bm);
@@ -472,12 +551,36 @@ __device__ __forceinline__ void cpa5i_body(const CpaArgs &a, const unsigned inst
     }
     umma_commit(mbar_mma);
   }
-  // 4. accumulators (one warp polls the MMA barrier, the others wait in the barrier)
-  if (ready) {
-    bool fin = true;
-    if (warp == 0) fin = mbar_wait_bounded(mbar_mma, 0);
-    done = __syncthreads_and(fin) != 0;
+  // 4. accumulators: one warp polls the MMA barrier and the CLC answer, the
+  // others wait in the CTA barrier.  The MMAs have read H and the other
+  // ciphertext buffer was last read before this instance's barriers, so the
+  // next instance's copies start here, beside the epilogue.
+  bool done = true;
+  if (warp == 0) {
+    done = mbar_wait_bounded(mbar_mma, par) && mbar_wait_bounded(mbar_clc, par);
+    done = __all_sync(0xffffffffu, done) != 0;
+    if (tid == 0) {
+      const uint32_t nx = done ? clc_answer(clc_resp + 16 * par) : ~0u;
+      *next_slot = nx;
+      if (nx != ~0u) {
+        const auto wn = at(nx);
+        cpa5i_load<OP, SET>(wn.a, wn.inst, smem_u32(sm), (uint32_t)LO::CTB - cbuf, mbar_in);
+      }
+      if (OP == kReenc && done) a.fail[inst] = 0;  // set below, after the barrier, by a warp that finds a difference
+    }
   }
+  done = __syncthreads_and(done) != 0;
+  if (!done) {
+    // the tensor core or the CLC answer did not come in time: report, and
+    // give what is still in flight a second bounded wait before releasing
+    if (tid == 0 && a.err) atomicOr(a.err, 2);
+    if (warp == 0) {
+      mbar_wait_bounded(mbar_mma, par);
+      mbar_wait_bounded(mbar_clc, par);
+    }
+    break;
+  }
+  const uint32_t next = *next_slot;
   tc_fence_after();
   // warp w reads TMEM lanes 32 (w % 4) .. +31 for coefficient
   // k = 128 hsel + 32 q4 + lane (hsel = w / 4): every digit column of k,
@@ -486,7 +589,7 @@ __device__ __forceinline__ void cpa5i_body(const CpaArgs &a, const unsigned inst
   const int k = 128 * hsel + 32 * q4 + lane;
   constexpr int G8 = 8 * LO::G;
   float xacc[G8];  // digit column c of coefficient k, times 2^-9 (exact)
-  if (done) {
+  {
     const uint32_t t0 = tmem + ((uint32_t)(32 * q4) << 16);
     uint32_t f[G8], g[G8];
     if constexpr (G8 == 8) {
@@ -506,9 +609,9 @@ __device__ __forceinline__ void cpa5i_body(const CpaArgs &a, const unsigned inst
     if constexpr (OP == kEncrypt || OP == kKeygen) {
       // coefficient k of every output polynomial, rounded (b, b') or encoded
       // with the message bit (c_m), as 16-bit values for the packing pass;
-      // the MMAs are done, so the operand region is free
+      // the MMAs are done, so the digit columns are free
       constexpr uint32_t qm = (1u << C::EQ) - 1u, pm = (1u << C::EP) - 1u;
-      uint16_t *vals = reinterpret_cast<uint16_t *>(sm + LO::ENG);
+      uint16_t *vals = reinterpret_cast<uint16_t *>(sm + LO::VALS);
 #pragma unroll
       for (int p = 0; p < S::R; p++) {
         uint32_t v = 0, off = 0;
@@ -523,24 +626,14 @@ __device__ __forceinline__ void cpa5i_body(const CpaArgs &a, const unsigned inst
         if (p < L) {
           vals[256 * p + k] = (uint16_t)(((v + C::H1) & qm) >> (C::EQ - C::EP));
         } else {
-          const uint32_t mk = (sm[LO::MSG + (k >> 3)] >> (k & 7)) & 1u;
+          const uint32_t mk = (sm[LO::MSG + cbuf + (k >> 3)] >> (k & 7)) & 1u;
           vals[256 * p + k] = (uint16_t)(((v + C::H1 - (mk << (C::EP - 1))) & pm) >> (C::EP - C::ET));
         }
       }
     }
-  } else {
-    // an input copy or the tensor core did not complete in time: report, and
-    // give what is still in flight a second bounded wait before releasing
-    if (tid == 0 && a.err) atomicOr(a.err, 2);
-    if (warp == 0) {
-      if (!ready) mbar_wait_bounded(mbar_in, 0);
-      else mbar_wait_bounded(mbar_mma, 0);
-    }
   }
-  tc_fence_before();
-  __syncthreads();
-  if (warp == 0) tmem_dealloc(tmem, S::TMEM_COLS);
-  if (!done) return;
+  tc_fence_before();  // the loads above come before the next instance's MMAs (its barriers lie between)
+  if constexpr (OP == kEncrypt || OP == kKeygen) __syncthreads();  // the 16-bit values are complete
 
   // 5. epilogues
   constexpr uint32_t qmask = (1u << C::EQ) - 1u, pmask = (1u << C::EP) - 1u;
@@ -569,7 +662,7 @@ __device__ __forceinline__ void cpa5i_body(const CpaArgs &a, const unsigned inst
     // m'_k = ((v_k + h2 - (c_m,k << (ep-et))) mod p) >> (ep-1): one bit per
     // thread, gathered into bytes by a ballot per warp
     const uint32_t v = combine1(0, S::DB);
-    const uint32_t cm = field(LO::CTO + L * C::POLYCOMP, k * C::ET, C::ET);
+    const uint32_t cm = field((int)cbuf + LO::CTO + L * C::POLYCOMP, k * C::ET, C::ET);
     const uint32_t t = (v + C::H2 - (cm << (C::EP - C::ET))) & pmask;
     const uint32_t bits = __ballot_sync(0xffffffffu, ((t >> (C::EP - 1)) & 1u) != 0u);
     uint8_t *mo = a.m_out + (size_t)inst * a.m_out_stride;
@@ -581,7 +674,7 @@ __device__ __forceinline__ void cpa5i_body(const CpaArgs &a, const unsigned inst
     for (int r = 0; r < S::R; r++) {
       if (r >= nvalid) break;
       const uint32_t v = combine1(r * S::DB, S::DB);
-      const uint32_t cm = field(LO::CTO + r * LO::CTS + L * C::POLYCOMP, k * C::ET, C::ET);
+      const uint32_t cm = field((int)cbuf + LO::CTO + r * LO::CTS + L * C::POLYCOMP, k * C::ET, C::ET);
       const uint32_t t = (v + C::H2 - (cm << (C::EP - C::ET))) & pmask;
       const uint32_t bits = __ballot_sync(0xffffffffu, ((t >> (C::EP - 1)) & 1u) != 0u);
       uint8_t *mo = a.m_out + (inst0 + r) * a.m_out_stride;
@@ -590,21 +683,20 @@ __device__ __forceinline__ void cpa5i_body(const CpaArgs &a, const unsigned inst
     }
   } else if constexpr (OP == kReenc) {
     // round coefficient k of b' and encode that of v', compare with the ciphertext
-    const uint32_t mk = (sm[LO::MSG + (k >> 3)] >> (k & 7)) & 1u;
+    const uint32_t mk = (sm[LO::MSG + cbuf + (k >> 3)] >> (k & 7)) & 1u;
     uint32_t diff = 0;
 #pragma unroll
     for (int p = 0; p < S::R; p++) {
       const uint32_t v = combine1(S::col_base(p), S::digits(p));
       if (p < L) {
         const uint32_t w = ((v + C::H1) & qmask) >> (C::EQ - C::EP);
-        diff |= w ^ field(LO::CTO + p * C::POLYCOMP, k * C::EP, C::EP);
+        diff |= w ^ field((int)cbuf + LO::CTO + p * C::POLYCOMP, k * C::EP, C::EP);
       } else {
         const uint32_t w = ((v + C::H1 - (mk << (C::EP - 1))) & pmask) >> (C::EP - C::ET);
-        diff |= w ^ field(LO::CTO + L * C::POLYCOMP, k * C::ET, C::ET);
+        diff |= w ^ field((int)cbuf + LO::CTO + L * C::POLYCOMP, k * C::ET, C::ET);
       }
     }
-    const int any = __syncthreads_or(diff != 0u);
-    if (tid == 0) a.fail[inst] = (uint8_t)(any != 0);
+    if (__any_sync(0xffffffffu, diff != 0u) && lane == 0) a.fail[inst] = 1;
   } else if constexpr (OP == kMatvec) {
     // coefficient k of every output polynomial, mod 2^eq
     const uint32_t m = (1u << a.mv_eq) - 1u;
@@ -613,7 +705,7 @@ __device__ __forceinline__ void cpa5i_body(const CpaArgs &a, const unsigned inst
     for (int p = 0; p < L; p++) o[256 * p] = (uint16_t)(combine1(S::col_base(p), S::DA) & m);
   } else if (OP == kEncrypt) {
     // pack the 16-bit values eight at a time: b' at EP bits, c_m at ET bits
-    const uint16_t *vals = reinterpret_cast<const uint16_t *>(sm + LO::ENG);
+    const uint16_t *vals = reinterpret_cast<const uint16_t *>(sm + LO::VALS);
     for (int idx = tid; idx < S::R * 32; idx += NT) {
       const int p = idx >> 5, grp = idx & 31;
       const uint4 q = *reinterpret_cast<const uint4 *>(vals + 256 * p + 8 * grp);
@@ -626,7 +718,7 @@ __device__ __forceinline__ void cpa5i_body(const CpaArgs &a, const unsigned inst
   } else if (OP == kKeygen) {
     constexpr int bbytes = L * C::POLYCOMP;
     uint8_t *outb = sm + LO::OUT;
-    const uint16_t *vals = reinterpret_cast<const uint16_t *>(sm + LO::ENG);
+    const uint16_t *vals = reinterpret_cast<const uint16_t *>(sm + LO::VALS);
     for (int idx = tid; idx < L * 32; idx += NT) {
       const int p = idx >> 5, grp = idx & 31;
       const uint4 q = *reinterpret_cast<const uint4 *>(vals + 256 * p + 8 * grp);
@@ -646,45 +738,47 @@ __device__ __forceinline__ void cpa5i_body(const CpaArgs &a, const unsigned inst
     __syncthreads();
     uint8_t *pko = a.pk_out + (size_t)inst * C::PK;
     uint8_t *sko = a.sk_out + (size_t)inst * a.sk_stride;
-    for (int i = tid; i < bbytes; i += NT) {
-      pko[i] = outb[i];
-      sko[C::INDCPA_SK + i] = outb[i];
-    }
     if (tid < 32) sko[C::INDCPA_SK + bbytes + tid] = pko[bbytes + tid];  // seed_A
-    for (int i = tid; i < C::INDCPA_SK; i += NT) sko[i] = outb[bbytes + i];
+    copy16(pko, outb, bbytes);
+    copy16(sko + C::INDCPA_SK, outb, bbytes);
+    copy16(sko, outb + bbytes, C::INDCPA_SK);
   }
+  if (next == ~0u) break;
+  gi = next;
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (threadIdx.x < 32) tmem_dealloc(tmem, S::TMEM_COLS);
 }
+
+// CTAs per SM that shared memory (228 KB, 1 KB of it per CTA reserved) and
+// tensor memory (512 columns) allow, 6 at most (40 registers, which every
+// kernel comes close to by itself; decryption needs 32 and gets its 8 CTAs):
+// the speed comes from the CTAs that overlap each other's phases.
+template <int OP, int SET>
+constexpr int min_ctas() {
+  constexpr int by_smem = (228 * 1024) / (LayoutC<OP, SET>::TOTAL + 1024), by_tmem = 512 / ShapeC<OP, SET>::TMEM_COLS;
+  constexpr int m = by_smem < by_tmem ? by_smem : by_tmem;
+  return m < 6 ? m : 6;
+}
+
+// The arguments and the instance that CTA gi of a launch stands for.
+struct CpaAt {
+  const CpaArgs &a;
+  unsigned inst;
+};
 
 template <int OP, int SET>
-__global__ void __launch_bounds__(kI5Threads, 2) k_cpa5i(CpaArgs a) {
+__global__ void __launch_bounds__(kI5Threads, min_ctas<OP, SET>()) k_cpa5i(const __grid_constant__ CpaArgs a) {
   extern __shared__ __align__(16) uint8_t sm[];
-  cpa5i_body<OP, SET>(a, blockIdx.x, sm);
-}
-
-// Mixed launch: CTA gi runs instance gi of the group table R (one CTA per
-// instance over all groups, whatever their parameter sets).
-template <int OP>
-__global__ void __launch_bounds__(kI5Threads, 2) k_cpa5m(const __grid_constant__ MixRef R) {
-  extern __shared__ __align__(16) uint8_t sm[];
-  const int gi = blockIdx.x;
-  const int g = find_group(R, gi);
-  const CpaArgs &a = group_args(R, g);
-  const unsigned inst = (unsigned)(gi - group_first(R, g));
-  switch (a.P.set) {
-    case 0: cpa5i_body<OP, 0>(a, inst, sm); break;
-    case 1: cpa5i_body<OP, 1>(a, inst, sm); break;
-    case 2: cpa5i_body<OP, 2>(a, inst, sm); break;
-    case 3: cpa5i_body<OP, 3>(a, inst, sm); break;
-    case 4: cpa5i_body<OP, 4>(a, inst, sm); break;
-    case 5: cpa5i_body<OP, 5>(a, inst, sm); break;
-  }
+  cpa5i_run<OP, SET>([&](unsigned gi) { return CpaAt{a, gi}; }, sm);
 }
 
 // Mixed launch whose groups all have parameter set SET (the per-set launches
 // of a mixed pass): the group table travels as a kernel parameter (constant
 // bank), so a CTA finds its group and reads its arguments without a global
 // round trip; then the same body as k_cpa5i, with the same registers and
-// occupancy.  CTA gi runs instance gi of the table.
+// occupancy.  CTA gi stands for instance gi of the table.
 struct MixParam {
   int ngroups, total;
   int first[kMaxGroups + 1];
@@ -693,30 +787,20 @@ struct MixParam {
 static_assert(sizeof(MixParam) < 32000, "the group table fits the kernel-parameter space");
 
 template <int OP, int SET>
-__global__ void __launch_bounds__(kI5Threads, 2) k_cpa5ms(const __grid_constant__ MixParam T) {
+__global__ void __launch_bounds__(kI5Threads, min_ctas<OP, SET>()) k_cpa5ms(const __grid_constant__ MixParam T) {
   extern __shared__ __align__(16) uint8_t sm[];
-  const int gi = blockIdx.x;
-  int lo = 0, hi = T.ngroups - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (gi >= T.first[mid]) lo = mid;
-    else hi = mid - 1;
-  }
-  cpa5i_body<OP, SET>(T.g[lo], (unsigned)(gi - T.first[lo]), sm);
-}
-
-template <int OP>
-inline void layout5_of(int set, int &total, int &cols) {
-  switch (set) {
-#define TMVP_L5(S)                                 \
-  case S:                                          \
-    total = LayoutC<OP, S>::TOTAL;                 \
-    cols = ShapeC<OP, S>::TMEM_COLS;               \
-    break;
-    TMVP_L5(0) TMVP_L5(1) TMVP_L5(2) TMVP_L5(3) TMVP_L5(4) TMVP_L5(5)
-#undef TMVP_L5
-    default: total = 0; cols = 32;
-  }
+  cpa5i_run<OP, SET>(
+      [&](unsigned u) {
+        const int gi = (int)u;
+        int lo = 0, hi = T.ngroups - 1;
+        while (lo < hi) {
+          const int mid = (lo + hi + 1) >> 1;
+          if (gi >= T.first[mid]) lo = mid;
+          else hi = mid - 1;
+        }
+        return CpaAt{T.g[lo], (unsigned)(gi - T.first[lo])};
+      },
+      sm);
 }
 
 // Pads `smem` until at most 512 / cols CTAs of fn fit on an SM, so that every
@@ -761,45 +845,20 @@ inline int launch_cpa5ms(const CpaArgs *groups, int ng, cudaStream_t s) {
   return (int)cudaGetLastError();
 }
 
+// Groups of one parameter set (a mixed pass launches each set's groups by themselves).
 template <int OP>
-inline int launch_cpa5m(const CpaArgs *groups, int ng, const MixTable *dev_tab, cudaStream_t s) {
-  MixRef R{};
-  R.ngroups = ng;
-  R.total = 0;
-  int smem = 0, cols = 32;
-  for (int g = 0; g < ng; g++) {
-    R.total += groups[g].n;
-    int t, c;
-    layout5_of<OP>(groups[g].P.set, t, c);
-    smem = std::max(smem, t);
-    cols = std::max(cols, c);
+inline int launch_cpa5m(const CpaArgs *groups, int ng, cudaStream_t s) {
+  for (int g = 1; g < ng; g++)
+    if (groups[g].P.set != groups[0].P.set) return (int)cudaErrorInvalidValue;
+  switch (groups[0].P.set) {
+    case 0: return launch_cpa5ms<OP, 0>(groups, ng, s);
+    case 1: return launch_cpa5ms<OP, 1>(groups, ng, s);
+    case 2: return launch_cpa5ms<OP, 2>(groups, ng, s);
+    case 3: return launch_cpa5ms<OP, 3>(groups, ng, s);
+    case 4: return launch_cpa5ms<OP, 4>(groups, ng, s);
+    case 5: return launch_cpa5ms<OP, 5>(groups, ng, s);
   }
-  if (R.total <= 0) return 0;
-  if (ng == 1) {
-    R.one = groups[0];
-  } else {
-    if (!dev_tab) return (int)cudaErrorInvalidValue;
-    R.tab = dev_tab;
-  }
-  bool one_set = true;
-  for (int g = 1; g < ng; g++) one_set = one_set && groups[g].P.set == groups[0].P.set;
-  if (one_set) {
-    switch (groups[0].P.set) {
-      case 0: return launch_cpa5ms<OP, 0>(groups, ng, s);
-      case 1: return launch_cpa5ms<OP, 1>(groups, ng, s);
-      case 2: return launch_cpa5ms<OP, 2>(groups, ng, s);
-      case 3: return launch_cpa5ms<OP, 3>(groups, ng, s);
-      case 4: return launch_cpa5ms<OP, 4>(groups, ng, s);
-      case 5: return launch_cpa5ms<OP, 5>(groups, ng, s);
-    }
-  }
-  auto fn = k_cpa5m<OP>;
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-  if (e != cudaSuccess) return (int)e;
-  int rc = cap_tmem_residency(fn, smem, cols);
-  if (rc) return rc;
-  fn<<<R.total, kI5Threads, smem, s>>>(R);
-  return (int)cudaGetLastError();
+  return (int)cudaErrorInvalidValue;
 }
 
 template <int OP, int SET>

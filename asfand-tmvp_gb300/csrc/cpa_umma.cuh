@@ -137,6 +137,7 @@ __device__ __forceinline__ bool mbar_try_wait_sleep(uint32_t mbar, uint32_t pari
 // Bounded wait for phase `parity` of an mbarrier: sleeps in 20 us slices and
 // gives up after about two seconds (or 2^22 polls), returning false.
 __device__ __forceinline__ bool mbar_wait_bounded(uint32_t mbar, uint32_t parity) {
+  if (mbar_try_wait_sleep(mbar, parity, 20000u)) return true;
   const uint64_t t0 = global_ns();
   for (uint32_t it = 0; it < (1u << 22); it++) {
     if (mbar_try_wait_sleep(mbar, parity, 20000u)) return true;
