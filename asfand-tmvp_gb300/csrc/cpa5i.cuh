@@ -8,11 +8,12 @@
 //   2. secrets (CBD or unpacked) straight into s_ext, radix-16 digit columns
 //      (r16_digits, raw e4m3 bytes worth digit * 2^-9) with K reversed, then
 //      the Hankel core matrices (cpa_umma.cuh);
-//   3. one thread issues the 8 l tcgen05.mma (M = 128, N = 16 / 32, K = 32;
-//      each window of the Hankel sequence serves both M halves through the
+//   3. one thread issues the 4 l tcgen05.mma (M = 128, N = 16 .. 64, K = 32;
+//      each even tile of the Hankel sequence serves four K steps through the
 //      negacyclic wrap) into tensor memory and commits them to an mbarrier;
 //   4. accumulators -> registers (tcgen05.ld: every digit column of one
-//      coefficient per thread) -> the compare / decode / output epilogue
+//      coefficient per thread), the odd K steps' sums through shared memory to
+//      the warp of their coefficients -> the compare / decode / output epilogue
 //      (encryption and key generation: rounded 16-bit values, then packed
 //      eight coefficients at a time).
 // Same results as the runtime-shaped kernels (cpa_tc_kernel.cuh,
@@ -54,9 +55,15 @@ struct ShapeC {
   static constexpr int DA = r16_digits(WA), DB = r16_digits(WB);
   static constexpr int NCOLS = RA * DA + (R - RA) * DB;
   static_assert(NCOLS <= 16, "at most two 8-column groups per K step");
-  static constexpr int G = NCOLS <= 8 ? 1 : 2;     // 8-column groups per K step
-  static constexpr int NU = 16 * G;                // N of every MMA (two K steps side by side)
-  static constexpr int TMEM_COLS = 32 * G;         // two accumulator regions of NU columns
+  static constexpr int NC4 = (NCOLS + 3) & ~3;     // column slots of one K step
+  static constexpr int PG = NC4 / 4;               // 8-column groups of two K steps
+  static constexpr int NU = 4 * NC4;               // N of every MMA (four K steps' columns)
+  static_assert(NU % 16 == 0, "an N that M = 128 admits");
+  static constexpr int TMEM_COLS = NU <= 32 ? 32 : 64;
+  // Largest |secret| (CBD: mu / 2; sk and matvec secrets: what small4 admits)
+  // and the K rows that one accumulator sums, for combine()
+  static constexpr int SMAX = (OP == kMatvec || OP == kDecrypt || OP == kDecryptK) ? 7 : C::MU / 2;
+  static constexpr int ROWS = 128 * L;
   static constexpr int col_base(int p) { return p < RA ? p * DA : RA * DA + (p - RA) * DB; }
   static constexpr int digits(int p) { return p < RA ? DA : DB; }
 };
@@ -67,22 +74,25 @@ constexpr int al16c(int x) { return (x + 15) & ~15; }
 // an instance; tensor memory is read by warps w and w + 4 (two M halves).
 constexpr int kI5Threads = 256;
 
-// Hankel core matrices per secret polynomial: windows 0..7 (core 4w) over
-// row groups 0..15 and two K chunks reach core 4 * 7 + 15 + 2 = 45.
-constexpr int kHankelCores5 = 46;
-constexpr int kHankelBytes5 = kHankelCores5 * 128;
+// Rows of the Hankel core matrices that one thread makes from one window of
+// s_ext: 6 rows take 4 128-bit loads and 14 byte permutes (2 rows at a time,
+// from one copy of s_ext, took 3 x 2 loads, 3 x 7 selects for the odd
+// windows and 3 x 6 permutes for Saber's three polynomials).
+constexpr int kHankelRun = 6;
 
 // Shared-memory layout of one CTA (byte offsets).  The operand region ENG
 // holds the Hankel core matrices H (l x kHankelBytes5), the digit columns B
 // and s_ext; the packed GenMatrix / GenSecret / b streams and the packed
 // secret key are only read before H is written, so they land inside H.
 //
-// Digit columns of one j: K step t (32 K rows, K reversed) has G groups of 8
-// columns and sits in block t & 3, at group slots 0..G-1 for t >= 4 and
-// G..2G-1 for t < 4, so one N = 16 G descriptor on block r reads step r + 4
-// (columns 0..8G-1) beside step r (columns 8G..16G-1).  Within a block the
-// second K chunk of every slot lies LB = 2G * 128 + 16 bytes after the
-// first (the pad spreads one column's chunks over the banks).
+// Digit columns of one j: K step t is 32 K rows (K reversed), two 16-byte K
+// chunks, in blocks of two steps: column 2n + (t & 1) of a block, PG groups of
+// 8 columns (SB bytes a group, the chunks LB apart), in two sequences,
+// [4 5][0 1][-4 -5] and [6 7][2 3][-6 -7] (-t: the digits of step t negated),
+// so that one descriptor at the start of a sequence reads steps (4, 5 | 0, 1)
+// and one a block later (0, 1 | -4, -5).
+// The strides put the 16-byte pieces that a store instruction writes at once
+// into different banks.
 template <int OP, int SET>
 struct LayoutC {
   using C = SetC<SET>;
@@ -98,23 +108,40 @@ struct LayoutC {
   // matvec: A as 16-bit coefficients (l x l x 512 bytes) inside H, int8 secrets after it
   static constexpr bool HAS_MV = OP == kMatvec;
   static constexpr int MV_A = C::L * C::L * 512, MV_S = C::L * 256;
-  static constexpr int G = S::G;
-  static constexpr int LB = 2 * G * 128 + 16;  // second K chunk of a block
-  static constexpr int RB = 2 * LB;            // one block
-  static constexpr int BJ = 4 * RB;            // digit columns of one j
-  // byte offset of K chunk a (16 K rows, K reversed) within one j
-  __host__ __device__ static constexpr int chunk_off(int a) {
-    return ((a >> 1) & 3) * RB + (a < 8 ? G * 128 : 0) + (a & 1) * LB;
+  // Hankel core matrices per secret polynomial: tiles start at block w of 32
+  // rows (core 4w, w <= 6) and reach 15 row groups and two K chunks on; in
+  // whole runs of kHankelRun rows a thread
+  static constexpr int CORES = 42;
+  static constexpr int PAIRS = CORES / kHankelRun;  // 8-thread groups per polynomial
+  static_assert(CORES % kHankelRun == 0 && C::L * PAIRS <= kI5Threads / 8, "one run per thread");
+  // s_ext of one j: 96 words (what the cores read), and the same one word on,
+  // EXC bytes after the first (4 of 8 16-byte units apart in the banks)
+  static constexpr int EXC = 448, EXJ = 2 * EXC;
+  static_assert(4 * (2 * (CORES - kHankelRun) + 16) <= 384, "the loads stay inside one copy");
+  static constexpr int HJ = CORES * 128;
+  static constexpr int LB = 160;
+  static constexpr int SB = S::NC4 == 16 ? 304 : 288;
+  static constexpr int QB = 16 * (S::NC4 == 16 ? 234 : (S::NC4 == 12 ? 164 : (S::NC4 == 8 ? 114 : 60)));  // one sequence, padded
+  static_assert(QB >= 3 * S::PG * SB, "a sequence's three blocks");
+  static constexpr int BJ = 2 * QB;  // digit columns of one j
+  // byte offset of step t's columns within one j, and of their negated copy (t >= 4)
+  __device__ static __forceinline__ uint32_t step_off(int t) {
+    return (uint32_t)(((t >> 1) & 1) * QB + (t >= 4 ? 0 : S::PG * SB) + (t & 1) * 16);
   }
+  __device__ static __forceinline__ uint32_t neg_off(int t) {
+    return (uint32_t)(((t >> 1) & 1) * QB + 2 * S::PG * SB + (t & 1) * 16);
+  }
+  // byte offset of digit column n from there
+  __host__ __device__ static constexpr int col_off(int n) { return (n >> 2) * SB + (n & 3) * 32; }
   static constexpr int ENG = 0;
   static constexpr int H = ENG;
   static constexpr int A = H;                                    // streams inside H
   static constexpr int SS = HAS_AS ? al16c(A + C::GM + 16) : (HAS_MV ? al16c(A + MV_A) : A);
   static constexpr int B = HAS_AS ? al16c(SS + C::GS + 16) : SS;
   static constexpr int SKO = H;
-  static constexpr int BM = H + C::L * kHankelBytes5;
+  static constexpr int BM = H + C::L * HJ;
   static constexpr int EXT = BM + C::L * BJ;
-  static constexpr int ENG_END_OPS = EXT + C::L * 512;
+  static constexpr int ENG_END_OPS = EXT + C::L * EXJ;
   static constexpr int ENG_BYTES = ENG_END_OPS;
   // the output ops' 16-bit values (R x 512 bytes), over the digit columns
   // (the next instance's inputs are landing in H)
@@ -126,16 +153,24 @@ struct LayoutC {
   static constexpr int MSG = HAS_CT ? al16c(CTO + NCT * CTS) : CTO;
   static constexpr int CTB = (HAS_B ? al16c(MSG + 32 + 16) : MSG) - CTO;
   static constexpr int SEC8 = CTO + 2 * CTB;
-  static constexpr int OUT = OP == kKeygen ? al16c(SEC8 + C::L * 256) : SEC8;
+  // Epilogue buffers inside H, past the inputs of the next instance that are
+  // landing there (the MMAs have read H; the next instance writes its core
+  // matrices after a barrier that follows the epilogue): accumulator sums that
+  // another warp finishes, and the packed outputs.
+  static constexpr int XWORDS = (S::R + 1) / 2;
+  static constexpr int XCH = HAS_AS ? al16c(B + (HAS_B ? C::L * C::POLYCOMP + 16 : 16))
+                                    : (HAS_SK ? al16c(SKO + C::INDCPA_SK + 16) : al16c(SS + MV_S + 16));
+  static constexpr int OUT = XCH + XWORDS * 1024;
   static constexpr int OUT_BYTES = OP == kEncrypt ? C::CT + 16
                                    : (OP == kKeygen ? C::L * C::POLYCOMP + C::INDCPA_SK + 16 : 0);
   // mbarriers in, mma, clc; TMEM base; the next instance; two CLC responses
-  static constexpr int BAR = al16c(OUT + OUT_BYTES);
+  static_assert(OUT + OUT_BYTES <= H + C::L * HJ, "the epilogue buffers fit H");
+  static constexpr int BAR = al16c(SEC8 + (OP == kKeygen ? C::L * 256 : 0));
   static constexpr int TOTAL = BAR + 64;
   static constexpr int IN_BYTES = (HAS_AS ? C::GM + C::GS : 0) + (HAS_B ? C::L * C::POLYCOMP + 32 : 0) +
                                   (HAS_CT ? C::CT : 0) + (HAS_SK ? C::INDCPA_SK : 0) + (HAS_MV ? MV_A + MV_S : 0);
   static_assert(!HAS_AS || B + (HAS_B ? C::L * C::POLYCOMP + 16 : 0) <= BM, "streams fit inside H");
-  static_assert(!HAS_SK || C::INDCPA_SK + 16 <= C::L * kHankelBytes5, "secret key fits inside H");
+  static_assert(!HAS_SK || C::INDCPA_SK + 16 <= C::L * HJ, "secret key fits inside H");
   static_assert(!HAS_MV || SS + MV_S + 16 <= BM, "matvec inputs fit inside H");
 };
 
@@ -161,11 +196,34 @@ __device__ __forceinline__ void unpack8c(const uint8_t *base, int byte0, uint32_
   }
 }
 
-// Four signed 5-bit top digits t (one per byte) as raw e4m3 bytes: t for
-// t < 16, else 0x80 | (32 - t), the number t - 32 (magnitudes up to 16).
+// The same fields two at a time, without clearing the bits above them in
+// each 16-bit lane (raw_digits8 masks its digits).
+template <int W>
+__device__ __forceinline__ uint32_t field_pair(const uint32_t *w, int nw, int bit) {
+  const int i = bit >> 5, sh = bit & 31;
+  const uint32_t y = (sh + 2 * W <= 32 || i + 1 >= nw) ? (w[i] >> sh) : __funnelshift_r(w[i], w[i + 1], sh);
+  return __byte_perm(y, y << (16 - W), 0x7610);
+}
+template <int W>
+__device__ __forceinline__ void unpack8d(const uint8_t *base, int byte0, uint32_t (&X)[4]) {
+  const uint32_t wp = smem_u32(base) + (uint32_t)(byte0 & ~3);
+  const int sh = 8 * (byte0 & 3);
+  uint32_t q[5];
+#pragma unroll
+  for (int i = 0; i < 5; i++) q[i] = lds32(wp + 4 * i);
+  uint32_t a[4];
+#pragma unroll
+  for (int i = 0; i < 4; i++) a[i] = __funnelshift_r(q[i], q[i + 1], sh);
+#pragma unroll
+  for (int k = 0; k < 4; k++) X[k] = field_pair<W>(a, 4, 2 * W * k);
+}
+
+// Signed 5-bit top digits t (the low five bits of each byte) as raw e4m3
+// bytes: t for t < 16, else 0x80 | (32 - t), the number t - 32 (magnitudes up
+// to 16): 32 - t = 15 - (t & 15) + 1.
 __device__ __forceinline__ uint32_t raw_sdigits4(uint32_t t) {
-  const uint32_t m = ((t >> 4) & 0x01010101u) * 0xFFu;  // bytes with t >= 16
-  return (m & ((0x20202020u - t) | 0x80808080u)) | (~m & t);
+  const uint32_t s = (t >> 4) & 0x01010101u;
+  return ((t & 0x0F0F0F0Fu) ^ (s * 15u)) + s * 0x81u;
 }
 
 // Radix-16 digit d (r16_digits) of eight W-bit coefficients X (four words of
@@ -190,55 +248,70 @@ __device__ __forceinline__ uint2 raw_digits8(const uint32_t (&X)[4], int d) {
     a = __byte_perm(X[2] >> lo, X[3] >> lo, 0x0246);
     b = __byte_perm(X[0] >> lo, X[1] >> lo, 0x0246);
   }
-  a &= mask;
-  b &= mask;
-  if (wd == 5) {
-    a = raw_sdigits4(a);
-    b = raw_sdigits4(b);
-  }
-  return make_uint2(a, b);
+  if (wd == 5) return make_uint2(raw_sdigits4(a), raw_sdigits4(b));
+  return make_uint2(a & mask, b & mask);
+}
+
+// The Hankel core matrices of the L polynomials (row x = 8m + i of core m,
+// s_ext[x .. x + 15], at byte 16x of H + j * HJ).  Eight threads (four byte
+// shifts sh, two parities) make the rows of kHankelRun consecutive cores;
+// thread (sh, par) the rows 4q + sh, q = 2m + par, windows of s_ext words
+// that start at q: from the copy of s_ext one word on for par = 1, so that
+// every window starts on a 16-byte boundary.
+template <class LO, int L>
+__device__ __forceinline__ void stage_hankel6(uint32_t H, uint32_t ext, int tid) {
+  const int item = tid >> 3;
+  if (item >= L * LO::PAIRS) return;
+  const int sh = tid & 3, par = (tid >> 2) & 1, j = item / LO::PAIRS, m0 = (item % LO::PAIRS) * kHankelRun;
+  const uint32_t sel = 0x3210u + 0x1111u * (uint32_t)sh;
+  const uint32_t e = ext + (uint32_t)(j * LO::EXJ + par * LO::EXC + 8 * m0);
+  constexpr int NP = 2 * kHankelRun + 2;  // permuted words
+  uint32_t w[NP + 2];
+#pragma unroll
+  for (int i = 0; i < NP + 2; i += 4) lds128(e + 4 * i, w[i], w[i + 1], w[i + 2], w[i + 3]);
+#pragma unroll
+  for (int i = 0; i < NP; i++) w[i] = __byte_perm(w[i], w[i + 1], sel);
+  const uint32_t h = H + (uint32_t)(j * LO::HJ + 128 * m0 + 64 * par + 16 * sh);
+#pragma unroll
+  for (int r = 0; r < kHankelRun; r++) sts128(h + 128 * r, w[2 * r], w[2 * r + 1], w[2 * r + 2], w[2 * r + 3]);
 }
 
 // Digit columns of 32 coefficients of one W-bit packed polynomial: lane m
 // (0..7) of an 8-lane group takes coefficients 32m .. 32m + 31, exactly W
 // aligned words of the stream at src, so that four groups (a warp) reading
 // four polynomials load conflict-free, one 32-bit word per lane per load.
-// Coefficient groups 4m .. 4m + 3 of 8 (K rows 8 kq .. 8 kq + 7, kq = 31 - g,
-// K reversed) fill the two 16-byte K chunks a = 15 - 2m and 14 - 2m of each
-// digit column, one 128-bit store each.  colbase: the digit columns of this
-// j (LO::BM + j * LO::BJ as a shared-window address); cb: first column.
+// They are K step t = 7 - m: coefficient groups 4m, 4m + 1 of 8 fill the second
+// 16-byte K chunk of each digit column and 4m + 2, 4m + 3 the first, one 128-bit
+// store each (and one more for the negated copy of steps 4..7).  colbase: the
+// digit columns of this j (LO::BM + j * LO::BJ as a shared-window address); cb:
+// first column.
 template <int W, class LO>
 __device__ __forceinline__ void stage_digits32(const uint8_t *sm, int src, uint32_t colbase, int cb, int m) {
   const uint32_t wp = smem_u32(sm) + (uint32_t)(src + 4 * W * m);
   uint32_t w[W];
 #pragma unroll
   for (int i = 0; i < W; i++) w[i] = lds32(wp + 4 * i);
-  constexpr uint32_t mask = (1u << W) - 1u;
-  uint32_t X[16];  // coefficients 2k, 2k + 1 as the low / high 16-bit lanes of X[k]
+  uint32_t X[16];  // coefficients 2k, 2k + 1 in the low / high 16-bit lanes of X[k]
 #pragma unroll
-  for (int k = 0; k < 16; k++) {
-    uint32_t v[2];
-#pragma unroll
-    for (int h = 0; h < 2; h++) {
-      const int bit = W * (2 * k + h), i = bit >> 5, sh = bit & 31;
-      v[h] = ((sh + W <= 32) ? (w[i] >> sh) : __funnelshift_r(w[i], w[i + 1], sh)) & mask;
-    }
-    X[k] = __byte_perm(v[0], v[1], 0x5410);
-  }
-  const int a1 = 14 - 2 * m;  // and a0 = a1 + 1, LB bytes after it
-  const uint32_t c1 = colbase + (uint32_t)LO::chunk_off(a1);
+  for (int k = 0; k < 16; k++) X[k] = field_pair<W>(w, W, 2 * W * k);
+  const int t = 7 - m;
+  const uint32_t c1 = colbase + LO::step_off(t), cn = colbase + LO::neg_off(t);
 #pragma unroll
   for (int d = 0; d < r16_digits(W); d++) {
     uint2 v[4];
 #pragma unroll
-    for (int t = 0; t < 4; t++) {
-      const uint32_t Xt[4] = {X[4 * t], X[4 * t + 1], X[4 * t + 2], X[4 * t + 3]};
-      v[t] = raw_digits8<W>(Xt, d);
+    for (int g = 0; g < 4; g++) {
+      const uint32_t Xg[4] = {X[4 * g], X[4 * g + 1], X[4 * g + 2], X[4 * g + 3]};
+      v[g] = raw_digits8<W>(Xg, d);
     }
-    const int n = cb + d;
-    const uint32_t col = c1 + (uint32_t)((n >> 3) * 128 + (n & 7) * 16);
-    sts128(col + LO::LB, v[1].x, v[1].y, v[0].x, v[0].y);  // chunk a0: kq 30 - 4m, then 31 - 4m
-    sts128(col, v[3].x, v[3].y, v[2].x, v[2].y);           // chunk a1: kq 28 - 4m, then 29 - 4m
+    const uint32_t co = (uint32_t)LO::col_off(cb + d);
+    sts128(c1 + co + LO::LB, v[1].x, v[1].y, v[0].x, v[0].y);
+    sts128(c1 + co, v[3].x, v[3].y, v[2].x, v[2].y);
+    if (t >= 4) {
+      constexpr uint32_t n = 0x80808080u;
+      sts128(cn + co + LO::LB, v[1].x ^ n, v[1].y ^ n, v[0].x ^ n, v[0].y ^ n);
+      sts128(cn + co, v[3].x ^ n, v[3].y ^ n, v[2].x ^ n, v[2].y ^ n);
+    }
   }
 }
 
@@ -299,6 +372,29 @@ __device__ __forceinline__ void cpa5i_load(const CpaArgs &a, const unsigned inst
     bulk_g2s(d + LO::A, reinterpret_cast<const uint8_t *>(a.mv_A) + (size_t)inst * LO::MV_A, LO::MV_A, mbar);
     bulk_g2s(d + LO::SS, reinterpret_cast<const uint8_t *>(a.mv_s) + (size_t)inst * LO::MV_S, LO::MV_S, mbar);
   }
+}
+
+// Digit sums.  An accumulator holds x * 2^-9 for an exact integer x with
+// |x| < 2^22, so adding 1.5 * 2^14 (24576) leaves x in the low bits of the
+// f32 pattern; the pattern of 24576.0 itself is 0 in its low 16 bits, which
+// are all that the results (mod 2^13 or less) need.  sum_d 16^d x_d is formed
+// in f32 by fused multiply-adds where it stays below 2^22 for every
+// admissible secret (exact: an integer below 2^24 in units of 2^-9), else the
+// digit of weight 256 joins as an integer.
+constexpr int digit_bound(int w) { return w == 13 ? 17 * 256 : (w == 9 ? 17 * 16 : (1 << w) - 1); }
+
+// Product p's share of the even (par 0) or odd (1) K steps of one coefficient,
+// from its accumulator columns f, in the low 16 bits.
+template <int OP, int SET>
+__device__ __forceinline__ uint32_t combine5(const uint32_t (&f)[2 * ShapeC<OP, SET>::NC4], int p, int par) {
+  using S = ShapeC<OP, SET>;
+  const int c0 = S::col_base(p), D = S::digits(p), W = p < S::RA ? S::WA : S::WB;
+  auto col = [&](int d) { return __uint_as_float(f[2 * (c0 + d) + par]); };
+  float x = col(0) + 24576.0f;
+  if (D > 1) x = __fmaf_rn(16.0f, col(1), x);
+  if (D < 3) return __float_as_uint(x);
+  if (digit_bound(W) * S::SMAX * S::ROWS < (1 << 22)) return __float_as_uint(__fmaf_rn(256.0f, col(2), x));
+  return __float_as_uint(x) + 256u * __float_as_uint(col(2) + 24576.0f);
 }
 
 // The instances of a launch, from the CTA of kI5Threads threads that runs
@@ -362,7 +458,7 @@ __device__ __forceinline__ void cpa5i_run(const AT &at, uint8_t *sm) {
   bool ok = true;
   if (ready) {
     // 1. secrets, straight into s_ext (s_ext[d] = -s[d + 1] for d < 255,
-    // s[d - 255] for 255 <= d <= 510, 0 at 511; 128 words per j).  Warp
+    // s[d - 255] for 255 <= d; the first 96 words, twice).  Warp
     // j < L makes polynomial j: lane g encodes the words 2g, 2g + 1
     // (coefficients 8g..8g+7) and takes word 2g + 2 from the next lane
     // (word 0 for lane 31).
@@ -428,8 +524,15 @@ __device__ __forceinline__ void cpa5i_run(const AT &at, uint8_t *sm) {
       // word 63: s_ext[255] = s[0] keeps its sign; word 127: s_ext[511] = 0
       const uint32_t n1 = p1 ^ (g == 31 ? 0x00808080u : 0x80808080u);
       const uint32_t q1 = g == 31 ? __byte_perm(e1, 0u, 0x4321) : p1;
-      sts64(ext32 + 512 * j + 8 * g, p0 ^ 0x80808080u, n1);
-      sts64(ext32 + 512 * j + 256 + 8 * g, p0, q1);
+      // word 2g + 2, from the next lane (word 64 = s_ext[256] on for lane 31)
+      const uint32_t np = __shfl_sync(0xffffffffu, p0, (lane + 1) & 31);
+      const uint32_t ex = ext32 + (uint32_t)(LO::EXJ * j + 8 * g);
+      sts64(ex, p0 ^ 0x80808080u, n1);
+      sts64(ex + LO::EXC, n1, g == 31 ? np : np ^ 0x80808080u);
+      if (g < 16) {
+        sts64(ex + 256, p0, q1);
+        sts64(ex + LO::EXC + 256, q1, np);
+      }
     }
     // 2. digit columns (K reversed, core-matrix order): lane g converts
     // coefficients 8g..8g+7 (K rows k' = 8kq+7..8kq, kq = 31 - g) of one
@@ -438,16 +541,19 @@ __device__ __forceinline__ void cpa5i_run(const AT &at, uint8_t *sm) {
     // NCOLS of each stored group are left as they are: they only feed
     // accumulator columns that are never read.
     const int kq = 31 - lane;
-    const uint32_t bl = smem_u32(Bm) + LO::chunk_off(kq >> 1) + 8 * (kq & 1);
+    const uint32_t bh = smem_u32(Bm) + (uint32_t)(((kq >> 1) & 1) * LO::LB + 8 * (kq & 1));
+    const uint32_t bl = bh + LO::step_off(kq >> 2), bn = bh + LO::neg_off(kq >> 2);
+    auto put = [&](int j, int n, uint2 v) {
+      sts64(bl + j * LO::BJ + LO::col_off(n), v.x, v.y);
+      if (kq >= 16) sts64(bn + j * LO::BJ + LO::col_off(n), v.x ^ 0x80808080u, v.y ^ 0x80808080u);
+    };
     auto item = [&](auto wc, uint32_t src, int cb, int j) {
       constexpr int W = decltype(wc)::value;
       uint32_t X[4];
-      unpack8c<W>(sm + src, lane * W, X);
+      unpack8d<W>(sm + src, lane * W, X);
 #pragma unroll
       for (int d = 0; d < r16_digits(W); d++) {
-        const uint2 v = raw_digits8<W>(X, d);
-        const int n = cb + d;
-        sts64(bl + j * LO::BJ + (n >> 3) * 128 + (n & 7) * 16, v.x, v.y);
+        put(j, cb + d, raw_digits8<W>(X, d));
       }
     };
     if constexpr (OP == kMatvec) {
@@ -464,27 +570,17 @@ __device__ __forceinline__ void cpa5i_run(const AT &at, uint8_t *sm) {
           for (int i = 0; i < 4; i++) X[i] = lds32(src + 4 * i);
 #pragma unroll
           for (int d = 0; d < S::DA; d++) {
-            const uint2 v = raw_digits8<S::WA>(X, d);
-            const int n = p * S::DA + d;
-            sts64(bl + j * LO::BJ + (n >> 3) * 128 + (n & 7) * 16, v.x, v.y);
+            put(j, p * S::DA + d, raw_digits8<S::WA>(X, d));
           }
         }
       }
     } else if constexpr (DECK) {
-      // warp r makes ciphertext r's b'_j for every j (zero columns past the batch)
-      if (warp < S::R) {
+      // warp r makes ciphertext r's b'_j for every j
+      if (warp < nvalid) {
 #pragma unroll
-        for (int j = 0; j < L; j++) {
-          if (warp < nvalid) {
-            item(std::integral_constant<int, S::WB>{}, (int)cbuf + LO::CTO + warp * LO::CTS + 32 * j * S::WB, warp * S::DB, j);
-          } else {
-#pragma unroll
-            for (int d0 = 0; d0 < S::DB; d0++) {
-              const int n = warp * S::DB + d0;
-              sts64(bl + j * LO::BJ + (n >> 3) * 128 + (n & 7) * 16, 0u, 0u);
-            }
-          }
-        }
+        for (int j = 0; j < L; j++)
+          item(std::integral_constant<int, S::WB>{}, (int)cbuf + LO::CTO + warp * LO::CTS + 32 * j * S::WB, warp * S::DB,
+               j);
       }
     } else if constexpr (S::R == 1) {
       if (warp < L) item(std::integral_constant<int, S::WB>{}, (int)cbuf + LO::CTO + 32 * warp * S::WB, 0, warp);
@@ -522,34 +618,66 @@ __device__ __forceinline__ void cpa5i_run(const AT &at, uint8_t *sm) {
     }
     break;
   }
-  stage_hankel_ct<L, NT, kHankelCores5>(smem_u32(H), ext32, tid);
+  stage_hankel6<LO, L>(smem_u32(H), ext32, tid);
   fence_async_smem();  // generic-proxy writes -> visible to the tensor core
   ok = __syncthreads_and(ok) != 0;
   if (!ok && tid == 0 && a.err) atomicOr(a.err, 1);
 
-  // 3. the MMAs (one thread).  Window w of the Hankel sequence (core 4w)
-  // holds rows r of s_ext[r + 32w + e]; rows 128 + r of K step t equal
-  // window t + 4 for t < 4, and -(window t - 4) for t >= 4 (s_ext[d + 256] =
-  // -s_ext[d] for d < 255).  The descriptor on block r reads steps r + 4 and
-  // r, so window r + 4 gives (top, step r + 4 | bottom, step r) in region 0
-  // and window r gives (-bottom, step r + 4 | top, step r) in region 1:
-  // 8 MMAs per j, top = region0[0] + region1[1], bottom = region0[1] - region1[0].
+  // 3. the MMAs (one thread).  Coefficients and K steps come in blocks of 32:
+  // coefficient block o takes step t through the 32 x 32 Hankel block
+  // B = o + t (rows 32B + r of s_ext[. + e]), where block B + 8 = -block B
+  // (s_ext[d + 256] = -s_ext[d] for d < 255).  A tile w is the blocks
+  // w .. w + 3, four lane quadrants rho, read from core 4w on.  An MMA costs
+  // about (4 KB + 32 N bytes) / 128 cycles, the reads of its operands from
+  // shared memory (N = 16: 39, 32: 40, 64: 48 cycles measured), so fewer MMAs of a
+  // larger N do the same products in less time.
+  // So only the even tiles are used, each against four steps: tile w against
+  // step w gives blocks o = rho, against step w - 4 (w < 4: the negated step
+  // w + 4) blocks o = rho + 4; against the odd steps w + 1 and w - 3 (-(w + 5))
+  // blocks o = rho - 1 (block -1 = -block 7) and rho + 3, which other warps
+  // finish.  Two sets of 2 NC4 columns, for rho and rho + 4, even and odd
+  // steps in turn.  12 MMAs of N = 48 for Saber's re-encryption (24 of N = 32
+  // with a tile per step): 342 -> 301 us at 65536 with the stagings above, the
+  // decryption 246 -> 216.  (Two tiles against all eight steps, 6 MMAs of
+  // N = 32 for the decryption, took 225: the sums of eight products of each
+  // block then cross all warps.)
   if (tid == 0) {
     tc_fence_after();  // the previous instance's accumulator loads come before these MMAs
     constexpr uint32_t idesc = umma_idesc_e4m3(NU);
     const uint64_t ad0 = umma_desc(smem_u32(H), 256, 128);
-    const uint32_t b0 = smem_u32(Bm);
+    const uint64_t bd0 = umma_desc(smem_u32(Bm), LO::LB, LO::SB);
 #pragma unroll
     for (int j = 0; j < L; j++) {
-      const uint64_t hj = ad0 + (uint64_t)((j * kHankelBytes5) >> 4);
+      const uint64_t hj = ad0 + (uint64_t)((j * LO::HJ) >> 4), bj = bd0 + (uint64_t)((j * LO::BJ) >> 4);
 #pragma unroll
-      for (int r = 0; r < 4; r++) {
-        const uint64_t bd = umma_desc(b0 + j * LO::BJ + r * LO::RB, LO::LB, 128);
-        umma_f8(tmem, hj + (uint64_t)((4 * (r + 4) * 128) >> 4), bd, idesc, (j | r) != 0);
-        umma_f8(tmem + NU, hj + (uint64_t)((4 * r * 128) >> 4), bd, idesc, (j | r) != 0);
-      }
+      for (int w = 0; w < 8; w += 2)
+        umma_f8(tmem, hj + (uint64_t)((4 * w * 128) >> 4),
+                bj + (uint64_t)((((w >> 1) & 1) * LO::QB + (w < 4 ? S::PG * LO::SB : 0)) >> 4), idesc, (j | w) != 0);
     }
     umma_commit(mbar_mma);
+  }
+  // The thread's coefficient k (block o = 4 hsel + q4 of 32; its warp reads
+  // tensor-memory lanes 32 q4 ..), and beside the MMAs what the epilogue needs
+  // of the inputs: the ciphertext's coefficient k, the message bit.
+  const int q4 = warp & 3, hsel = warp >> 2;
+  const int k = 128 * hsel + 32 * q4 + lane;
+  // W-bit field at bit `bit` of a 4-byte-aligned shared-memory stream
+  auto field = [&](int byte_off, int bit, int W) -> uint32_t {
+    const uint32_t *w = reinterpret_cast<const uint32_t *>(sm + byte_off) + (bit >> 5);
+    return __funnelshift_r(w[0], w[1], bit & 31) & ((1u << W) - 1u);
+  };
+
+  uint32_t cf[LO::HAS_CT ? S::R : 1], mk = 0;
+  if constexpr (IS_DEC) {  // c_m of each ciphertext
+#pragma unroll
+    for (int r = 0; r < S::R; r++)
+      cf[r] = field((int)cbuf + LO::CTO + r * LO::CTS + L * C::POLYCOMP, k * C::ET, C::ET);
+  }
+  if constexpr (LO::HAS_B) mk = (sm[LO::MSG + cbuf + (k >> 3)] >> (k & 7)) & 1u;
+  if constexpr (OP == kReenc) {
+#pragma unroll
+    for (int p = 0; p < L; p++) cf[p] = field((int)cbuf + LO::CTO + p * C::POLYCOMP, k * C::EP, C::EP);
+    cf[L] = field((int)cbuf + LO::CTO + L * C::POLYCOMP, k * C::ET, C::ET);
   }
   // 4. accumulators: one warp polls the MMA barrier and the CLC answer, the
   // others wait in the CTA barrier.  The MMAs have read H and the other
@@ -582,88 +710,64 @@ __device__ __forceinline__ void cpa5i_run(const AT &at, uint8_t *sm) {
   }
   const uint32_t next = *next_slot;
   tc_fence_after();
-  // warp w reads TMEM lanes 32 (w % 4) .. +31 for coefficient
-  // k = 128 hsel + 32 q4 + lane (hsel = w / 4): every digit column of k,
-  // top = region0[0] + region1[1], bottom = region0[1] - region1[0]
-  const int q4 = warp & 3, hsel = warp >> 2;
-  const int k = 128 * hsel + 32 * q4 + lane;
-  constexpr int G8 = 8 * LO::G;
-  float xacc[G8];  // digit column c of coefficient k, times 2^-9 (exact)
+  const uint32_t xch = smem_u32(sm + LO::XCH);
+  // coefficient k of every product, in the low 16 bits (a.. the sums of an
+  // accumulator's digit columns, see combine5)
+  uint32_t val[S::R];
   {
     const uint32_t t0 = tmem + ((uint32_t)(32 * q4) << 16);
-    uint32_t f[G8], g[G8];
-    if constexpr (G8 == 8) {
-      tmem_ld8(t0 + (hsel ? 8 : 0), f);
-      tmem_ld8(t0 + (hsel ? 16 : 24), g);
-    } else {
-      tmem_ld16(t0 + (hsel ? 16 : 0), f);
-      tmem_ld16(t0 + (hsel ? 32 : 48), g);
+    // odd steps first: block o' = q4 - 1 (hsel 0; block 7 negated for
+    // q4 = 0) or q4 + 3, for the warp of that block; two 16-bit values a word
+    uint32_t f[2 * S::NC4];
+    uint32_t odd[2 * LO::XWORDS];
+    odd[2 * LO::XWORDS - 1] = 0;
+    tmem_ld_cols(t0 + (uint32_t)(2 * S::NC4 * hsel), f);
+    const int od = (warp + 7) & 7;  // the block the odd steps belong to
+#pragma unroll
+    for (int p = 0; p < S::R; p++) odd[p] = combine5<OP, SET>(f, p, 1);
+    if (warp == 0) {
+#pragma unroll
+      for (int p = 0; p < S::R; p++) odd[p] = 0u - odd[p];
     }
-    if (hsel) {
 #pragma unroll
-      for (int c = 0; c < S::NCOLS; c++) xacc[c] = __uint_as_float(f[c]) - __uint_as_float(g[c]);
-    } else {
+    for (int i = 0; i < LO::XWORDS; i++)
+      sts32(xch + (uint32_t)((i * 256 + 32 * od + lane) * 4), __byte_perm(odd[2 * i], odd[2 * i + 1], 0x5410));
 #pragma unroll
-      for (int c = 0; c < S::NCOLS; c++) xacc[c] = __uint_as_float(f[c]) + __uint_as_float(g[c]);
-    }
-    if constexpr (OP == kEncrypt || OP == kKeygen) {
-      // coefficient k of every output polynomial, rounded (b, b') or encoded
-      // with the message bit (c_m), as 16-bit values for the packing pass;
-      // the MMAs are done, so the digit columns are free
-      constexpr uint32_t qm = (1u << C::EQ) - 1u, pm = (1u << C::EP) - 1u;
-      uint16_t *vals = reinterpret_cast<uint16_t *>(sm + LO::VALS);
+    for (int p = 0; p < S::R; p++) val[p] = combine5<OP, SET>(f, p, 0);
+    tc_fence_before();  // the loads above come before the next instance's MMAs (its barriers lie between)
+    __syncthreads();
 #pragma unroll
-      for (int p = 0; p < S::R; p++) {
-        uint32_t v = 0, off = 0;
-#pragma unroll
-        for (int d = 0; d < 4; d++) {
-          if (d < S::digits(p)) {
-            v += (1u << (4 * d)) * __float_as_uint(xacc[S::col_base(p) + d] + 24576.0f);
-            off += (1u << (4 * d)) * 0x46C00000u;
-          }
-        }
-        v -= off;
-        if (p < L) {
-          vals[256 * p + k] = (uint16_t)(((v + C::H1) & qm) >> (C::EQ - C::EP));
-        } else {
-          const uint32_t mk = (sm[LO::MSG + cbuf + (k >> 3)] >> (k & 7)) & 1u;
-          vals[256 * p + k] = (uint16_t)(((v + C::H1 - (mk << (C::EP - 1))) & pm) >> (C::EP - C::ET));
-        }
-      }
+    for (int i = 0; i < LO::XWORDS; i++) {
+      const uint32_t x = lds32(xch + (uint32_t)((i * 256 + tid) * 4));
+      val[2 * i] += x;
+      if (2 * i + 1 < S::R) val[2 * i + 1] += x >> 16;
     }
   }
-  tc_fence_before();  // the loads above come before the next instance's MMAs (its barriers lie between)
-  if constexpr (OP == kEncrypt || OP == kKeygen) __syncthreads();  // the 16-bit values are complete
+  if constexpr (OP == kEncrypt || OP == kKeygen) {
+    // coefficient k of every output polynomial, rounded (b, b') or encoded
+    // with the message bit (c_m), as 16-bit values for the packing pass;
+    // the MMAs are done, so the digit columns are free
+    constexpr uint32_t qm = (1u << C::EQ) - 1u, pm = (1u << C::EP) - 1u;
+    uint16_t *vals = reinterpret_cast<uint16_t *>(sm + LO::VALS);
+#pragma unroll
+    for (int p = 0; p < S::R; p++) {
+      const uint32_t v = val[p];
+      if (p < L) {
+        vals[256 * p + k] = (uint16_t)(((v + C::H1) & qm) >> (C::EQ - C::EP));
+      } else {
+        vals[256 * p + k] = (uint16_t)(((v + C::H1 - (mk << (C::EP - 1))) & pm) >> (C::EP - C::ET));
+      }
+    }
+    __syncthreads();  // the 16-bit values are complete
+  }
 
   // 5. epilogues
   constexpr uint32_t qmask = (1u << C::EQ) - 1u, pmask = (1u << C::EP) - 1u;
-  // sum_d 16^d acc_d of the digit columns c0..: each f32
-  // accumulator holds x * 2^-9 for an exact integer |x| < 2^22, so adding
-  // 1.5 * 2^14 leaves x + 0x46C00000 in its bit pattern; the offsets are
-  // removed at the end
-  auto combine1 = [&](int c0, int D) -> uint32_t {
-    uint32_t v = 0, off = 0;
-#pragma unroll
-    for (int d = 0; d < 4; d++) {
-      if (d < D) {
-        v += (1u << (4 * d)) * __float_as_uint(xacc[c0 + d] + 24576.0f);
-        off += (1u << (4 * d)) * 0x46C00000u;
-      }
-    }
-    return v - off;
-  };
-  // W-bit field at bit `bit` of a 4-byte-aligned shared-memory stream
-  auto field = [&](int byte_off, int bit, int W) -> uint32_t {
-    const uint32_t *w = reinterpret_cast<const uint32_t *>(sm + byte_off) + (bit >> 5);
-    return __funnelshift_r(w[0], w[1], bit & 31) & ((1u << W) - 1u);
-  };
-
   if constexpr (OP == kDecrypt) {
     // m'_k = ((v_k + h2 - (c_m,k << (ep-et))) mod p) >> (ep-1): one bit per
     // thread, gathered into bytes by a ballot per warp
-    const uint32_t v = combine1(0, S::DB);
-    const uint32_t cm = field((int)cbuf + LO::CTO + L * C::POLYCOMP, k * C::ET, C::ET);
-    const uint32_t t = (v + C::H2 - (cm << (C::EP - C::ET))) & pmask;
+    const uint32_t v = val[0];
+    const uint32_t t = (v + C::H2 - (cf[0] << (C::EP - C::ET))) & pmask;
     const uint32_t bits = __ballot_sync(0xffffffffu, ((t >> (C::EP - 1)) & 1u) != 0u);
     uint8_t *mo = a.m_out + (size_t)inst * a.m_out_stride;
     if (lane < 4) mo[4 * (4 * hsel + q4) + lane] = (uint8_t)(bits >> (8 * lane));
@@ -673,9 +777,8 @@ __device__ __forceinline__ void cpa5i_run(const AT &at, uint8_t *sm) {
 #pragma unroll
     for (int r = 0; r < S::R; r++) {
       if (r >= nvalid) break;
-      const uint32_t v = combine1(r * S::DB, S::DB);
-      const uint32_t cm = field((int)cbuf + LO::CTO + r * LO::CTS + L * C::POLYCOMP, k * C::ET, C::ET);
-      const uint32_t t = (v + C::H2 - (cm << (C::EP - C::ET))) & pmask;
+      const uint32_t v = val[r];
+      const uint32_t t = (v + C::H2 - (cf[r] << (C::EP - C::ET))) & pmask;
       const uint32_t bits = __ballot_sync(0xffffffffu, ((t >> (C::EP - 1)) & 1u) != 0u);
       uint8_t *mo = a.m_out + (inst0 + r) * a.m_out_stride;
       if (lane < 4) mo[4 * (4 * hsel + q4) + lane] = (uint8_t)(bits >> (8 * lane));
@@ -683,17 +786,16 @@ __device__ __forceinline__ void cpa5i_run(const AT &at, uint8_t *sm) {
     }
   } else if constexpr (OP == kReenc) {
     // round coefficient k of b' and encode that of v', compare with the ciphertext
-    const uint32_t mk = (sm[LO::MSG + cbuf + (k >> 3)] >> (k & 7)) & 1u;
     uint32_t diff = 0;
 #pragma unroll
     for (int p = 0; p < S::R; p++) {
-      const uint32_t v = combine1(S::col_base(p), S::digits(p));
+      const uint32_t v = val[p];
       if (p < L) {
         const uint32_t w = ((v + C::H1) & qmask) >> (C::EQ - C::EP);
-        diff |= w ^ field((int)cbuf + LO::CTO + p * C::POLYCOMP, k * C::EP, C::EP);
+        diff |= w ^ cf[p];
       } else {
         const uint32_t w = ((v + C::H1 - (mk << (C::EP - 1))) & pmask) >> (C::EP - C::ET);
-        diff |= w ^ field((int)cbuf + LO::CTO + L * C::POLYCOMP, k * C::ET, C::ET);
+        diff |= w ^ cf[L];
       }
     }
     if (__any_sync(0xffffffffu, diff != 0u) && lane == 0) a.fail[inst] = 1;
@@ -702,7 +804,7 @@ __device__ __forceinline__ void cpa5i_run(const AT &at, uint8_t *sm) {
     const uint32_t m = (1u << a.mv_eq) - 1u;
     uint16_t *o = a.mv_out + (size_t)inst * (L * 256) + k;
 #pragma unroll
-    for (int p = 0; p < L; p++) o[256 * p] = (uint16_t)(combine1(S::col_base(p), S::DA) & m);
+    for (int p = 0; p < L; p++) o[256 * p] = (uint16_t)(val[p] & m);
   } else if (OP == kEncrypt) {
     // pack the 16-bit values eight at a time: b' at EP bits, c_m at ET bits
     const uint16_t *vals = reinterpret_cast<const uint16_t *>(sm + LO::VALS);
@@ -752,14 +854,17 @@ __device__ __forceinline__ void cpa5i_run(const AT &at, uint8_t *sm) {
 }
 
 // CTAs per SM that shared memory (228 KB, 1 KB of it per CTA reserved) and
-// tensor memory (512 columns) allow, 6 at most (40 registers, which every
-// kernel comes close to by itself; decryption needs 32 and gets its 8 CTAs):
-// the speed comes from the CTAs that overlap each other's phases.
+// tensor memory (512 columns) allow, and at most what the registers allow
+// without spilling more than a few words: 8 of 32 registers (decryption, 212
+// against 216 us with 6 at 65536), 6 of 40, and 5 of 48 where a thread loads
+// 32 accumulator columns.  The speed comes from the CTAs that overlap each
+// other's phases.
 template <int OP, int SET>
 constexpr int min_ctas() {
   constexpr int by_smem = (228 * 1024) / (LayoutC<OP, SET>::TOTAL + 1024), by_tmem = 512 / ShapeC<OP, SET>::TMEM_COLS;
   constexpr int m = by_smem < by_tmem ? by_smem : by_tmem;
-  return m < 6 ? m : 6;
+  constexpr int cap = ShapeC<OP, SET>::NC4 == 16 ? 5 : (OP == kDecrypt ? 8 : 6);
+  return m < cap ? m : cap;
 }
 
 // The arguments and the instance that CTA gi of a launch stands for.

@@ -8,8 +8,8 @@
 //     c = 255 - k';
 //   * B_j holds N digit columns of the public polynomials of module index j,
 //     coefficient c at row k' = 255 - c;
-// with tcgen05.mma kind::f8f6f4 (e4m3 x e4m3 -> f32), M = 128 (two halves),
-// N = 16 or 32, K = 32 per instruction, A and B read from shared memory and D
+// with tcgen05.mma kind::f8f6f4 (e4m3 x e4m3 -> f32), M = 128, N = 16 .. 64,
+// K = 32 per instruction, A and B read from shared memory and D
 // accumulated in tensor memory (TMEM).
 //
 // Operand layout (K-major, no swizzle): the MMA reads "core matrices" of 8
@@ -20,12 +20,13 @@
 //     s_ext[8b + 16a + i + e] (row i, byte e), which depends on m = b + 2a
 //     only.  So H_j is stored as distinct core matrices at m * 128 bytes and
 //     described with SBO = 128 and LBO = 256: the MMA's core matrix (b, a)
-//     lands on m = b + 2a.  The per-instance kernel (cpa5i.cuh) reads eight
-//     windows of the sequence and needs 46 of them, m = 0..45 (5.75 KB per
-//     secret polynomial, kHankelCores5); the persistent kernel
-//     (cpa_persist.cuh) keeps the earlier layout of 62 (7.75 KB,
-//     kHankelCores) -- either instead of the 64 KB of the dense matrix.
-//   * B_j: dense, core (8-column group c, K chunk a) at a * (16 N) + c * 128.
+//     lands on m = b + 2a.  The per-instance kernel (cpa5i.cuh) reads even
+//     tiles of the sequence and needs 42 of them (5.25 KB per secret
+//     polynomial); the persistent kernel (cpa_persist.cuh) keeps the earlier
+//     layout of 62 (7.75 KB, kHankelCores) -- either instead of the 64 KB of
+//     the dense matrix.
+//   * B_j, persistent kernel: dense, core (8-column group c, K chunk a) at
+//     a * (16 N) + c * 128; per-instance kernel: LayoutC there.
 //
 // Every product of an e4m3 digit (0..15) and an e4m3 secret (|s| <= 7) is an
 // integer of magnitude <= 105, and every sum the MMA forms is an integer of
@@ -172,6 +173,31 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
       : "memory");
 }
 
+// 8, 16, 24 or 32 columns, one wait
+__device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t (&r)[8]) { tmem_ld8(taddr, r); }
+__device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t (&r)[16]) { tmem_ld16(taddr, r); }
+__device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t (&r)[24]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%24];\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%16,%17,%18,%19,%20,%21,%22,%23}, [%25];\n\t"
+      "tcgen05.wait::ld.sync.aligned;"
+      : "=&r"(r[0]), "=&r"(r[1]), "=&r"(r[2]), "=&r"(r[3]), "=&r"(r[4]), "=&r"(r[5]), "=&r"(r[6]), "=&r"(r[7]), "=&r"(r[8]), "=&r"(r[9]), "=&r"(r[10]), "=&r"(r[11]), "=&r"(r[12]), "=&r"(r[13]), "=&r"(r[14]), "=&r"(r[15]), "=&r"(r[16]), "=&r"(r[17]), "=&r"(r[18]), "=&r"(r[19]), "=&r"(r[20]), "=&r"(r[21]), "=&r"(r[22]), "=&r"(r[23])
+      : "r"(taddr), "r"(taddr + 16)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t (&r)[32]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%32];\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%33];\n\t"
+      "tcgen05.wait::ld.sync.aligned;"
+      : "=&r"(r[0]), "=&r"(r[1]), "=&r"(r[2]), "=&r"(r[3]), "=&r"(r[4]), "=&r"(r[5]), "=&r"(r[6]), "=&r"(r[7]), "=&r"(r[8]), "=&r"(r[9]), "=&r"(r[10]), "=&r"(r[11]), "=&r"(r[12]), "=&r"(r[13]), "=&r"(r[14]), "=&r"(r[15]), "=&r"(r[16]), "=&r"(r[17]), "=&r"(r[18]), "=&r"(r[19]), "=&r"(r[20]), "=&r"(r[21]), "=&r"(r[22]), "=&r"(r[23]), "=&r"(r[24]), "=&r"(r[25]), "=&r"(r[26]), "=&r"(r[27]), "=&r"(r[28]), "=&r"(r[29]), "=&r"(r[30]), "=&r"(r[31])
+      : "r"(taddr), "r"(taddr + 16)
+      : "memory");
+}
+
 // Byte-wise e4m3 encoding of four digits 0..15 (one per byte).
 constexpr uint32_t kE4m3Lo8 = 0x44403800u;  // 3, 2, 1, 0
 constexpr uint32_t kE4m3Hi8 = 0x4E4C4A48u;  // 7, 6, 5, 4
@@ -233,6 +259,9 @@ __device__ __forceinline__ uint32_t lds32(uint32_t a) {
   asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(a));
   return v;
 }
+__device__ __forceinline__ void sts32(uint32_t a, uint32_t x) {
+  asm volatile("st.shared.b32 [%0], %1;" ::"r"(a), "r"(x) : "memory");
+}
 __device__ __forceinline__ void lds128(uint32_t a, uint32_t &x, uint32_t &y, uint32_t &z, uint32_t &w) {
   asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(x), "=r"(y), "=r"(z), "=r"(w) : "r"(a));
 }
@@ -241,42 +270,6 @@ __device__ __forceinline__ void sts64(uint32_t a, uint32_t x, uint32_t y) {
 }
 __device__ __forceinline__ void sts128(uint32_t a, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
   asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
-}
-
-// stage_hankel with compile-time sizes and 32-bit shared addresses (H, ext:
-// shared-window byte addresses): the same thread groups, each thread's rows
-// unrolled from one load of the ext words they span.  A thread's window
-// starts at word q = 2 u0 + par with u0 even, so it loads the 16-byte-aligned
-// words from q - par with 128-bit loads (the eight lanes of a row pair share
-// them, so a warp's load is one 64-byte wavefront) and takes word i + par by
-// a funnel shift.
-template <int L, int NT, int CORES>
-__device__ __forceinline__ void stage_hankel_ct(uint32_t H, uint32_t ext, int tid) {
-  constexpr int PAIRS = NT >> 3;
-  constexpr int RUN = (CORES + PAIRS - 1) / PAIRS;  // rows per thread and polynomial
-  constexpr int NW = (2 * RUN + 4 + 3) & ~3;         // the 2 RUN + 3 window words, plus one for par
-  static_assert(RUN % 2 == 0, "every thread's window starts on a 16-byte boundary");
-  static_assert(2 * (CORES - 1) + NW <= 128, "the loads stay inside one polynomial's 512-byte s_ext");
-  const int sh = tid & 3, par = (tid >> 2) & 1, u0 = (tid >> 3) * RUN;
-  if (u0 >= CORES) return;
-  const uint32_t sel = 0x3210u + 0x1111u * (uint32_t)sh;
-  const int b = 2 * u0;  // q - par, a multiple of 4
-  const int q = b + par;
-#pragma unroll
-  for (int j = 0; j < L; j++) {
-    uint32_t a[NW];
-#pragma unroll
-    for (int i = 0; i < NW; i += 4) lds128(ext + 512 * j + 4 * (b + i), a[i], a[i + 1], a[i + 2], a[i + 3]);
-    uint32_t w[2 * RUN + 3];
-#pragma unroll
-    for (int i = 0; i < 2 * RUN + 3; i++) w[i] = __funnelshift_rc(a[i], a[i + 1], 32u * (uint32_t)par);
-    const uint32_t h = H + (uint32_t)(j * CORES * 128) + 16 * (4 * q + sh);
-#pragma unroll
-    for (int r = 0; r < RUN; r++)
-      if (CORES % PAIRS == 0 || u0 + r < CORES)
-        sts128(h + 128 * r, __byte_perm(w[2 * r], w[2 * r + 1], sel), __byte_perm(w[2 * r + 1], w[2 * r + 2], sel),
-               __byte_perm(w[2 * r + 2], w[2 * r + 3], sel), __byte_perm(w[2 * r + 3], w[2 * r + 4], sel));
-  }
 }
 
 // The first `cores` Hankel core matrices of every j < L (H: cores * 128 bytes
