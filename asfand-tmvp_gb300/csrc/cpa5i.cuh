@@ -143,10 +143,10 @@ struct LayoutC {
   static constexpr int EXT = BM + C::L * BJ;
   static constexpr int ENG_END_OPS = EXT + C::L * EXJ;
   static constexpr int ENG_BYTES = ENG_END_OPS;
-  // the output ops' 16-bit values (R x 512 bytes), over the digit columns
-  // (the next instance's inputs are landing in H)
+  // the output ops' 16-bit values (R x 8 runs of 80 bytes), over the digit
+  // columns (the next instance's inputs are landing in H)
   static constexpr int VALS = BM;
-  static_assert(HAS_CT || HAS_MV || S::R * 512 <= C::L * BJ, "epilogue values fit the digit columns");
+  static_assert(HAS_CT || HAS_MV || S::R * 640 <= C::L * BJ, "epilogue values fit the digit columns");
   // ciphertext and message, read until the end of an instance: two buffers of
   // CTB bytes, so that the next instance's copies land beside them
   static constexpr int CTO = al16c(ENG + ENG_BYTES);
@@ -224,6 +224,13 @@ __device__ __forceinline__ void unpack8d(const uint8_t *base, int byte0, uint32_
 __device__ __forceinline__ uint32_t raw_sdigits4(uint32_t t) {
   const uint32_t s = (t >> 4) & 0x01010101u;
   return ((t & 0x0F0F0F0Fu) ^ (s * 15u)) + s * 0x81u;
+}
+
+// Four secrets -7 .. 7 (int8) as raw e4m3 bytes, sign and magnitude: worth
+// s * 2^-9 as the digits are, so that the accumulators hold x * 2^-18.
+__device__ __forceinline__ uint32_t raw_secrets4(uint32_t v) {
+  const uint32_t s = (v >> 7) & 0x01010101u;
+  return ((v & 0x0F0F0F0Fu) ^ (s * 15u)) + s * 0x81u;
 }
 
 // Radix-16 digit d (r16_digits) of eight W-bit coefficients X (four words of
@@ -315,6 +322,39 @@ __device__ __forceinline__ void stage_digits32(const uint8_t *sm, int src, uint3
   }
 }
 
+// 32 W-bit values (16-bit lanes of x, each below 2^W) as W words at dst.
+template <int W>
+__device__ __forceinline__ void pack32(uint32_t dst, const uint32_t (&x)[16]) {
+  uint32_t o[W + 1] = {};
+#pragma unroll
+  for (int k = 0; k < 16; k++) {
+    const uint32_t y = (x[k] & 0xFFFFu) + ((x[k] >> 16) << W);
+    const int bit = 2 * W * k, i = bit >> 5, sh = bit & 31;
+    o[i] |= y << sh;
+    if (sh + 2 * W > 32) o[i + 1] |= y >> (32 - sh);
+  }
+#pragma unroll
+  for (int i = 0; i < W; i++) sts32(dst + 4 * i, o[i]);
+}
+
+// 16-bit values of coefficients 32m .. 32m + 31 of polynomial p (epilogue
+// values: 80 bytes a run of 32, so that eight lanes' 128-bit loads differ in
+// banks).
+__device__ __forceinline__ constexpr int vals_off(int p, int m) { return 80 * (8 * p + m); }
+__device__ __forceinline__ void load_vals32(uint32_t src, uint32_t (&x)[16]) {
+#pragma unroll
+  for (int i = 0; i < 16; i += 4) lds128(src + 4 * i, x[i], x[i + 1], x[i + 2], x[i + 3]);
+}
+
+// Two int8 of v sign-extended to 16-bit lanes (SEL: per lane the byte and, with
+// bit 3 set, its sign replicated).
+template <int SEL>
+__device__ __forceinline__ uint32_t sext2(uint32_t v) {
+  uint32_t r;
+  asm("prmt.b32 %0, %1, 0, %2;" : "=r"(r) : "r"(v), "n"(SEL));
+  return r;
+}
+
 // Cluster launch control: asks for a CTA of this grid that has not been
 // launched yet, to run its work here instead.  The 16-byte answer lands at
 // resp and counts on mbar.
@@ -374,27 +414,30 @@ __device__ __forceinline__ void cpa5i_load(const CpaArgs &a, const unsigned inst
   }
 }
 
-// Digit sums.  An accumulator holds x * 2^-9 for an exact integer x with
-// |x| < 2^22, so adding 1.5 * 2^14 (24576) leaves x in the low bits of the
-// f32 pattern; the pattern of 24576.0 itself is 0 in its low 16 bits, which
-// are all that the results (mod 2^13 or less) need.  sum_d 16^d x_d is formed
-// in f32 by fused multiply-adds where it stays below 2^22 for every
-// admissible secret (exact: an integer below 2^24 in units of 2^-9), else the
-// digit of weight 256 joins as an integer.
+// Digit sums.  An accumulator holds x * 2^-18 for an exact integer x with
+// |x| < 2^22, so adding 1.5 * 2^5 (48) leaves x in the low bits of the f32
+// pattern; the pattern of 48.0 itself is 0 in its low 16 bits, which are all
+// that the results (mod 2^13 or less) need.  sum_d 16^d x_d is formed in f32 by
+// fused multiply-adds where it stays below 2^22 for every admissible secret
+// (exact: an integer below 2^24 in units of 2^-18), else the digit of weight
+// 256 joins as an integer.
 constexpr int digit_bound(int w) { return w == 13 ? 17 * 256 : (w == 9 ? 17 * 16 : (1 << w) - 1); }
 
-// Product p's share of the even (par 0) or odd (1) K steps of one coefficient,
-// from its accumulator columns f, in the low 16 bits.
+// Product p's share of the even (par 0) or odd (1) K steps of one coefficient
+// from its accumulator columns f, plus `add` (a small integer), in the low 16
+// bits.
 template <int OP, int SET>
-__device__ __forceinline__ uint32_t combine5(const uint32_t (&f)[2 * ShapeC<OP, SET>::NC4], int p, int par) {
+__device__ __forceinline__ uint32_t combine5(const uint32_t (&f)[2 * ShapeC<OP, SET>::NC4], int p, int par, int add) {
   using S = ShapeC<OP, SET>;
   const int c0 = S::col_base(p), D = S::digits(p), W = p < S::RA ? S::WA : S::WB;
   auto col = [&](int d) { return __uint_as_float(f[2 * (c0 + d) + par]); };
-  float x = col(0) + 24576.0f;
+  static_assert(digit_bound(13) * 7 < (1 << 15) && S::ROWS <= 512, "255 * 7 * 512 + add < 2^22");
+  float x = col(0) + (48.0f + (float)add / 262144.0f);
   if (D > 1) x = __fmaf_rn(16.0f, col(1), x);
   if (D < 3) return __float_as_uint(x);
-  if (digit_bound(W) * S::SMAX * S::ROWS < (1 << 22)) return __float_as_uint(__fmaf_rn(256.0f, col(2), x));
-  return __float_as_uint(x) + 256u * __float_as_uint(col(2) + 24576.0f);
+  if (digit_bound(W) * S::SMAX * S::ROWS + (1 << 13) < (1 << 22))
+    return __float_as_uint(__fmaf_rn(256.0f, col(2), x));
+  return __float_as_uint(x) + 256u * __float_as_uint(col(2) + 48.0f);
 }
 
 // The instances of a launch, from the CTA of kI5Threads threads that runs
@@ -513,12 +556,13 @@ __device__ __forceinline__ void cpa5i_run(const AT &at, uint8_t *sm) {
           }
         }
       }
-      ok = ok && small4(sb[0]) && small4(sb[1]);
+      // (CBD secrets are at most mu / 2 <= 5 in magnitude)
+      if (IS_DEC || OP == kMatvec) ok = ok && small4(sb[0]) && small4(sb[1]);
       if (OP == kKeygen) {
         sec8w[64 * j + 2 * g] = sb[0];
         sec8w[64 * j + 2 * g + 1] = sb[1];
       }
-      const uint32_t e0 = enc4<kFp8Tcgen05>(sb[0]), e1 = enc4<kFp8Tcgen05>(sb[1]);
+      const uint32_t e0 = raw_secrets4(sb[0]), e1 = raw_secrets4(sb[1]);
       const uint32_t nx = __shfl_sync(0xffffffffu, e0, (lane + 1) & 31);
       const uint32_t p0 = __byte_perm(e0, e1, 0x4321), p1 = __byte_perm(e1, nx, 0x4321);
       // word 63: s_ext[255] = s[0] keeps its sign; word 127: s_ext[511] = 0
@@ -620,8 +664,12 @@ __device__ __forceinline__ void cpa5i_run(const AT &at, uint8_t *sm) {
   }
   stage_hankel6<LO, L>(smem_u32(H), ext32, tid);
   fence_async_smem();  // generic-proxy writes -> visible to the tensor core
-  ok = __syncthreads_and(ok) != 0;
-  if (!ok && tid == 0 && a.err) atomicOr(a.err, 1);
+  if constexpr (IS_DEC || OP == kMatvec) {
+    ok = __syncthreads_and(ok) != 0;
+    if (!ok && tid == 0 && a.err) atomicOr(a.err, 1);
+  } else {
+    __syncthreads();
+  }
 
   // 3. the MMAs (one thread).  Coefficients and K steps come in blocks of 32:
   // coefficient block o takes step t through the 32 x 32 Hankel block
@@ -656,29 +704,6 @@ __device__ __forceinline__ void cpa5i_run(const AT &at, uint8_t *sm) {
     }
     umma_commit(mbar_mma);
   }
-  // The thread's coefficient k (block o = 4 hsel + q4 of 32; its warp reads
-  // tensor-memory lanes 32 q4 ..), and beside the MMAs what the epilogue needs
-  // of the inputs: the ciphertext's coefficient k, the message bit.
-  const int q4 = warp & 3, hsel = warp >> 2;
-  const int k = 128 * hsel + 32 * q4 + lane;
-  // W-bit field at bit `bit` of a 4-byte-aligned shared-memory stream
-  auto field = [&](int byte_off, int bit, int W) -> uint32_t {
-    const uint32_t *w = reinterpret_cast<const uint32_t *>(sm + byte_off) + (bit >> 5);
-    return __funnelshift_r(w[0], w[1], bit & 31) & ((1u << W) - 1u);
-  };
-
-  uint32_t cf[LO::HAS_CT ? S::R : 1], mk = 0;
-  if constexpr (IS_DEC) {  // c_m of each ciphertext
-#pragma unroll
-    for (int r = 0; r < S::R; r++)
-      cf[r] = field((int)cbuf + LO::CTO + r * LO::CTS + L * C::POLYCOMP, k * C::ET, C::ET);
-  }
-  if constexpr (LO::HAS_B) mk = (sm[LO::MSG + cbuf + (k >> 3)] >> (k & 7)) & 1u;
-  if constexpr (OP == kReenc) {
-#pragma unroll
-    for (int p = 0; p < L; p++) cf[p] = field((int)cbuf + LO::CTO + p * C::POLYCOMP, k * C::EP, C::EP);
-    cf[L] = field((int)cbuf + LO::CTO + L * C::POLYCOMP, k * C::ET, C::ET);
-  }
   // 4. accumulators: one warp polls the MMA barrier and the CLC answer, the
   // others wait in the CTA barrier.  The MMAs have read H and the other
   // ciphertext buffer was last read before this instance's barriers, so the
@@ -710,10 +735,37 @@ __device__ __forceinline__ void cpa5i_run(const AT &at, uint8_t *sm) {
   }
   const uint32_t next = *next_slot;
   tc_fence_after();
+  // The thread's coefficient k (block o = 4 hsel + q4 of 32; its warp reads
+  // tensor-memory lanes 32 q4 ..), and what the epilogue needs of the inputs:
+  // the ciphertext's coefficient k, the message bit.  (Read here: beside the
+  // MMAs, which read shared memory at full rate, the same loads made the
+  // re-encryption 299 instead of 285 us at 65536, by shuffles from one load a
+  // warp 303.)
+  const int q4 = warp & 3, hsel = warp >> 2;
+  const int k = 128 * hsel + 32 * q4 + lane;
+  const uint32_t ctb = smem_u32(sm) + cbuf + (uint32_t)LO::CTO;
+  constexpr int CMO = L * C::POLYCOMP;
+  auto field = [&](uint32_t off, int W) -> uint32_t {  // coefficient k of the W-bit stream at ctb + off
+    const uint32_t p = ctb + off + (uint32_t)(((W * k) >> 5) * 4);
+    return __funnelshift_r(lds32(p), lds32(p + 4), (W * k) & 31) & ((1u << W) - 1u);
+  };
+  uint32_t cf[LO::HAS_CT ? S::R : 1], mk = 0;
+  if constexpr (IS_DEC) {  // c_m of each ciphertext
+#pragma unroll
+    for (int r = 0; r < S::R; r++) cf[r] = field((uint32_t)(r * LO::CTS + CMO), C::ET);
+  }
+  if constexpr (LO::HAS_B) mk = (sm[LO::MSG + cbuf + (k >> 3)] >> (k & 7)) & 1u;
+  if constexpr (OP == kReenc) {
+#pragma unroll
+    for (int p = 0; p < L; p++) cf[p] = field((uint32_t)(p * C::POLYCOMP), C::EP);
+    cf[L] = field((uint32_t)CMO, C::ET);
+  }
   const uint32_t xch = smem_u32(sm + LO::XCH);
   // coefficient k of every product, in the low 16 bits (a.. the sums of an
   // accumulator's digit columns, see combine5)
   uint32_t val[S::R];
+  // the rounding constant that the op adds to every product
+  constexpr int ROUND = IS_DEC ? C::H2 : (OP == kMatvec ? 0 : C::H1);
   {
     const uint32_t t0 = tmem + ((uint32_t)(32 * q4) << 16);
     // odd steps first: block o' = q4 - 1 (hsel 0; block 7 negated for
@@ -724,7 +776,7 @@ __device__ __forceinline__ void cpa5i_run(const AT &at, uint8_t *sm) {
     tmem_ld_cols(t0 + (uint32_t)(2 * S::NC4 * hsel), f);
     const int od = (warp + 7) & 7;  // the block the odd steps belong to
 #pragma unroll
-    for (int p = 0; p < S::R; p++) odd[p] = combine5<OP, SET>(f, p, 1);
+    for (int p = 0; p < S::R; p++) odd[p] = combine5<OP, SET>(f, p, 1, 0);
     if (warp == 0) {
 #pragma unroll
       for (int p = 0; p < S::R; p++) odd[p] = 0u - odd[p];
@@ -733,7 +785,7 @@ __device__ __forceinline__ void cpa5i_run(const AT &at, uint8_t *sm) {
     for (int i = 0; i < LO::XWORDS; i++)
       sts32(xch + (uint32_t)((i * 256 + 32 * od + lane) * 4), __byte_perm(odd[2 * i], odd[2 * i + 1], 0x5410));
 #pragma unroll
-    for (int p = 0; p < S::R; p++) val[p] = combine5<OP, SET>(f, p, 0);
+    for (int p = 0; p < S::R; p++) val[p] = combine5<OP, SET>(f, p, 0, ROUND);
     tc_fence_before();  // the loads above come before the next instance's MMAs (its barriers lie between)
     __syncthreads();
 #pragma unroll
@@ -748,26 +800,26 @@ __device__ __forceinline__ void cpa5i_run(const AT &at, uint8_t *sm) {
     // with the message bit (c_m), as 16-bit values for the packing pass;
     // the MMAs are done, so the digit columns are free
     constexpr uint32_t qm = (1u << C::EQ) - 1u, pm = (1u << C::EP) - 1u;
-    uint16_t *vals = reinterpret_cast<uint16_t *>(sm + LO::VALS);
 #pragma unroll
     for (int p = 0; p < S::R; p++) {
       const uint32_t v = val[p];
+      uint16_t *at32 = reinterpret_cast<uint16_t *>(sm + LO::VALS + vals_off(p, warp)) + lane;
       if (p < L) {
-        vals[256 * p + k] = (uint16_t)(((v + C::H1) & qm) >> (C::EQ - C::EP));
+        *at32 = (uint16_t)((v & qm) >> (C::EQ - C::EP));
       } else {
-        vals[256 * p + k] = (uint16_t)(((v + C::H1 - (mk << (C::EP - 1))) & pm) >> (C::EP - C::ET));
+        *at32 = (uint16_t)(((v - (mk << (C::EP - 1))) & pm) >> (C::EP - C::ET));
       }
     }
     __syncthreads();  // the 16-bit values are complete
   }
 
   // 5. epilogues
-  constexpr uint32_t qmask = (1u << C::EQ) - 1u, pmask = (1u << C::EP) - 1u;
+  constexpr uint32_t pmask = (1u << C::EP) - 1u;
   if constexpr (OP == kDecrypt) {
     // m'_k = ((v_k + h2 - (c_m,k << (ep-et))) mod p) >> (ep-1): one bit per
     // thread, gathered into bytes by a ballot per warp
     const uint32_t v = val[0];
-    const uint32_t t = (v + C::H2 - (cf[0] << (C::EP - C::ET))) & pmask;
+    const uint32_t t = (v - (cf[0] << (C::EP - C::ET))) & pmask;
     const uint32_t bits = __ballot_sync(0xffffffffu, ((t >> (C::EP - 1)) & 1u) != 0u);
     uint8_t *mo = a.m_out + (size_t)inst * a.m_out_stride;
     if (lane < 4) mo[4 * (4 * hsel + q4) + lane] = (uint8_t)(bits >> (8 * lane));
@@ -778,7 +830,7 @@ __device__ __forceinline__ void cpa5i_run(const AT &at, uint8_t *sm) {
     for (int r = 0; r < S::R; r++) {
       if (r >= nvalid) break;
       const uint32_t v = val[r];
-      const uint32_t t = (v + C::H2 - (cf[r] << (C::EP - C::ET))) & pmask;
+      const uint32_t t = (v - (cf[r] << (C::EP - C::ET))) & pmask;
       const uint32_t bits = __ballot_sync(0xffffffffu, ((t >> (C::EP - 1)) & 1u) != 0u);
       uint8_t *mo = a.m_out + (inst0 + r) * a.m_out_stride;
       if (lane < 4) mo[4 * (4 * hsel + q4) + lane] = (uint8_t)(bits >> (8 * lane));
@@ -786,18 +838,14 @@ __device__ __forceinline__ void cpa5i_run(const AT &at, uint8_t *sm) {
     }
   } else if constexpr (OP == kReenc) {
     // round coefficient k of b' and encode that of v', compare with the ciphertext
-    uint32_t diff = 0;
+    uint32_t diff = 0, diffm = 0;
 #pragma unroll
     for (int p = 0; p < S::R; p++) {
       const uint32_t v = val[p];
-      if (p < L) {
-        const uint32_t w = ((v + C::H1) & qmask) >> (C::EQ - C::EP);
-        diff |= w ^ cf[p];
-      } else {
-        const uint32_t w = ((v + C::H1 - (mk << (C::EP - 1))) & pmask) >> (C::EP - C::ET);
-        diff |= w ^ cf[L];
-      }
+      if (p < L) diff |= (v >> (C::EQ - C::EP)) ^ cf[p];
+      else diffm = ((v - (mk << (C::EP - 1))) >> (C::EP - C::ET)) ^ cf[L];
     }
+    diff = (diff & pmask) | (diffm & ((1u << C::ET) - 1u));
     if (__any_sync(0xffffffffu, diff != 0u) && lane == 0) a.fail[inst] = 1;
   } else if constexpr (OP == kMatvec) {
     // coefficient k of every output polynomial, mod 2^eq
@@ -806,36 +854,39 @@ __device__ __forceinline__ void cpa5i_run(const AT &at, uint8_t *sm) {
 #pragma unroll
     for (int p = 0; p < L; p++) o[256 * p] = (uint16_t)(val[p] & m);
   } else if (OP == kEncrypt) {
-    // pack the 16-bit values eight at a time: b' at EP bits, c_m at ET bits
-    const uint16_t *vals = reinterpret_cast<const uint16_t *>(sm + LO::VALS);
-    for (int idx = tid; idx < S::R * 32; idx += NT) {
-      const int p = idx >> 5, grp = idx & 31;
-      const uint4 q = *reinterpret_cast<const uint4 *>(vals + 256 * p + 8 * grp);
-      const uint32_t W[4] = {q.x, q.y, q.z, q.w};
-      if (p < L) pack8(sm + LO::OUT + (32 * p + grp) * C::EP, W, C::EP);
-      else pack8(sm + LO::OUT + L * C::POLYCOMP + grp * C::ET, W, C::ET);
+    // pack the 16-bit values, 32 to a lane: b' at EP bits (warp 0), c_m at ET
+    // bits (warp 1)
+    const uint32_t out = smem_u32(sm + LO::OUT), vals = smem_u32(sm + LO::VALS);
+    uint32_t x[16];
+    if (warp == 0 && lane < 8 * L) {
+      load_vals32(vals + vals_off(0, lane), x);
+      pack32<C::EP>(out + 4 * C::EP * lane, x);
+    } else if (warp == 1 && lane < 8) {
+      load_vals32(vals + vals_off(L, lane), x);
+      pack32<C::ET>(out + L * C::POLYCOMP + 4 * C::ET * lane, x);
     }
     __syncthreads();
     copy16(a.ct_out + (size_t)inst * C::CT, sm + LO::OUT, C::CT);
   } else if (OP == kKeygen) {
     constexpr int bbytes = L * C::POLYCOMP;
     uint8_t *outb = sm + LO::OUT;
-    const uint16_t *vals = reinterpret_cast<const uint16_t *>(sm + LO::VALS);
-    for (int idx = tid; idx < L * 32; idx += NT) {
-      const int p = idx >> 5, grp = idx & 31;
-      const uint4 q = *reinterpret_cast<const uint4 *>(vals + 256 * p + 8 * grp);
-      const uint32_t W[4] = {q.x, q.y, q.z, q.w};
-      pack8(outb + (32 * p + grp) * C::EP, W, C::EP);
-    }
-    // secret key: 13-bit two's complement (Saber) or 2-bit (Sable) of sec8
-    constexpr int sw = C::SABLE ? 2 : C::EQ;
-    const int8_t *s8 = reinterpret_cast<const int8_t *>(sm + LO::SEC8);
-    for (int grp = tid; grp < L * 32; grp += NT) {
-      uint32_t Sv[4];
+    const uint32_t out = smem_u32(outb);
+    uint32_t x[16];
+    if (warp == 0 && lane < 8 * L) {
+      load_vals32(smem_u32(sm + LO::VALS) + vals_off(0, lane), x);
+      pack32<C::EP>(out + 4 * C::EP * lane, x);
+    } else if (warp == 1 && lane < 8 * L) {
+      // secret key: 13-bit two's complement (Saber) or 2-bit (Sable) of sec8,
+      // two int8 at a time sign-extended to 16-bit lanes
+      constexpr int sw = C::SABLE ? 2 : C::EQ;
+      const uint32_t s8 = smem_u32(sm + LO::SEC8) + 32 * lane;
 #pragma unroll
-      for (int i = 0; i < 4; i++)
-        Sv[i] = ((uint32_t)(int)s8[8 * grp + 2 * i] & 0xffffu) | ((uint32_t)(int)s8[8 * grp + 2 * i + 1] << 16);
-      pack8(outb + bbytes + grp * sw, Sv, sw);
+      for (int i = 0; i < 8; i++) {
+        const uint32_t v = lds32(s8 + 4 * i);
+        x[2 * i] = sext2<0x9180>(v) & (((1u << sw) - 1u) * 0x10001u);
+        x[2 * i + 1] = sext2<0xB3A2>(v) & (((1u << sw) - 1u) * 0x10001u);
+      }
+      pack32<sw>(out + bbytes + 4 * sw * lane, x);
     }
     __syncthreads();
     uint8_t *pko = a.pk_out + (size_t)inst * C::PK;
