@@ -23,13 +23,15 @@ SCHEMES = {"saber": "libref_saber.so", "sable": "libref_sable.so"}
 
 def reference_root() -> str:
     """Where the reference sources are read from: $TMVP_REFERENCE_ROOT, else
-    the recipe's own default (``make -C oracle/ref_build print-ref``)."""
+    the recipe's own default (``make -C oracle/ref_build print-ref``); "" if
+    that folder is empty or absent."""
     env = os.environ.get("TMVP_REFERENCE_ROOT")
     if env:
         return env
     r = subprocess.run(["make", "-s", "-C", os.path.join(_HERE, "ref_build"), "print-ref"],
                        capture_output=True, text=True)
-    return r.stdout.strip() if r.returncode == 0 else ""
+    root = r.stdout.strip() if r.returncode == 0 else ""
+    return root if root and os.path.isdir(root) and os.listdir(root) else ""
 
 
 def build(ref_root: str | None = None) -> bool:
