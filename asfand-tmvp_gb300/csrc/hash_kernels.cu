@@ -1,274 +1,390 @@
-// hash_kernels.cu — the Keccak stages of the batched KEM: one thread per
-// sponge, register-resident state, 8-byte global accesses.
+// hash_kernels.cu — the Keccak stages of the batched KEM, each written once
+// for the three forms of a sponge (hash_engine.cuh), and the planner that
+// spreads a launch's sponges over the GPU.
 //
 // Replaces the reference's single-block hash kernels and its 25-lane
 // shake128_gpu (TMVP-Saber/SABER-GPU/src/poly.cu:918-1114,
 // TMVP_SABLE/src/fips202.cu:409-668), which cap the batch at 1024 and rely
-// on implicit warp synchrony.  Every kernel here covers any batch size with a
-// 1-D grid and has no inter-thread communication.
+// on implicit warp synchrony.
 #include "hash_kernels.cuh"
-#include "keccak.cuh"
+
+#include <algorithm>
+
+#include "hash_engine.cuh"
 
 namespace tmvp {
 
-__device__ __forceinline__ void load_words(uint64_t *dst, const uint8_t *src, int nw) {
-  const uint64_t *s = reinterpret_cast<const uint64_t *>(src);
-#pragma unroll 4
-  for (int i = 0; i < nw; i++) dst[i] = s[i];
-}
+namespace {
 
-__device__ __forceinline__ void run_shake_job(const ShakeJob &J, size_t i) {
-  uint64_t seed[4];
-  load_words(seed, J.src + i * J.src_stride + J.src_off, 4);
-  if (J.prehash) {
-    // seed_A <- SHAKE-128(seed_A)[0:32] (Saber round-3 key generation)
-    uint64_t h[4];
-    shake128_32(h, 32, seed);
-#pragma unroll
-    for (int k = 0; k < 4; k++) seed[k] = h[k];
-    if (J.seed_out) {
-      uint64_t *so = reinterpret_cast<uint64_t *>(J.seed_out + i * J.seed_out_stride + J.seed_out_off);
-#pragma unroll
-      for (int k = 0; k < 4; k++) so[k] = seed[k];
-    }
+// ---- the stages: run<E>(e, role, i) makes sponge i of a role ---------------
+
+struct GenMatrix {
+  KemParams P;
+  const uint8_t *pk;
+  size_t pk_stride;
+  uint8_t *a_stream;
+  template <class E>
+  __device__ __forceinline__ void run(const E &e, int, size_t i) const {
+    const auto seed = e.load(pk + i * pk_stride + (size_t)P.l * P.polycompbytes, 4);
+    e.shake128(seed, a_stream + i * P.gm_bytes, P.gm_bytes);
   }
-  shake128_32(reinterpret_cast<uint64_t *>(J.out + i * J.out_stride), J.out_bytes, seed);
+};
+
+template <class E>
+__device__ __forceinline__ void dec_hash_ct(const E &e, const KemParams &P, const uint8_t *ct, uint8_t *hc, size_t i) {
+  e.store(hc + i * 32, e.sha3_256_mem(ct + i * P.ct_bytes, P.ct_bytes), 4);
 }
 
-__global__ void __launch_bounds__(128) k_shake_jobs(ShakeJob j0, ShakeJob j1, int n) {
-  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x, nal = warp_round((size_t)n);
-  if (t < (size_t)n) {
-    run_shake_job(j0, t);
-  } else if (j1.out && t >= nal && t < nal + n) {
-    run_shake_job(j1, t - nal);
-  }
+template <class E>
+__device__ __forceinline__ void dec_genmatrix(const E &e, const KemParams &P, const uint8_t *sk, uint8_t *a_stream,
+                                              size_t i) {
+  const auto seed = e.load(sk + i * P.sk_bytes + P.indcpa_sk_bytes + (size_t)P.l * P.polycompbytes, 4);
+  e.shake128(seed, a_stream + i * P.gm_bytes, P.gm_bytes);
 }
 
-// Encapsulation front (saber_enc, cuda_kernel.cu:116-127): thread i < n runs
-// m = H(coins), H(pk), kr = G(m || H(pk)) and the GenSecret stream
-// SHAKE-128(kr[32:64]); threads warp_round(n) + i expand GenMatrix from pk's
-// seed.
-__global__ void __launch_bounds__(128) k_enc_front(KemParams P, const uint8_t *pk,
-                                                    const uint8_t *coins, uint8_t *mbuf,
-                                                    uint8_t *kr, uint8_t *s_stream,
-                                                    uint8_t *a_stream, int n) {
-  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x, nal = warp_round((size_t)n);
-  if (t < (size_t)n) {
-    uint64_t c[4], buf[8], g[8];
-    load_words(c, coins + t * 32, 4);
-    sha3_256_32(buf, c);  // m
-    sha3_256_words(buf + 4, reinterpret_cast<const uint64_t *>(pk + t * P.pk_bytes), P.pk_bytes);
-    sha3_512_64(g, buf);
-    uint64_t *mo = reinterpret_cast<uint64_t *>(mbuf + t * 64);
-    uint64_t *ko = reinterpret_cast<uint64_t *>(kr + t * 64);
-#pragma unroll
-    for (int k = 0; k < 8; k++) {
-      mo[k] = buf[k];
-      ko[k] = g[k];
-    }
-    uint64_t seed[4] = {g[4], g[5], g[6], g[7]};
-    shake128_32(reinterpret_cast<uint64_t *>(s_stream + t * P.gs_bytes), P.gs_bytes, seed);
-  } else if (t >= nal && t < nal + n) {
-    const size_t i = t - nal;
-    uint64_t seed[4];
-    load_words(seed, pk + i * P.pk_bytes + (size_t)P.l * P.polycompbytes, 4);
-    shake128_32(reinterpret_cast<uint64_t *>(a_stream + i * P.gm_bytes), P.gm_bytes, seed);
-  }
+template <class E>
+__device__ __forceinline__ void dec_g_one(const E &e, const KemParams &P, const uint8_t *mbuf, uint8_t *kr,
+                                          uint8_t *s_stream, size_t i) {
+  const auto g = e.sha3_512_64(e.load(mbuf + i * 64, 8));
+  e.store(kr + i * 64, g, 8);
+  e.shake128(e.hi4(g), s_stream + i * P.gs_bytes, P.gs_bytes);
 }
 
-// Decapsulation step after decryption (saber_dec, cuda_kernel.cu:378-385):
-// kr = G(m' || H(pk)) and the GenSecret stream SHAKE-128(kr[32:64]).
-__device__ __forceinline__ void dec_g_one(const KemParams &P, const uint8_t *mbuf, uint8_t *kr,
-                                          uint8_t *s_stream, size_t t) {
-  uint64_t buf[8], g[8];
-  load_words(buf, mbuf + t * 64, 8);
-  sha3_512_64(g, buf);
-  uint64_t *ko = reinterpret_cast<uint64_t *>(kr + t * 64);
-#pragma unroll
-  for (int k = 0; k < 8; k++) ko[k] = g[k];
-  uint64_t seed[4] = {g[4], g[5], g[6], g[7]};
-  shake128_32(reinterpret_cast<uint64_t *>(s_stream + t * P.gs_bytes), P.gs_bytes, seed);
-}
-
-__global__ void __launch_bounds__(128) k_dec_g(KemParams P, const uint8_t *mbuf, uint8_t *kr,
-                                                uint8_t *s_stream, int n) {
-  size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < (size_t)n) dec_g_one(P, mbuf, kr, s_stream, t);
-}
-
-// GenMatrix stream of public key t (seed_A at the end of pk + t * pk_stride),
-// for callers that keep one expanded A per key (GenMatrix, saber_enc
-// cuda_kernel.cu:116-127).
-__global__ void __launch_bounds__(128) k_genmatrix(KemParams P, const uint8_t *pk, size_t pk_stride,
-                                                    uint8_t *a_stream, int n) {
-  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (size_t)n) return;
-  uint64_t seed[4];
-  load_words(seed, pk + t * pk_stride + (size_t)P.l * P.polycompbytes, 4);
-  shake128_32(reinterpret_cast<uint64_t *>(a_stream + t * P.gm_bytes), P.gm_bytes, seed);
-}
-
-// GenMatrix of instance t from the seed of the pk embedded in sk.
-__device__ __forceinline__ void dec_genmatrix_one(const KemParams &P, const uint8_t *sk, uint8_t *a_stream,
-                                                  size_t t) {
-  uint64_t seed[4];
-  load_words(seed, sk + t * P.sk_bytes + P.indcpa_sk_bytes + (size_t)P.l * P.polycompbytes, 4);
-  shake128_32(reinterpret_cast<uint64_t *>(a_stream + t * P.gm_bytes), P.gm_bytes, seed);
-}
-
-// H(c) of instance i.
-__device__ __forceinline__ void dec_hash_ct_one(const KemParams &P, const uint8_t *ct, uint8_t *hc, size_t i) {
-  uint64_t h[4];
-  sha3_256_words(h, reinterpret_cast<const uint64_t *>(ct + i * P.ct_bytes), P.ct_bytes);
-  uint64_t *o = reinterpret_cast<uint64_t *>(hc + i * 32);
-#pragma unroll
-  for (int w = 0; w < 4; w++) o[w] = h[w];
-}
-
-// Decapsulation front, independent of the decryption: GenMatrix from the seed
-// of the pk embedded in sk, and the ciphertext hash H(c) (saber_dec,
-// cuda_kernel.cu:383-384 and :447).  part 0: threads i < n expand GenMatrix,
-// threads warp_round(n) + i hash; part 1: GenMatrix only; part 2: H(c) only
-// (n threads each).
-__global__ void __launch_bounds__(128) k_dec_front(KemParams P, const uint8_t *sk,
-                                                    const uint8_t *ct, uint8_t *a_stream,
-                                                    uint8_t *hc, int n, int part) {
-  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x, nal = warp_round((size_t)n);
-  if (part != 0) {
-    if (t < (size_t)n) {
-      if (part == 1) dec_genmatrix_one(P, sk, a_stream, t);
-      else dec_hash_ct_one(P, ct, hc, t);
-    }
-    return;
-  }
-  if (t < (size_t)n)
-    dec_genmatrix_one(P, sk, a_stream, t);
-  else if (t >= nal && t < nal + n)
-    dec_hash_ct_one(P, ct, hc, t - nal);
-}
-
-// The same 2n sponges (GenMatrix, then H(c)) from a capped grid that leaves
-// room on every SM for the decryption beside it: threads stride over the
-// sponges, GenMatrix ones (the longer) first.  The stride is a multiple of
-// the block, so a warp's threads keep one role.
-__global__ void __launch_bounds__(128) k_dec_front_strided(KemParams P, const uint8_t *sk,
-                                                            const uint8_t *ct, uint8_t *a_stream,
-                                                            uint8_t *hc, int n) {
-  const size_t stride = (size_t)gridDim.x * blockDim.x, nal = warp_round((size_t)n);
-  for (size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x; t < nal + n; t += stride) {
-    if (t < (size_t)n)
-      dec_genmatrix_one(P, sk, a_stream, t);
-    else if (t >= nal)
-      dec_hash_ct_one(P, ct, hc, t - nal);
-  }
-}
-
-// Final key derivation.  Encapsulation (cuda_kernel.cu:185-186):
-// K = H(kr[0:32] || H(c)); hc, when given, holds H(c) already.  Decapsulation (cuda_kernel.cu:445-450, with the
-// FO selection done as specified): K = H((fail ? z : kr[0:32]) || H(c)), the
-// selection made with a mask so that it does not branch on `fail`.  sk of
-// instance t at sk + t * sk_stride (0: one key for every instance).
-__device__ __forceinline__ void final_key_one(const KemParams &P, const uint8_t *ct, const uint8_t *hc,
+template <class E>
+__device__ __forceinline__ void final_key_one(const E &e, const KemParams &P, const uint8_t *ct, const uint8_t *hc,
                                               const uint8_t *kr, const uint8_t *fail, const uint8_t *sk,
-                                              size_t sk_stride, uint8_t *ss, size_t t) {
-  uint64_t buf[8], k[4];
-  load_words(buf, kr + t * 64, 4);
-  if (fail) {
-    uint64_t mask = 0ull - (uint64_t)(fail[t] != 0);
-    uint64_t z[4];
-    load_words(z, sk + t * sk_stride + P.sk_bytes - 32, 4);
-#pragma unroll
-    for (int w = 0; w < 4; w++) buf[w] ^= mask & (buf[w] ^ z[w]);
+                                              size_t sk_stride, uint8_t *ss, size_t i) {
+  auto k = e.load(kr + i * 64, 4);
+  if (fail) k = e.sel4(k, e.load(sk + i * sk_stride + P.sk_bytes - 32, 4), fail[i] != 0);
+  const auto h = hc ? e.load(hc + i * 32, 4) : e.sha3_256_mem(ct + i * P.ct_bytes, P.ct_bytes);
+  e.store(ss + i * 32, e.template sha3_256<8>(e.cat4(k, h)), 4);
+}
+
+struct DecFront {  // role 0: GenMatrix, role 1: H(c)
+  KemParams P;
+  const uint8_t *sk, *ct;
+  uint8_t *a_stream, *hc;
+  template <class E>
+  __device__ __forceinline__ void run(const E &e, int role, size_t i) const {
+    if (role == 0) dec_genmatrix(e, P, sk, a_stream, i);
+    else dec_hash_ct(e, P, ct, hc, i);
   }
-  if (hc)
-    load_words(buf + 4, hc + t * 32, 4);
-  else
-    sha3_256_words(buf + 4, reinterpret_cast<const uint64_t *>(ct + t * P.ct_bytes), P.ct_bytes);
-  sha3_256_64(k, buf);
-  uint64_t *o = reinterpret_cast<uint64_t *>(ss + t * 32);
-#pragma unroll
-  for (int w = 0; w < 4; w++) o[w] = k[w];
-}
+};
 
-__global__ void __launch_bounds__(128) k_final_key(KemParams P, const uint8_t *ct,
-                                                    const uint8_t *hc, const uint8_t *kr,
-                                                    const uint8_t *fail, const uint8_t *sk,
-                                                    size_t sk_stride, uint8_t *ss, int n) {
-  size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < (size_t)n) final_key_one(P, ct, hc, kr, fail, sk, sk_stride, ss, t);
-}
-
-// ---- mixed-parameter decapsulation: one launch per stage over a group table
-
-__device__ __forceinline__ int hash_group(const HashGroup *T, int ng, int gi) {
-  int lo = 0, hi = ng - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (gi >= T[mid].first) lo = mid;
-    else hi = mid - 1;
+struct DecG {
+  KemParams P;
+  const uint8_t *mbuf;
+  uint8_t *kr, *s_stream;
+  template <class E>
+  __device__ __forceinline__ void run(const E &e, int, size_t i) const {
+    dec_g_one(e, P, mbuf, kr, s_stream, i);
   }
-  return lo;
+};
+
+struct FinalKey {
+  KemParams P;
+  const uint8_t *ct, *hc, *kr, *fail, *sk;
+  size_t sk_stride;
+  uint8_t *ss;
+  template <class E>
+  __device__ __forceinline__ void run(const E &e, int, size_t i) const {
+    final_key_one(e, P, ct, hc, kr, fail, sk, sk_stride, ss, i);
+  }
+};
+
+struct EncFront {  // role 0: GenMatrix, role 1: the chain to the GenSecret stream
+  KemParams P;
+  const uint8_t *pk, *coins;
+  uint8_t *mbuf, *kr, *s_stream, *a_stream;
+  template <class E>
+  __device__ __forceinline__ void run(const E &e, int role, size_t i) const {
+    if (role == 0) {
+      const auto seed = e.load(pk + i * P.pk_bytes + (size_t)P.l * P.polycompbytes, 4);
+      e.shake128(seed, a_stream + i * P.gm_bytes, P.gm_bytes);
+      return;
+    }
+    const auto m = e.template sha3_256<4>(e.load(coins + i * 32, 4));
+    const auto buf = e.cat4(m, e.sha3_256_mem(pk + i * P.pk_bytes, P.pk_bytes));
+    e.store(mbuf + i * 64, buf, 8);
+    const auto g = e.sha3_512_64(buf);
+    e.store(kr + i * 64, g, 8);
+    e.shake128(e.hi4(g), s_stream + i * P.gs_bytes, P.gs_bytes);
+  }
+};
+
+struct ShakeJobs {
+  ShakeJob j[2];
+  template <class E>
+  __device__ __forceinline__ void run(const E &e, int role, size_t i) const {
+    const ShakeJob &J = j[role];
+    auto seed = e.load(J.src + i * J.src_stride + J.src_off, 4);
+    if (J.prehash) {  // seed_A <- SHAKE-128(seed_A)[0:32] (Saber round-3 key generation)
+      seed = e.shake128_first(seed);
+      if (J.seed_out) e.store(J.seed_out + i * J.seed_out_stride + J.seed_out_off, seed, 4);
+    }
+    e.shake128(seed, J.out + i * J.out_stride, J.out_bytes);
+  }
+};
+
+struct KpFinal {
+  KemParams P;
+  const uint8_t *pk;
+  uint8_t *sk;
+  const uint8_t *coins;
+  template <class E>
+  __device__ __forceinline__ void run(const E &e, int, size_t i) const {
+    const auto h = e.sha3_256_mem(pk + i * P.pk_bytes, P.pk_bytes);
+    e.store(sk + i * P.sk_bytes + P.sk_bytes - 64, e.cat4(h, e.load(coins + i * 96 + 64, 4)), 8);
+  }
+};
+
+// Mixed-parameter stages: global sponge gi belongs to the group whose range
+// holds it.
+struct MixBase {
+  const HashGroup *T;
+  int ng;
+  __device__ __forceinline__ const HashGroup &group(size_t gi) const {
+    int lo = 0, hi = ng - 1;
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if ((int)gi >= T[mid].first) lo = mid;
+      else hi = mid - 1;
+    }
+    return T[lo];
+  }
+};
+struct MixFront : MixBase {
+  template <class E>
+  __device__ __forceinline__ void run(const E &e, int role, size_t gi) const {
+    const HashGroup &G = group(gi);
+    const size_t i = gi - (size_t)G.first;
+    if (role == 0) dec_genmatrix(e, G.P, G.sk, G.a_stream, i);
+    else dec_hash_ct(e, G.P, G.ct, G.hc, i);
+  }
+};
+struct MixG : MixBase {
+  template <class E>
+  __device__ __forceinline__ void run(const E &e, int, size_t gi) const {
+    const HashGroup &G = group(gi);
+    dec_g_one(e, G.P, G.mbuf, G.kr, G.s_stream, gi - (size_t)G.first);
+  }
+};
+struct MixFinal : MixBase {
+  template <class E>
+  __device__ __forceinline__ void run(const E &e, int, size_t gi) const {
+    const HashGroup &G = group(gi);
+    final_key_one(e, G.P, G.ct, G.hc, G.kr, G.fail, G.sk, (size_t)G.P.sk_bytes, G.ss, gi - (size_t)G.first);
+  }
+};
+
+// Blocks of 128 threads, one warp on each of an SM's four sub-partitions; of
+// one warp in a launch that has only the warp form (few sponges then spread
+// over all SMs: four on one SM share its shuffle unit, 51.2 against 49.2 us
+// for 17 LightSaber encapsulations).
+// The segment, form and role depend on blockIdx alone.  Past the end of a
+// segment the pair and warp forms repeat its last sponge (their shuffles need
+// every thread) and store nothing.
+template <class R>
+__global__ void __launch_bounds__(kHashBlock) k_sponges(const __grid_constant__ SpongePlan S,
+                                                        const __grid_constant__ R r) {
+  int k = 0;
+  while (k + 1 < S.nseg && blockIdx.x >= S.seg[k + 1].block0) k++;
+  const unsigned b = blockIdx.x - S.seg[k].block0, count = S.seg[k].count, first = S.seg[k].first;
+  const int role = S.seg[k].role;
+  switch (S.seg[k].form) {
+    case kHashThread: {
+      const unsigned i = b * kHashBlock + threadIdx.x;
+      if (i < count) r.run(ThreadSponge{}, role, first + i);
+      break;
+    }
+    case kHashPair: {
+      const unsigned i = b * (kHashBlock / 2) + (threadIdx.x >> 1);
+      const bool live = i < count;
+      r.run(PairSponge{(int)(threadIdx.x & 1), live}, role, first + (live ? i : count - 1));
+      break;
+    }
+    default: {
+      const int lane = (int)(threadIdx.x & 31);
+      const unsigned i = b * (blockDim.x >> 5) + (threadIdx.x >> 5);
+      const bool live = i < count;
+      r.run(WarpSponge{lane, live, warp_keccak_lane(lane)}, role, first + (live ? i : count - 1));
+    }
+  }
 }
 
-// part 1: GenMatrix of every instance; part 2: H(c); part 0: both, threads
-// warp_round(total) + i hashing.
-__global__ void __launch_bounds__(128) k_mix_front(const HashGroup *T, int ng, int total, int part) {
-  int gi = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  bool gen = part == 1;
-  if (part == 0) {
-    const int tal = (int)warp_round((size_t)total);
-    gen = gi < total;
-    if (!gen && (gi < tal || gi >= tal + total)) return;
-    if (!gen) gi -= tal;
-  } else if (gi >= total) {
+unsigned per_block(int form) {
+  return form == kHashThread ? kHashBlock : (form == kHashPair ? kHashBlock / 2 : kHashBlock / 32);
+}
+
+template <class R>
+cudaError_t launch_sponges(const SpongePlan &S, const R &r, cudaStream_t s) {
+  if (S.blocks == 0) return cudaSuccess;
+  auto fn = k_sponges<R>;
+  if (S.smem > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S.smem);
+    if (e != cudaSuccess) return e;
+  }
+  fn<<<S.blocks, S.threads, S.smem, s>>>(S, r);
+  return cudaGetLastError();
+}
+
+template <class R>
+cudaError_t launch_sponges(const HashCfg &cfg, const SpongeRole *roles, int nroles, const R &r, cudaStream_t s,
+                           cudaStream_t s2) {
+  SpongePlan S[2];
+  plan_sponges(cfg, roles, nroles, S);
+  for (SpongePlan &T : S) {
+    bool warp_only = true;
+    for (int k = 0; k < T.nseg; k++) warp_only = warp_only && T.seg[k].form == kHashWarp;
+    T.threads = warp_only ? 32 : kHashBlock;
+    if (warp_only) {
+      T.blocks = 0;
+      for (int k = 0; k < T.nseg; k++) {
+        T.seg[k].block0 = T.blocks;
+        T.blocks += T.seg[k].count;
+      }
+    }
+  }
+  const cudaError_t e = launch_sponges(S[0], r, s);
+  return e != cudaSuccess ? e : launch_sponges(S[1], r, s2);
+}
+
+}  // namespace
+
+// Adds role r's sponges [first, first + count) in `form` to S.
+static void add_seg(SpongePlan &S, int role, int form, size_t first, size_t count) {
+  if (!count) return;
+  S.seg[S.nseg++] = SpongeSeg{role, form, S.blocks, (unsigned)first, (unsigned)count};
+  S.blocks += (unsigned)((count + per_block(form) - 1) / per_block(form));
+}
+
+// Shared memory that leaves room for at most `blocks` blocks per SM (228 KB,
+// 1 KB of it per block reserved).
+static unsigned smem_limit(int blocks) { return blocks <= 1 ? 117000u : (unsigned)(227 * 1024 / (blocks + 1)); }
+
+bool sponges_split(const HashCfg &cfg, size_t n) {
+  return !cfg.limits && n >= (size_t)128 * cfg.sms && n < (size_t)192 * cfg.sms;
+}
+
+// Why the lines lie where they do (152 SMs, 608 sub-partitions; a sponge of 23
+// permutations):
+//  * A permutation's 4300 integer instructions fill a sub-partition's integer
+//    pipe from one thread-form warp on (92% of it; 99% from two), so a launch
+//    takes as long as its fullest sub-partition: 109 us per thread-form warp
+//    there.  128-thread blocks put one warp on each of an SM's four; with
+//    64-thread blocks, 16384 x (23 + 9) permutations took 209 us, with 128 147.
+//  * One warp a sponge takes 47 us up to about 2.75 sponges a sub-partition,
+//    two threads a sponge 67 us up to 16, one thread 109 us up to 32: the
+//    forms' lines.  Past whole rounds of 32, the rest goes the same way beside
+//    them: 20011 sponges in 122 us instead of 206.
+//  * Two roles side by side: longest first, and few blocks resident, so that
+//    an SM that finishes early takes the next block instead of all being
+//    placed at the start: with one block per SM 16384 x (23 + 9) takes 135
+//    us; with two per SM 32768 345 -> 266 and 65536 530 -> 502 (one: 272, 517).
+//  * Just above one round (up to 1.5) the longer role's thread-form blocks run
+//    alone at one per SM and the rest as a second launch beside them: as one
+//    launch, four SMs get two of those blocks (key generation of 20011: 386 us,
+//    as two 324).
+void plan_sponges(const HashCfg &cfg, const SpongeRole *roles, int nroles, SpongePlan (&S)[2]) {
+  S[0] = SpongePlan{};
+  S[1] = SpongePlan{};
+  int order[2] = {0, 1};
+  if (nroles == 2 && roles[1].perms > roles[0].perms) std::swap(order[0], order[1]);  // longest first
+  if (cfg.limits) {
+    size_t total = 0;
+    for (int r = 0; r < nroles; r++) total += roles[r].n;
+    const bool short_sponges = nroles == 1 && roles[0].perms <= 10;
+    const int form = (short_sponges ? 4 * total : total) <= cfg.warp_max   ? kHashWarp
+                     : (short_sponges ? 2 * total : total) <= cfg.pair_max ? kHashPair
+                                                                           : kHashThread;
+    for (int k = 0; k < nroles; k++) add_seg(S[0], roles[order[k]].id, form, 0, roles[order[k]].n);
+    if (cfg.cap > 0) S[0].smem = smem_limit(cfg.cap);
     return;
   }
-  const HashGroup &G = T[hash_group(T, ng, gi)];
-  const size_t i = (size_t)(gi - G.first);
-  if (gen) dec_genmatrix_one(G.P, G.sk, G.a_stream, i);
-  else dec_hash_ct_one(G.P, G.ct, G.hc, i);
-}
-
-__global__ void __launch_bounds__(128) k_mix_g(const HashGroup *T, int ng, int total) {
-  const int gi = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  if (gi >= total) return;
-  const HashGroup &G = T[hash_group(T, ng, gi)];
-  dec_g_one(G.P, G.mbuf, G.kr, G.s_stream, (size_t)(gi - G.first));
-}
-
-__global__ void __launch_bounds__(128) k_mix_final(const HashGroup *T, int ng, int total) {
-  const int gi = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  if (gi >= total) return;
-  const HashGroup &G = T[hash_group(T, ng, gi)];
-  final_key_one(G.P, G.ct, G.hc, G.kr, G.fail, G.sk, (size_t)G.P.sk_bytes, G.ss, (size_t)(gi - G.first));
-}
-
-// Key-generation tail: sk[SK-64 : SK-32] = H(pk), sk[SK-32 : SK] = z.
-__global__ void __launch_bounds__(128) k_kp_final(KemParams P, const uint8_t *pk, uint8_t *sk,
-                                                   const uint8_t *coins, int n) {
-  size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (size_t)n) return;
-  uint64_t h[4], z[4];
-  sha3_256_words(h, reinterpret_cast<const uint64_t *>(pk + t * P.pk_bytes), P.pk_bytes);
-  load_words(z, coins + t * 96 + 64, 4);
-  uint64_t *o = reinterpret_cast<uint64_t *>(sk + t * P.sk_bytes + P.sk_bytes - 64);
-#pragma unroll
-  for (int w = 0; w < 4; w++) {
-    o[w] = h[w];
-    o[4 + w] = z[w];
+  const size_t W = 4 * (size_t)cfg.sms;  // sub-partitions
+  const bool split = nroles == 2 && sponges_split(cfg, roles[order[0]].n);
+  size_t warps = 0;  // sponges in the warp form so far
+  for (int k = 0; k < nroles; k++) {
+    const SpongeRole &r = roles[order[k]];
+    const size_t full = r.n / (32 * W) * (32 * W), rest = r.n - full;
+    int form = kHashThread;
+    if (warps + rest <= (full ? 9 * W / 4 : 11 * W / 4)) form = kHashWarp;
+    else if (rest <= 16 * W) form = kHashPair;
+    if (form == kHashWarp) warps += rest;
+    add_seg(S[split && k == 1], r.id, kHashThread, 0, full);
+    add_seg(S[split && (k == 1 || form != kHashThread)], r.id, form, full, rest);
+    if (nroles == 2 && k == 0 && (full || form == kHashThread)) S[0].smem = smem_limit(cfg.cap > 0 ? cfg.cap : (full && !split ? 2 : 1));
   }
 }
 
-// Standalone SHA3-256 / SHA3-512 / SHAKE-128 over a batch (used by tests and
-// by the single-instance API).
-__global__ void k_sha3_256_batch(const uint8_t *in, int inbytes, uint8_t *out, int n) {
-  size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (size_t)n) return;
-  uint64_t h[4];
-  sha3_256_words(h, reinterpret_cast<const uint64_t *>(in + t * inbytes), inbytes);
-  uint64_t *o = reinterpret_cast<uint64_t *>(out + t * 32);
-#pragma unroll
-  for (int w = 0; w < 4; w++) o[w] = h[w];
+cudaError_t launch_dec_front(const HashCfg &cfg, const KemParams &P, const uint8_t *sk, const uint8_t *ct,
+                             uint8_t *a_stream, uint8_t *hc, size_t n, bool with_gm, cudaStream_t s, cudaStream_t s2) {
+  const SpongeRole roles[2] = {{n, gm_perms(P), 0}, {n, sha3_256_perms(P.ct_bytes), 1}};
+  return launch_sponges(cfg, with_gm ? roles : roles + 1, with_gm ? 2 : 1, DecFront{P, sk, ct, a_stream, hc}, s, s2);
+}
+
+cudaError_t launch_dec_g(const HashCfg &cfg, const KemParams &P, const uint8_t *mbuf, uint8_t *kr, uint8_t *s_stream,
+                         size_t n, cudaStream_t s) {
+  const SpongeRole role{n, 1 + gs_perms(P)};
+  return launch_sponges(cfg, &role, 1, DecG{P, mbuf, kr, s_stream}, s, s);
+}
+
+cudaError_t launch_final_key(const HashCfg &cfg, const KemParams &P, const uint8_t *ct, const uint8_t *hc,
+                             const uint8_t *kr, const uint8_t *fail, const uint8_t *sk, size_t sk_stride, uint8_t *ss,
+                             size_t n, cudaStream_t s) {
+  const SpongeRole role{n, 1 + (hc ? 0 : sha3_256_perms(P.ct_bytes))};
+  return launch_sponges(cfg, &role, 1, FinalKey{P, ct, hc, kr, fail, sk, sk_stride, ss}, s, s);
+}
+
+cudaError_t launch_enc_front(const HashCfg &cfg, const KemParams &P, const uint8_t *pk, const uint8_t *coins,
+                             uint8_t *mbuf, uint8_t *kr, uint8_t *s_stream, uint8_t *a_stream, size_t n, bool with_gm,
+                             cudaStream_t s, cudaStream_t s2) {
+  const SpongeRole roles[2] = {{n, gm_perms(P), 0}, {n, 2 + sha3_256_perms(P.pk_bytes) + gs_perms(P), 1}};
+  return launch_sponges(cfg, with_gm ? roles : roles + 1, with_gm ? 2 : 1, EncFront{P, pk, coins, mbuf, kr, s_stream, a_stream}, s, s2);
+}
+
+cudaError_t launch_genmatrix(const HashCfg &cfg, const KemParams &P, const uint8_t *pk, size_t pk_stride,
+                             uint8_t *a_stream, size_t n, cudaStream_t s) {
+  const SpongeRole role{n, gm_perms(P)};
+  return launch_sponges(cfg, &role, 1, GenMatrix{P, pk, pk_stride, a_stream}, s, s);
+}
+
+cudaError_t launch_shake_jobs(const HashCfg &cfg, const ShakeJob &j0, const ShakeJob &j1, size_t n, cudaStream_t s,
+                              cudaStream_t s2) {
+  const SpongeRole roles[2] = {{n, (j0.out_bytes + 167) / 168 + j0.prehash, 0},
+                               {n, (j1.out_bytes + 167) / 168 + j1.prehash, 1}};
+  return launch_sponges(cfg, roles, 2, ShakeJobs{{j0, j1}}, s, s2);
+}
+
+cudaError_t launch_kp_final(const HashCfg &cfg, const KemParams &P, const uint8_t *pk, uint8_t *sk,
+                            const uint8_t *coins, size_t n, cudaStream_t s) {
+  const SpongeRole role{n, sha3_256_perms(P.pk_bytes)};
+  return launch_sponges(cfg, &role, 1, KpFinal{P, pk, sk, coins}, s, s);
+}
+
+cudaError_t launch_mix_front(const HashCfg &cfg, const HashGroup *T, int ng, size_t total, int gm, int h,
+                             cudaStream_t s, cudaStream_t s2) {
+  const SpongeRole roles[2] = {{total, gm, 0}, {total, h, 1}};
+  MixFront r;
+  r.T = T;
+  r.ng = ng;
+  return launch_sponges(cfg, roles, 2, r, s, s2);
+}
+
+cudaError_t launch_mix_g(const HashCfg &cfg, const HashGroup *T, int ng, size_t total, int perms, cudaStream_t s) {
+  const SpongeRole role{total, perms};
+  MixG r;
+  r.T = T;
+  r.ng = ng;
+  return launch_sponges(cfg, &role, 1, r, s, s);
+}
+
+cudaError_t launch_mix_final(const HashCfg &cfg, const HashGroup *T, int ng, size_t total, cudaStream_t s) {
+  const SpongeRole role{total, 1};
+  MixFinal r;
+  r.T = T;
+  r.ng = ng;
+  return launch_sponges(cfg, &role, 1, r, s, s);
 }
 
 // dst[i * words + w] = src[w] for i < n (16-byte words): one key's bytes and

@@ -1,5 +1,8 @@
-// hash_kernels.cuh — declarations of the Keccak-stage kernels.
+// hash_kernels.cuh — the Keccak stages of the batched KEM: how a launch's
+// sponges are spread over the GPU, and the launches.
 #pragma once
+#include <cuda_runtime.h>
+
 #include <cstddef>
 #include <cstdint>
 
@@ -22,81 +25,76 @@ struct ShakeJob {
   size_t seed_out_stride, seed_out_off;
 };
 
-// The form of a Keccak launch.  One thread per sponge (this file's kernels)
-// keeps a warp's share of the integer pipe busy: ~4.7 us per permutation
-// however idle the GPU is, and the best rate once the pipe is full.  One warp
-// per sponge (the _w kernels): ~2.1 us per permutation until its shuffles
-// fill the SMs (~1 K GenMatrix sponges).  Two threads per sponge (the _p
-// kernels): ~3.3 us per permutation up to ~10 K sponges, the thread form's
-// integer work per sponge with twice its warps.  Launches of short sponges
-// (G, the final key, the key-generation tail: 1-10 permutations) count four
-// times against the warp form's limit and twice against the pair form's:
-// beside the other stages of a pass they lose there sooner (at batch 32768,
-// G and the final key in the pair form: 0.662 against 0.650 ms per pass,
-// while a GenMatrix + H(c) front of 32768 sponges gains: 0.352 against 0.369
-// ms at batch 16384).  kWarpHashDefault / kPairHashDefault are the limits a
-// context starts with (tmvp_ctx_set_warp_hash / _pair_hash).
-constexpr size_t kWarpHashDefault = 1024, kPairHashDefault = 32768;
+// The forms of a sponge: one thread, one warp, or two threads (hash_engine.cuh).
 enum HashForm { kHashThread, kHashWarp, kHashPair };
-inline HashForm hash_form_for(size_t sponges, bool short_sponges, size_t warp_max, size_t pair_max) {
-  if ((short_sponges ? 4 * sponges : sponges) <= warp_max) return kHashWarp;
-  if ((short_sponges ? 2 * sponges : sponges) <= pair_max) return kHashPair;
-  return kHashThread;
-}
 
-// Kernels with two sponge roles over n instances start the second role at
-// thread warp_round(n), so that no warp runs both roles: their loops differ
-// in length, and a warp holding both would run one after the other.  Their
-// grids cover warp_round(n) + n threads.
-__host__ __device__ inline size_t warp_round(size_t n) { return (n + 31) & ~(size_t)31; }
+// What a launch may use.  sms: SMs of the GPU.  The defaults let the planner
+// choose per role; with `limits`, the caller's own (tmvp_ctx_set_warp_hash /
+// _pair_hash), a launch of at most warp_max sponges runs one warp per sponge,
+// else of at most pair_max two threads per sponge, else one thread (short
+// sponges counting four times against the first and twice against the second).
+// cap: most 128-thread blocks per SM of a decapsulation front (0: the planner's).
+constexpr size_t kWarpHashDefault = 1024, kPairHashDefault = 32768;
+struct HashCfg {
+  int sms;
+  bool limits = false;
+  size_t warp_max = kWarpHashDefault, pair_max = kPairHashDefault;
+  int cap = 0;
+};
 
-__global__ void k_shake_jobs(ShakeJob j0, ShakeJob j1, int n);
-__global__ void k_enc_front(KemParams P, const uint8_t *pk, const uint8_t *coins, uint8_t *mbuf,
-                            uint8_t *kr, uint8_t *s_stream, uint8_t *a_stream, int n);
-__global__ void k_dec_g(KemParams P, const uint8_t *mbuf, uint8_t *kr, uint8_t *s_stream, int n);
-__global__ void k_genmatrix(KemParams P, const uint8_t *pk, size_t pk_stride, uint8_t *a_stream, int n);
-__global__ void k_replicate16(uint4 *dst, const uint4 *src, int words, size_t n);
-__global__ void k_final_key(KemParams P, const uint8_t *ct, const uint8_t *hc, const uint8_t *kr,
-                            const uint8_t *fail, const uint8_t *sk, size_t sk_stride, uint8_t *ss, int n);
-__global__ void k_dec_front(KemParams P, const uint8_t *sk, const uint8_t *ct, uint8_t *a_stream,
-                            uint8_t *hc, int n, int part);
-__global__ void k_dec_front_strided(KemParams P, const uint8_t *sk, const uint8_t *ct, uint8_t *a_stream,
-                                    uint8_t *hc, int n);
-__global__ void k_kp_final(KemParams P, const uint8_t *pk, uint8_t *sk, const uint8_t *coins,
-                           int n);
-__global__ void k_sha3_256_batch(const uint8_t *in, int inbytes, uint8_t *out, int n);
+// A launch's sponges: role r's sponges [first, first + count) in `form`, from
+// block block0 on.  Blocks start in order, so segments go longest role first.
+struct SpongeSeg {
+  int role, form;
+  unsigned block0, first, count;
+};
+struct SpongePlan {
+  int nseg;
+  unsigned blocks, threads, smem;  // threads: 128, or 32 with only the warp form
+  SpongeSeg seg[8];
+};
+struct SpongeRole {
+  size_t n;
+  int perms;   // Keccak-f per sponge
+  int id = 0;  // the stage's name for the role
+};
+constexpr unsigned kHashBlock = 128;
+// One or two roles over the GPU: S[0] and S[1] (empty unless sponges_split),
+// two launches that run side by side.
+void plan_sponges(const HashCfg &cfg, const SpongeRole *roles, int nroles, SpongePlan (&S)[2]);
+// Whether a launch of two roles over n instances becomes two: the two-role
+// launches below put the second on s2 (which the caller forks from and joins
+// to s).
+bool sponges_split(const HashCfg &cfg, size_t n);
 
-// The same stages with one warp per sponge (hash_warp.cu): sponge w of a
-// launch is block w of kWarpHashBlock threads, warp_blocks(sponges) blocks.
-constexpr unsigned kWarpHashBlock = 32;
-inline unsigned warp_blocks(size_t sponges) { return (unsigned)sponges; }
-__global__ void k_dec_front_w(KemParams P, const uint8_t *sk, const uint8_t *ct, uint8_t *a_stream, uint8_t *hc,
-                              int n, int part);
-__global__ void k_dec_g_w(KemParams P, const uint8_t *mbuf, uint8_t *kr, uint8_t *s_stream, int n);
-__global__ void k_final_key_w(KemParams P, const uint8_t *ct, const uint8_t *hc, const uint8_t *kr,
-                              const uint8_t *fail, const uint8_t *sk, size_t sk_stride, uint8_t *ss, int n);
-__global__ void k_enc_front_w(KemParams P, const uint8_t *pk, const uint8_t *coins, uint8_t *mbuf, uint8_t *kr,
-                              uint8_t *s_stream, uint8_t *a_stream, int n, int with_gm);
-__global__ void k_genmatrix_w(KemParams P, const uint8_t *pk, size_t pk_stride, uint8_t *a_stream, int n);
-__global__ void k_shake_jobs_w(ShakeJob j0, ShakeJob j1, int n);
-__global__ void k_kp_final_w(KemParams P, const uint8_t *pk, uint8_t *sk, const uint8_t *coins, int n);
-
-// The same stages with two threads per sponge (hash_pair.cu): thread t holds
-// half t & 1 of sponge t >> 1; kernels with two roles start the second at
-// thread warp_round(2n).  Grids of pair_blocks(threads) blocks of
-// kPairHashBlock.
-constexpr unsigned kPairHashBlock = 128;
-inline unsigned pair_blocks(size_t threads) { return (unsigned)((threads + kPairHashBlock - 1) / kPairHashBlock); }
-__global__ void k_dec_front_p(KemParams P, const uint8_t *sk, const uint8_t *ct, uint8_t *a_stream, uint8_t *hc,
-                              int n, int part);
-__global__ void k_dec_g_p(KemParams P, const uint8_t *mbuf, uint8_t *kr, uint8_t *s_stream, int n);
-__global__ void k_final_key_p(KemParams P, const uint8_t *ct, const uint8_t *hc, const uint8_t *kr,
-                              const uint8_t *fail, const uint8_t *sk, size_t sk_stride, uint8_t *ss, int n);
-__global__ void k_enc_front_p(KemParams P, const uint8_t *pk, const uint8_t *coins, uint8_t *mbuf, uint8_t *kr,
-                              uint8_t *s_stream, uint8_t *a_stream, int n, int with_gm);
-__global__ void k_genmatrix_p(KemParams P, const uint8_t *pk, size_t pk_stride, uint8_t *a_stream, int n);
-__global__ void k_shake_jobs_p(ShakeJob j0, ShakeJob j1, int n);
-__global__ void k_kp_final_p(KemParams P, const uint8_t *pk, uint8_t *sk, const uint8_t *coins, int n);
+// Decapsulation front: GenMatrix from the seed of the pk embedded in sk, and
+// H(c) (saber_dec, cuda_kernel.cu:383-384 and :447); with_gm = false: H(c) only.
+cudaError_t launch_dec_front(const HashCfg &cfg, const KemParams &P, const uint8_t *sk, const uint8_t *ct,
+                             uint8_t *a_stream, uint8_t *hc, size_t n, bool with_gm, cudaStream_t s,
+                             cudaStream_t s2);
+// kr = G(m' || H(pk)) and the GenSecret stream (saber_dec, cuda_kernel.cu:378-385).
+cudaError_t launch_dec_g(const HashCfg &cfg, const KemParams &P, const uint8_t *mbuf, uint8_t *kr, uint8_t *s_stream,
+                         size_t n, cudaStream_t s);
+// K = H((fail ? z : kr[0:32]) || H(c)) (cuda_kernel.cu:185-186, :445-450);
+// hc null: H(c) is made from ct; fail null: no selection; sk of instance i at
+// sk + i * sk_stride (0: one key).
+cudaError_t launch_final_key(const HashCfg &cfg, const KemParams &P, const uint8_t *ct, const uint8_t *hc,
+                             const uint8_t *kr, const uint8_t *fail, const uint8_t *sk, size_t sk_stride, uint8_t *ss,
+                             size_t n, cudaStream_t s);
+// Encapsulation front (saber_enc, cuda_kernel.cu:116-127): m = H(coins), H(pk),
+// kr = G(m || H(pk)), the GenSecret stream; with_gm: GenMatrix from pk's seed.
+cudaError_t launch_enc_front(const HashCfg &cfg, const KemParams &P, const uint8_t *pk, const uint8_t *coins,
+                             uint8_t *mbuf, uint8_t *kr, uint8_t *s_stream, uint8_t *a_stream, size_t n, bool with_gm,
+                             cudaStream_t s, cudaStream_t s2);
+// GenMatrix streams of n keys, seed_A at the end of pk + i * pk_stride.
+cudaError_t launch_genmatrix(const HashCfg &cfg, const KemParams &P, const uint8_t *pk, size_t pk_stride,
+                             uint8_t *a_stream, size_t n, cudaStream_t s);
+// Two SHAKE-128 jobs over n instances.
+cudaError_t launch_shake_jobs(const HashCfg &cfg, const ShakeJob &j0, const ShakeJob &j1, size_t n, cudaStream_t s,
+                              cudaStream_t s2);
+// Key-generation tail: sk[SK-64 : SK-32] = H(pk), sk[SK-32 : SK] = z.
+cudaError_t launch_kp_final(const HashCfg &cfg, const KemParams &P, const uint8_t *pk, uint8_t *sk,
+                            const uint8_t *coins, size_t n, cudaStream_t s);
 
 // Mixed-parameter decapsulation: group g covers global instances
 // [first, first + n) with its own parameters and buffers (device table).
@@ -106,9 +104,18 @@ struct HashGroup {
   const uint8_t *sk, *ct;
   uint8_t *a_stream, *s_stream, *mbuf, *kr, *fail, *hc, *ss;
 };
-// part 1: GenMatrix; part 2: H(c)
-__global__ void k_mix_front(const HashGroup *T, int ng, int total, int part);
-__global__ void k_mix_g(const HashGroup *T, int ng, int total);
-__global__ void k_mix_final(const HashGroup *T, int ng, int total);
+// perms: the roles' longest sponge among the groups.
+cudaError_t launch_mix_front(const HashCfg &cfg, const HashGroup *T, int ng, size_t total, int gm_perms, int h_perms,
+                             cudaStream_t s, cudaStream_t s2);
+cudaError_t launch_mix_g(const HashCfg &cfg, const HashGroup *T, int ng, size_t total, int perms, cudaStream_t s);
+cudaError_t launch_mix_final(const HashCfg &cfg, const HashGroup *T, int ng, size_t total, cudaStream_t s);
+
+// dst[i * words + w] = src[w] for i < n (16-byte words)
+__global__ void k_replicate16(uint4 *dst, const uint4 *src, int words, size_t n);
+
+// Keccak-f of one GenMatrix / GenSecret / H(c) / H(pk) sponge.
+inline int gm_perms(const KemParams &P) { return (P.gm_bytes + 167) / 168; }
+inline int gs_perms(const KemParams &P) { return (P.gs_bytes + 167) / 168; }
+inline int sha3_256_perms(int nbytes) { return nbytes / 136 + 1; }
 
 }  // namespace tmvp

@@ -54,6 +54,23 @@ __device__ __forceinline__ uint64_t rotl64(uint64_t v, int n) {
 // the constant is indexed by the round counter).
 __constant__ KeccakTables kKeccak = make_keccak_tables();
 
+// The same constants by halves, for the forms that hold halves.
+struct KeccakHalves {
+  uint32_t rc[24][2];  // [round][0: low half, 1: high half]
+};
+
+__host__ __device__ constexpr KeccakHalves make_keccak_halves() {
+  KeccakHalves h{};
+  const KeccakTables t = make_keccak_tables();
+  for (int i = 0; i < 24; i++) {
+    h.rc[i][0] = (uint32_t)t.rc[i];
+    h.rc[i][1] = (uint32_t)(t.rc[i] >> 32);
+  }
+  return h;
+}
+
+__constant__ KeccakHalves kKeccakHalves = make_keccak_halves();
+
 // a ^ b ^ c on both 32-bit halves, one three-input LOP3 each.  Theta applies
 // C[x-1] ^ rot(C[x+1], 1) to a lane this way instead of first forming that
 // term per column and then XORing it into five lanes (one XOR per column

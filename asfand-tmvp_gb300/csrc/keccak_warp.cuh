@@ -66,9 +66,10 @@ __device__ __forceinline__ uint32_t lop3_xor3(uint32_t a, uint32_t b, uint32_t c
   return d;
 }
 
-// One round; rc is the round constant, applied on lane 0 only.
-__device__ __forceinline__ void warp_keccak_round(uint32_t &lo, uint32_t &hi, const WarpKeccakLane &L,
-                                                  uint64_t rc) {
+// One round; rcl / rch are the halves of the round constant, applied on lane 0
+// only.
+__device__ __forceinline__ void warp_keccak_round(uint32_t &lo, uint32_t &hi, const WarpKeccakLane &L, uint32_t rcl,
+                                                  uint32_t rch) {
   constexpr unsigned F = 0xFFFFFFFFu;
   // theta: column parity C[x], then D = C[x-1] ^ rot(C[x+1], 1)
   uint32_t c0 = __shfl_sync(F, lo, L.col[0]), c1 = __shfl_sync(F, lo, L.col[1]);
@@ -89,14 +90,21 @@ __device__ __forceinline__ void warp_keccak_round(uint32_t &lo, uint32_t &hi, co
   const uint32_t b0l = __shfl_sync(F, bl, L.chi[0]), b0h = __shfl_sync(F, bh, L.chi[0]);
   const uint32_t b1l = __shfl_sync(F, bl, L.chi[1]), b1h = __shfl_sync(F, bh, L.chi[1]);
   const uint32_t b2l = __shfl_sync(F, bl, L.chi[2]), b2h = __shfl_sync(F, bh, L.chi[2]);
-  lo = (b0l ^ (~b1l & b2l)) ^ ((uint32_t)rc & L.iota);
-  hi = (b0h ^ (~b1h & b2h)) ^ ((uint32_t)(rc >> 32) & L.iota);
+  lo = (b0l ^ (~b1l & b2l)) ^ (rcl & L.iota);
+  hi = (b0h ^ (~b1h & b2h)) ^ (rch & L.iota);
 }
 
+// U rounds a loop iteration.  24 (straight-line) serves a sponge that runs
+// many permutations from one place (Saber decapsulation of one key 59.4
+// against 61.4 us with 8); 8 the places that run one, which cost the fetch of
+// their instructions.
+template <int U>
 __device__ __forceinline__ void warp_keccak_f1600(uint32_t &lo, uint32_t &hi, const WarpKeccakLane &L) {
-  constexpr KeccakTables T = make_keccak_tables();
+#pragma unroll 1
+  for (int ir = 0; ir < 24; ir += U)
 #pragma unroll
-  for (int ir = 0; ir < 24; ir++) warp_keccak_round(lo, hi, L, T.rc[ir]);
+    for (int r = 0; r < U; r++)
+      warp_keccak_round(lo, hi, L, kKeccakHalves.rc[ir + r][0], kKeccakHalves.rc[ir + r][1]);
 }
 
 // Sponge helpers.  `lane` is the caller's lane in the warp; the state lives
@@ -111,23 +119,30 @@ __device__ __forceinline__ void warp_xor_word(uint32_t &lo, uint32_t &hi, uint64
   hi ^= (uint32_t)(w >> 32);
 }
 
-// Absorb nbytes (a multiple of 8) from 8-byte-aligned global memory at rate
-// RATE_W words with the given domain byte, then pad10*1; the state starts at
-// zero and is left ready for the first squeeze permutation.
+// SHA3-256 / SHA3-512-style hash (rate RATE_W words) of nbytes (a multiple of
+// 8) from 8-byte-aligned global memory, with the domain byte and pad10*1: the
+// state after the last block's permutation.  The words of a block are loaded
+// before the permutation of the one before it (a load takes about a third of
+// a permutation).
 template <int RATE_W>
-__device__ __forceinline__ void warp_absorb_words(uint32_t &lo, uint32_t &hi, const WarpKeccakLane &L, int lane,
-                                                  const uint64_t *in, int nbytes, uint64_t domain) {
+__device__ __forceinline__ void warp_hash_words(uint32_t &lo, uint32_t &hi, const WarpKeccakLane &L, int lane,
+                                                const uint64_t *in, int nbytes, uint64_t domain) {
   lo = hi = 0;
   int nw = nbytes >> 3;
-  while (nw >= RATE_W) {
-    if (lane < RATE_W) warp_xor_word(lo, hi, in[lane]);
-    warp_keccak_f1600(lo, hi, L);
+  uint64_t w = lane < RATE_W && lane < nw ? in[lane] : 0ull;
+  for (;;) {
+    warp_xor_word(lo, hi, w);
+    const bool last = nw < RATE_W;
+    if (last) {
+      if (lane == nw) warp_xor_word(lo, hi, domain);
+      if (lane == RATE_W - 1) hi ^= 0x80000000u;
+    }
     in += RATE_W;
     nw -= RATE_W;
+    w = lane < RATE_W && lane < nw ? in[lane] : 0ull;
+    warp_keccak_f1600<24>(lo, hi, L);
+    if (last) break;
   }
-  if (lane < nw) warp_xor_word(lo, hi, in[lane]);
-  if (lane == nw) warp_xor_word(lo, hi, domain);
-  if (lane == RATE_W - 1) hi ^= 0x80000000u;
 }
 
 // Absorb a short message of nw < RATE_W words held one per lane (lane k < nw
@@ -139,20 +154,6 @@ __device__ __forceinline__ void warp_absorb_lanes(uint32_t &lo, uint32_t &hi, in
   if (lane < nw) warp_xor_word(lo, hi, w);
   if (lane == nw) warp_xor_word(lo, hi, domain);
   if (lane == RATE_W - 1) hi ^= 0x80000000u;
-}
-
-// Squeeze nbytes (a multiple of 8) of SHAKE-128 (rate 21 words) to
-// 8-byte-aligned global memory, the state already absorbed and padded.
-__device__ __forceinline__ void warp_shake128_squeeze(uint32_t &lo, uint32_t &hi, const WarpKeccakLane &L,
-                                                      int lane, uint64_t *out, int nbytes) {
-  int nw = nbytes >> 3;
-  while (nw > 0) {
-    warp_keccak_f1600(lo, hi, L);
-    const int k = nw < 21 ? nw : 21;
-    if (lane < k) out[lane] = warp_lane_word(lo, hi);
-    out += 21;
-    nw -= k;
-  }
 }
 
 }  // namespace tmvp

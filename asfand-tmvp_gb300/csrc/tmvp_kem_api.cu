@@ -3,13 +3,13 @@
 // NIST-style API and the reference-compatible shims.
 //
 // Pipelines (kernels in launch order, all on the caller's stream):
-//   keypair : k_shake_jobs (seed_A' = SHAKE(seed_A), GenMatrix; GenSecret)
-//             -> k_cpa<kKeygen> -> k_kp_final (H(pk), z)
-//   encaps  : k_enc_front (H(coins), H(pk), G, GenSecret; GenMatrix)
-//             -> k_cpa<kEncrypt> -> k_final_key
-//   decaps  : k_dec_front (GenMatrix; H(c)) on two side streams, concurrent
-//             with k_cpa<kDecrypt> -> k_dec_g; k_cpa<kReenc> waits only for
-//             GenMatrix, k_final_key (implicit rejection) also for H(c)
+//   keypair : launch_shake_jobs (seed_A' = SHAKE(seed_A), GenMatrix; GenSecret)
+//             -> k_cpa<kKeygen> -> launch_kp_final (H(pk), z)
+//   encaps  : launch_enc_front (H(coins), H(pk), G, GenSecret; GenMatrix)
+//             -> k_cpa<kEncrypt> -> launch_final_key
+//   decaps  : launch_dec_front (GenMatrix; H(c)) on side streams, concurrent
+//             with k_cpa<kDecrypt> -> launch_dec_g; k_cpa<kReenc> waits for
+//             it, then launch_final_key (implicit rejection)
 // They replace the launch sequences of saber_enc / saber_dec
 // (TMVP-Saber/SABER-GPU/src/cuda_kernel.cu:25-479) and SABLE_enc / SABLE_dec
 // (TMVP_SABLE/src/SABLE_indcpa.cu:24-610).
@@ -67,13 +67,15 @@ struct tmvp_ctx {
   int *d_err = nullptr;   // device-side input-range flag
   uint64_t launches = 0;
   cudaStream_t side = nullptr;          // GenMatrix and H(c) beside the decryption (highest priority)
-  cudaEvent_t fork_ev = nullptr, join_ev = nullptr;
+  cudaStream_t side2 = nullptr;         // the second launch of a split Keccak front, beside the first
+  cudaEvent_t fork_ev = nullptr, join_ev = nullptr, fork2_ev = nullptr, join2_ev = nullptr;
   cudaEvent_t gm_ev = nullptr;                     // whole-batch GenMatrix of a host-input call
   size_t host_chunk = 16384;                       // chunk of host-input decapsulation (0: none)
   int host_ramp = 1;                               // first chunks host_chunk >> ramp, >> ramp-1, ...
   size_t dev_chunk = 32768;                        // chunk of device-input decapsulation (0: none)
   bool serial = false;                             // every stage on the caller's stream, one at a time
   int front_cap = 0;                               // Keccak-front blocks per SM (0: one thread per sponge)
+  bool hash_limits = false;                        // the caller set one of the next two (else plan_sponges chooses)
   size_t warp_hash = kWarpHashDefault;             // Keccak launches of <= this many sponges: a warp per sponge
   size_t pair_hash = kPairHashDefault;             // else of <= this many: two threads per sponge
   // set by the caller (tmvp_ctx_set_*): then the autotuner's per-batch choice does not apply
@@ -82,6 +84,7 @@ struct tmvp_ctx {
   static constexpr int kLanes = 4;                 // streams for chunk chains
   cudaStream_t lane[kLanes] = {};
   cudaStream_t lane_side[kLanes] = {};             // the Keccak front of each lane (highest priority)
+  cudaStream_t lane_side2[kLanes] = {};            // and its second launch
   cudaEvent_t lane_ev[kLanes] = {};
   cudaStream_t copy[2] = {};                       // host-to-device copies of chunked calls
   static constexpr int kSlots = 5;                 // input slots of chunked host calls
@@ -316,27 +319,27 @@ int run_cpa(tmvp_ctx *c, int form, int op, CpaArgs &a, cudaStream_t s) {
   return e == 0 ? TMVP_OK : TMVP_EDEVICE;
 }
 
-inline unsigned blocks_for(size_t threads, unsigned bs) { return (unsigned)((threads + bs - 1) / bs); }
-
-// Threads per block of the Keccak kernels (one sponge per thread): small
-// blocks spread a batch evenly over the 152 SMs of an ALU-bound stage.
-constexpr unsigned kHashBlock = 64;
-// The form of a Keccak launch under the context's limits (hash_form_for).
-inline HashForm hash_form(const tmvp_ctx *c, size_t sponges, bool short_sponges = false) {
-  return hash_form_for(sponges, short_sponges, c->warp_hash, c->pair_hash);
+// What the Keccak launches of a context may use (plan_sponges).
+inline HashCfg hash_cfg(const tmvp_ctx *c) {
+  HashCfg h{c->nsm};
+  h.limits = c->hash_limits;
+  h.warp_max = c->warp_hash;
+  h.pair_max = c->pair_hash;
+  return h;
 }
 
-// GenMatrix streams of n keys (seed_A at the end of pk + i * pk_stride) in
-// the form the launch size gives.
-void launch_genmatrix(const tmvp_ctx *c, const KemParams &P, const uint8_t *pk, size_t pk_stride,
-                      uint8_t *a_stream, size_t n, cudaStream_t s) {
-  const HashForm f = hash_form(c, n);
-  if (f == kHashWarp)
-    k_genmatrix_w<<<warp_blocks(n), kWarpHashBlock, 0, s>>>(P, pk, pk_stride, a_stream, (int)n);
-  else if (f == kHashPair)
-    k_genmatrix_p<<<pair_blocks(2 * n), kPairHashBlock, 0, s>>>(P, pk, pk_stride, a_stream, (int)n);
-  else
-    k_genmatrix<<<blocks_for(n, kHashBlock), kHashBlock, 0, s>>>(P, pk, pk_stride, a_stream, (int)n);
+// A two-role Keccak launch on s, its second launch (if n splits it) on a lane
+// forked from s and joined back.
+template <class F>
+int forked(tmvp_ctx *c, size_t n, cudaStream_t s, F launch) {
+  if (c->serial || !sponges_split(hash_cfg(c), n)) return cuda_err(launch(s));
+  cudaStream_t s2 = c->lane[0];
+  TRY_CUDA(cudaEventRecord(c->fork2_ev, s));
+  TRY_CUDA(cudaStreamWaitEvent(s2, c->fork2_ev, 0));
+  TRY(cuda_err(launch(s2)));
+  TRY_CUDA(cudaEventRecord(c->join2_ev, s2));
+  TRY_CUDA(cudaStreamWaitEvent(s, c->join2_ev, 0));
+  return TMVP_OK;
 }
 
 int check_common(tmvp_ctx *c, int set, size_t n, int form, KemParams *P) {
@@ -377,10 +380,6 @@ struct Guard {
   }
 };
 
-// Host-resident decapsulation inputs are copied and processed in chunks (the
-// context's host_chunk instances, default below), so that the copy of one
-// chunk overlaps the kernels of the previous one.
-constexpr size_t kHostChunk = 16384;
 // Largest whole-batch GenMatrix buffer a host-input decapsulation expands
 // ahead of its chunks (1M Saber instances take 3.6 GiB).
 constexpr size_t kGmFirstBytes = size_t(4) << 30;
@@ -483,31 +482,23 @@ int dec_pipeline(tmvp_ctx *c, const KemParams &P, size_t n, uint8_t *ss, const u
     TRY_CUDA(cudaEventRecord(c->fork_ev, s));
     TRY_CUDA(cudaStreamWaitEvent(side, c->fork_ev, 0));
   }
-  if (a_cached) {  // GenMatrix given: the front is H(c) alone
+  HashCfg h = hash_cfg(c);
+  if (!a_cached && !c->serial) h.cap = (c->front_cap + 1) / 2;  // 64-thread blocks asked for, launched as 128
+  // (GenMatrix given: the front is H(c) alone)
+  const bool split = !a_cached && fork && sponges_split(h, n);
+  cudaStream_t side2 = side;
+  if (split) {
+    side2 = c->side2;
+    for (int l = 0; l < tmvp_ctx::kLanes; l++)
+      if (side == c->lane_side[l]) side2 = c->lane_side2[l];
+    TRY_CUDA(cudaStreamWaitEvent(side2, c->fork_ev, 0));
+  }
+  {
     StageTimer tm_(c, "dec_front", side);
-    const HashForm f = hash_form(c, n);
-    if (f == kHashWarp)
-      k_dec_front_w<<<warp_blocks(n), kWarpHashBlock, 0, side>>>(P, sk, ct, w.a_stream, w.hc, (int)n, 2);
-    else if (f == kHashPair)
-      k_dec_front_p<<<pair_blocks(2 * n), kPairHashBlock, 0, side>>>(P, sk, ct, w.a_stream, w.hc, (int)n, 2);
-    else
-      k_dec_front<<<blocks_for(n, kHashBlock), kHashBlock, 0, side>>>(P, sk, ct, w.a_stream, w.hc, (int)n, 2);
-  } else {
-    StageTimer tm_(c, "dec_front", side);
-    const unsigned grid = blocks_for(warp_round(n) + n, kHashBlock);
-    const HashForm f = hash_form(c, 2 * n);
-    if (f == kHashWarp)
-      k_dec_front_w<<<warp_blocks(2 * n), kWarpHashBlock, 0, side>>>(P, sk, ct, w.a_stream, w.hc, (int)n, 0);
-    else if (f == kHashPair)
-      k_dec_front_p<<<pair_blocks(warp_round(2 * n) + 2 * n), kPairHashBlock, 0, side>>>(P, sk, ct, w.a_stream,
-                                                                                        w.hc, (int)n, 0);
-    else if (c->front_cap > 0 && !c->serial && grid > (unsigned)(c->nsm * c->front_cap))
-      k_dec_front_strided<<<(unsigned)(c->nsm * c->front_cap), kHashBlock, 0, side>>>(P, sk, ct, w.a_stream, w.hc,
-                                                                                   (int)n);
-    else
-      k_dec_front<<<grid, kHashBlock, 0, side>>>(P, sk, ct, w.a_stream, w.hc, (int)n, 0);
+    TRY_CUDA(launch_dec_front(h, P, sk, ct, w.a_stream, w.hc, n, !a_cached, side, side2));
   }
   TRY_CUDA(cudaEventRecord(c->join_ev, side));
+  if (split) TRY_CUDA(cudaEventRecord(c->join2_ev, side2));
   c->launches++;
   CpaArgs a{};
   a.P = P;
@@ -530,16 +521,11 @@ int dec_pipeline(tmvp_ctx *c, const KemParams &P, size_t n, uint8_t *ss, const u
   }
   {
     StageTimer tm_(c, "dec_g", s);
-    const HashForm f = hash_form(c, n, true);
-    if (f == kHashWarp)
-      k_dec_g_w<<<warp_blocks(n), kWarpHashBlock, 0, s>>>(P, w.mbuf, w.kr, w.s_stream, (int)n);
-    else if (f == kHashPair)
-      k_dec_g_p<<<pair_blocks(2 * n), kPairHashBlock, 0, s>>>(P, w.mbuf, w.kr, w.s_stream, (int)n);
-    else
-      k_dec_g<<<blocks_for(n, kHashBlock), kHashBlock, 0, s>>>(P, w.mbuf, w.kr, w.s_stream, (int)n);
+    TRY_CUDA(launch_dec_g(hash_cfg(c), P, w.mbuf, w.kr, w.s_stream, n, s));
   }
   c->launches++;
   TRY_CUDA(cudaStreamWaitEvent(s, c->join_ev, 0));  // join: GenMatrix
+  if (split) TRY_CUDA(cudaStreamWaitEvent(s, c->join2_ev, 0));
   if (a_ready) TRY_CUDA(cudaStreamWaitEvent(s, a_ready, 0));  // a_cached written on another stream
   CpaArgs b{};
   b.P = P;
@@ -557,16 +543,7 @@ int dec_pipeline(tmvp_ctx *c, const KemParams &P, size_t n, uint8_t *ss, const u
   if ((r = run_cpa(c, form, kReenc, b, s))) return r;
   {
     StageTimer tm_(c, "final_key", s);
-    const size_t sk_stride = key_shared ? 0 : (size_t)P.sk_bytes;
-    const HashForm f = hash_form(c, n, true);
-    if (f == kHashWarp)
-      k_final_key_w<<<warp_blocks(n), kWarpHashBlock, 0, s>>>(P, ct, w.hc, w.kr, w.fail, sk, sk_stride, ss, (int)n);
-    else if (f == kHashPair)
-      k_final_key_p<<<pair_blocks(2 * n), kPairHashBlock, 0, s>>>(P, ct, w.hc, w.kr, w.fail, sk, sk_stride, ss,
-                                                                  (int)n);
-    else
-      k_final_key<<<blocks_for(n, kHashBlock), kHashBlock, 0, s>>>(P, ct, w.hc, w.kr, w.fail, sk, sk_stride, ss,
-                                                                   (int)n);
+    TRY_CUDA(launch_final_key(hash_cfg(c), P, ct, w.hc, w.kr, w.fail, sk, key_shared ? 0 : (size_t)P.sk_bytes, ss, n, s));
   }
   c->launches++;
   return TMVP_OK;
@@ -677,6 +654,9 @@ int tmvp_ctx_create(int device, size_t mem_budget, tmvp_ctx **out) {
       cudaStreamCreateWithPriority(&c->side, cudaStreamNonBlocking, pri_high) != cudaSuccess ||
       cudaEventCreateWithFlags(&c->fork_ev, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&c->join_ev, cudaEventDisableTiming) != cudaSuccess ||
+      cudaStreamCreateWithPriority(&c->side2, cudaStreamNonBlocking, pri_high) != cudaSuccess ||
+      cudaEventCreateWithFlags(&c->fork2_ev, cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&c->join2_ev, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&c->gm_ev, cudaEventDisableTiming) != cudaSuccess ||
       cudaStreamCreateWithFlags(&c->copy[0], cudaStreamNonBlocking) != cudaSuccess ||
       cudaStreamCreateWithFlags(&c->copy[1], cudaStreamNonBlocking) != cudaSuccess) {
@@ -697,6 +677,7 @@ int tmvp_ctx_create(int device, size_t mem_budget, tmvp_ctx **out) {
   for (int i = 0; i < tmvp_ctx::kLanes; i++)
     if (cudaStreamCreateWithPriority(&c->lane[i], cudaStreamNonBlocking, pri_low) != cudaSuccess ||
         cudaStreamCreateWithPriority(&c->lane_side[i], cudaStreamNonBlocking, pri_high) != cudaSuccess ||
+        cudaStreamCreateWithPriority(&c->lane_side2[i], cudaStreamNonBlocking, pri_high) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->lane_ev[i], cudaEventDisableTiming) != cudaSuccess) {
     delete c;
     return set_err(TMVP_EDEVICE);
@@ -715,12 +696,16 @@ void tmvp_ctx_destroy(tmvp_ctx *c) {
     if (c->ws && !c->ws_external) cudaFree(c->ws);
     if (c->d_err) cudaFree(c->d_err);
     if (c->side) cudaStreamDestroy(c->side);
+    if (c->side2) cudaStreamDestroy(c->side2);
+    if (c->fork2_ev) cudaEventDestroy(c->fork2_ev);
+    if (c->join2_ev) cudaEventDestroy(c->join2_ev);
     if (c->fork_ev) cudaEventDestroy(c->fork_ev);
     if (c->join_ev) cudaEventDestroy(c->join_ev);
     if (c->gm_ev) cudaEventDestroy(c->gm_ev);
     for (int i = 0; i < tmvp_ctx::kLanes; i++) {
       if (c->lane[i]) cudaStreamDestroy(c->lane[i]);
       if (c->lane_side[i]) cudaStreamDestroy(c->lane_side[i]);
+      if (c->lane_side2[i]) cudaStreamDestroy(c->lane_side2[i]);
       if (c->lane_ev[i]) cudaEventDestroy(c->lane_ev[i]);
     }
     for (int i = 0; i < 2; i++)
@@ -764,6 +749,7 @@ int tmvp_ctx_set_warp_hash(tmvp_ctx *c, size_t max_sponges) {
   if (!c) return set_err(TMVP_EINVAL);
   std::lock_guard<std::mutex> lk(c->mu);
   c->warp_hash = max_sponges;
+  c->hash_limits = true;
   return set_err(TMVP_OK);
 }
 
@@ -771,6 +757,7 @@ int tmvp_ctx_set_pair_hash(tmvp_ctx *c, size_t max_sponges) {
   if (!c) return set_err(TMVP_EINVAL);
   std::lock_guard<std::mutex> lk(c->mu);
   c->pair_hash = max_sponges;
+  c->hash_limits = true;
   return set_err(TMVP_OK);
 }
 
@@ -864,13 +851,8 @@ int tmvp_kem_keypair_batch(tmvp_ctx *c, tmvp_param_set set, size_t n, uint8_t *p
   ShakeJob j1{bco.dev, 96, 32, s_stream, (size_t)P.gs_bytes, P.gs_bytes, 0, nullptr, 0, 0};
   {
     StageTimer tm_(c, "shake_jobs", s);
-    const HashForm f = hash_form(c, 2 * n);
-    if (f == kHashWarp)
-      k_shake_jobs_w<<<warp_blocks(2 * n), kWarpHashBlock, 0, s>>>(j0, j1, (int)n);
-    else if (f == kHashPair)
-      k_shake_jobs_p<<<pair_blocks(warp_round(2 * n) + 2 * n), kPairHashBlock, 0, s>>>(j0, j1, (int)n);
-    else
-      k_shake_jobs<<<blocks_for(warp_round(n) + n, kHashBlock), kHashBlock, 0, s>>>(j0, j1, (int)n);
+    if ((r = forked(c, n, s, [&](cudaStream_t s2) { return launch_shake_jobs(hash_cfg(c), j0, j1, n, s, s2); })))
+      return set_err(r);
   }
   c->launches++;
   CpaArgs a{};
@@ -884,13 +866,7 @@ int tmvp_kem_keypair_batch(tmvp_ctx *c, tmvp_param_set set, size_t n, uint8_t *p
   if ((r = run_cpa(c, form, kKeygen, a, s))) return set_err(r);
   {
     StageTimer tm_(c, "kp_final", s);
-    const HashForm f = hash_form(c, n, true);
-    if (f == kHashWarp)
-      k_kp_final_w<<<warp_blocks(n), kWarpHashBlock, 0, s>>>(P, bpk.dev, bsk.dev, bco.dev, (int)n);
-    else if (f == kHashPair)
-      k_kp_final_p<<<pair_blocks(2 * n), kPairHashBlock, 0, s>>>(P, bpk.dev, bsk.dev, bco.dev, (int)n);
-    else
-      k_kp_final<<<blocks_for(n, kHashBlock), kHashBlock, 0, s>>>(P, bpk.dev, bsk.dev, bco.dev, (int)n);
+    if (cudaError_t e_ = launch_kp_final(hash_cfg(c), P, bpk.dev, bsk.dev, bco.dev, n, s)) return set_err(cuda_err(e_));
   }
   c->launches++;
   if ((r = download(bpk, s)) || (r = download(bsk, s))) return set_err(r);
@@ -928,17 +904,10 @@ int enc_batch(tmvp_ctx *c, tmvp_param_set set, size_t n, uint8_t *ct, uint8_t *s
   if ((r = upload(bpk, s)) || (r = upload(bco, s))) return set_err(r);
   {
     StageTimer tm_(c, "enc_front", s);
-    // the second role expands GenMatrix, unless it is given
-    const HashForm f = hash_form(c, a_cached ? n : 2 * n);
-    if (f == kHashWarp)
-      k_enc_front_w<<<warp_blocks(a_cached ? n : 2 * n), kWarpHashBlock, 0, s>>>(
-          P, bpk.dev, bco.dev, mbuf, kr, s_stream, a_stream, (int)n, a_cached ? 0 : 1);
-    else if (f == kHashPair)
-      k_enc_front_p<<<pair_blocks(a_cached ? 2 * n : warp_round(2 * n) + 2 * n), kPairHashBlock, 0, s>>>(
-          P, bpk.dev, bco.dev, mbuf, kr, s_stream, a_stream, (int)n, a_cached ? 0 : 1);
-    else
-      k_enc_front<<<blocks_for(a_cached ? n : warp_round(n) + n, kHashBlock), kHashBlock, 0, s>>>(
-          P, bpk.dev, bco.dev, mbuf, kr, s_stream, a_stream, (int)n);
+    auto launch = [&](cudaStream_t s2) {
+      return launch_enc_front(hash_cfg(c), P, bpk.dev, bco.dev, mbuf, kr, s_stream, a_stream, n, !a_cached, s, s2);
+    };
+    if ((r = a_cached ? cuda_err(launch(s)) : forked(c, n, s, launch))) return set_err(r);
   }
   c->launches++;
   CpaArgs a{};
@@ -955,16 +924,8 @@ int enc_batch(tmvp_ctx *c, tmvp_param_set set, size_t n, uint8_t *ct, uint8_t *s
   if ((r = run_cpa(c, form, kEncrypt, a, s))) return set_err(r);
   {
     StageTimer tm_(c, "final_key", s);
-    const HashForm f = hash_form(c, n, true);
-    if (f == kHashWarp)
-      k_final_key_w<<<warp_blocks(n), kWarpHashBlock, 0, s>>>(P, bct.dev, nullptr, kr, nullptr, nullptr, 0, bss.dev,
-                                                               (int)n);
-    else if (f == kHashPair)
-      k_final_key_p<<<pair_blocks(2 * n), kPairHashBlock, 0, s>>>(P, bct.dev, nullptr, kr, nullptr, nullptr, 0,
-                                                                  bss.dev, (int)n);
-    else
-      k_final_key<<<blocks_for(n, kHashBlock), kHashBlock, 0, s>>>(P, bct.dev, nullptr, kr, nullptr, nullptr, 0,
-                                                                   bss.dev, (int)n);
+    if (cudaError_t e_ = launch_final_key(hash_cfg(c), P, bct.dev, nullptr, kr, nullptr, nullptr, 0, bss.dev, n, s))
+      return set_err(cuda_err(e_));
   }
   c->launches++;
   if ((r = download(bct, s)) || (r = download(bss, s))) return set_err(r);
@@ -997,7 +958,7 @@ int tmvp_genmatrix_batch(tmvp_ctx *c, tmvp_param_set set, size_t n, uint8_t *a_s
   if (classify(a_stream, n * P.gm_bytes, c->device).host || classify(pk, n * pk_stride, c->device).host)
     return set_err(TMVP_EINVAL);  // device buffers only
   cudaStream_t s = (cudaStream_t)stream;
-  launch_genmatrix(c, P, pk, pk_stride, a_stream, n, s);
+  if (cudaError_t e_ = launch_genmatrix(hash_cfg(c), P, pk, pk_stride, a_stream, n, s)) return set_err(cuda_err(e_));
   c->launches++;
   return set_err(finish(c, s, false));
 }
@@ -1078,10 +1039,7 @@ int tmvp_kem_dec_batch_onekey(tmvp_ctx *c, tmvp_param_set set, size_t n, uint8_t
     TRY_CUDA(cudaStreamWaitEvent(c->side, c->fork_ev, 0));
     {
       StageTimer tm_(c, "genmatrix", c->side);
-      if (hash_form(c, 1) == kHashWarp)
-        k_genmatrix_w<<<1, kWarpHashBlock, 0, c->side>>>(P, bsk.dev + P.indcpa_sk_bytes, 0, a_one, 1);
-      else
-        k_genmatrix<<<1, kHashBlock, 0, c->side>>>(P, bsk.dev + P.indcpa_sk_bytes, 0, a_one, 1);
+      TRY_CUDA(launch_genmatrix(hash_cfg(c), P, bsk.dev + P.indcpa_sk_bytes, 0, a_one, 1, c->side));
     }
     c->launches++;
     TRY_CUDA(cudaEventRecord(c->gm_ev, c->side));
@@ -1135,10 +1093,7 @@ int tmvp_kem_dec_batch_onekey(tmvp_ctx *c, tmvp_param_set set, size_t n, uint8_t
   TRY_CUDA(cudaStreamWaitEvent(gs, c->fork_ev, 0));
   {
     StageTimer tm_(c, "genmatrix", gs);
-    if (hash_form(c, 1) == kHashWarp)
-      k_genmatrix_w<<<1, kWarpHashBlock, 0, gs>>>(P, bsk.dev + P.indcpa_sk_bytes, 0, a_one, 1);
-    else
-      k_genmatrix<<<1, kHashBlock, 0, gs>>>(P, bsk.dev + P.indcpa_sk_bytes, 0, a_one, 1);
+    TRY_CUDA(launch_genmatrix(hash_cfg(c), P, bsk.dev + P.indcpa_sk_bytes, 0, a_one, 1, gs));
     if (!shared)
       k_replicate16<<<grid, 256, 0, gs>>>(reinterpret_cast<uint4 *>(a_rep), reinterpret_cast<const uint4 *>(a_one),
                                           P.gm_bytes / 16, n);
@@ -1215,8 +1170,7 @@ int tmvp_kem_dec_batch(tmvp_ctx *c, tmvp_param_set set, size_t n, uint8_t *ss, c
       TRY_CUDA(cudaStreamWaitEvent(c->side, c->fork_ev, 0));
       {
         StageTimer tm_(c, "genmatrix", c->side);
-        k_genmatrix<<<blocks_for(n, kHashBlock), kHashBlock, 0, c->side>>>(P, sk_seed + P.indcpa_sk_bytes,
-                                                                           P.sk_bytes, a_full, (int)n);
+        TRY_CUDA(launch_genmatrix(hash_cfg(c), P, sk_seed + P.indcpa_sk_bytes, P.sk_bytes, a_full, n, c->side));
       }
       c->launches++;
       TRY_CUDA(cudaEventRecord(c->gm_ev, c->side));
@@ -1285,7 +1239,7 @@ int tmvp_kem_dec_batch(tmvp_ctx *c, tmvp_param_set set, size_t n, uint8_t *ss, c
     TRY_CUDA(cudaStreamWaitEvent(gs, c->fork_ev, 0));
     {
       StageTimer tm_(c, "genmatrix", gs);
-      launch_genmatrix(c, P, sk_map + P.indcpa_sk_bytes, P.sk_bytes, a_early, n, gs);
+      TRY_CUDA(launch_genmatrix(hash_cfg(c), P, sk_map + P.indcpa_sk_bytes, P.sk_bytes, a_early, n, gs));
     }
     c->launches++;
     TRY_CUDA(cudaEventRecord(c->gm_ev, gs));
@@ -1330,13 +1284,8 @@ int tmvp_indcpa_keypair_batch(tmvp_ctx *c, tmvp_param_set set, size_t n, uint8_t
   ShakeJob j1{bse.dev, 64, 32, s_stream, (size_t)P.gs_bytes, P.gs_bytes, 0, nullptr, 0, 0};
   {
     StageTimer tm_(c, "shake_jobs", s);
-    const HashForm f = hash_form(c, 2 * n);
-    if (f == kHashWarp)
-      k_shake_jobs_w<<<warp_blocks(2 * n), kWarpHashBlock, 0, s>>>(j0, j1, (int)n);
-    else if (f == kHashPair)
-      k_shake_jobs_p<<<pair_blocks(warp_round(2 * n) + 2 * n), kPairHashBlock, 0, s>>>(j0, j1, (int)n);
-    else
-      k_shake_jobs<<<blocks_for(warp_round(n) + n, kHashBlock), kHashBlock, 0, s>>>(j0, j1, (int)n);
+    if ((r = forked(c, n, s, [&](cudaStream_t s2) { return launch_shake_jobs(hash_cfg(c), j0, j1, n, s, s2); })))
+      return set_err(r);
   }
   c->launches++;
   CpaArgs a{};
@@ -1383,13 +1332,8 @@ int tmvp_indcpa_enc_batch(tmvp_ctx *c, tmvp_param_set set, size_t n, uint8_t *ct
               (size_t)P.gm_bytes, P.gm_bytes, 0, nullptr, 0, 0};
   {
     StageTimer tm_(c, "shake_jobs", s);
-    const HashForm f = hash_form(c, 2 * n);
-    if (f == kHashWarp)
-      k_shake_jobs_w<<<warp_blocks(2 * n), kWarpHashBlock, 0, s>>>(j0, j1, (int)n);
-    else if (f == kHashPair)
-      k_shake_jobs_p<<<pair_blocks(warp_round(2 * n) + 2 * n), kPairHashBlock, 0, s>>>(j0, j1, (int)n);
-    else
-      k_shake_jobs<<<blocks_for(warp_round(n) + n, kHashBlock), kHashBlock, 0, s>>>(j0, j1, (int)n);
+    if ((r = forked(c, n, s, [&](cudaStream_t s2) { return launch_shake_jobs(hash_cfg(c), j0, j1, n, s, s2); })))
+      return set_err(r);
   }
   c->launches++;
   CpaArgs a{};
@@ -1668,18 +1612,18 @@ size_t mixed_tab_bytes(size_t ng) {
 // memory; tabs: mixed_tab_bytes of device memory for the group tables, which
 // are built into host_tabs and, if upload_tabs, copied on s.  Makes no
 // allocation and no host synchronisation, so it can be captured into a graph.
-// Streams of one mixed chain: its own stream, the side stream of its Keccak
+// Streams of one mixed chain: its own stream, the side streams of its Keccak
 // front, and the lanes [lane0, lane0 + nlanes) its per-set launches spread over.
 struct MixStreams {
-  cudaStream_t side;
+  cudaStream_t side, side2;
   int lane0, nlanes;
 };
 
 int mixed_enqueue(tmvp_ctx *c, size_t ng, const tmvp_dec_group *gr, uint8_t *ws, uint8_t *tabs,
                   std::vector<uint8_t> &host_tabs, bool upload_tabs, cudaStream_t s,
-                  MixStreams ms = MixStreams{nullptr, 0, tmvp_ctx::kLanes}) {
-  if (!ms.side) ms.side = c->side;
-  if (c->serial) ms.side = s;  // measurement: every stage alone on s
+                  MixStreams ms = MixStreams{nullptr, nullptr, 0, tmvp_ctx::kLanes}) {
+  if (!ms.side) ms.side = c->side, ms.side2 = c->side2;
+  if (c->serial) ms.side = ms.side2 = s;  // measurement: every stage alone on s
   std::vector<CpaArgs> ga(ng), gb(ng);
   std::vector<HashGroup> hg(ng);
   Arena A{ws};
@@ -1769,16 +1713,23 @@ int mixed_enqueue(tmvp_ctx *c, size_t ng, const tmvp_dec_group *gr, uint8_t *ws,
   auto tdec = [&](int st) { return reinterpret_cast<const MixTable *>(tabs + st * tb); };
   auto tre = [&](int st) { return reinterpret_cast<const MixTable *>(tabs + (kNumSets + st) * tb); };
   const HashGroup *th = reinterpret_cast<const HashGroup *>(tabs + 2 * kNumSets * tb);
-  const unsigned nb = blocks_for((size_t)total, kHashBlock);
+  int gm = 0, hp = 0, gp = 0;  // the longest sponges
+  for (const HashGroup &h : hg) {
+    gm = std::max(gm, gm_perms(h.P));
+    hp = std::max(hp, sha3_256_perms(h.P.ct_bytes));
+    gp = std::max(gp, 1 + gs_perms(h.P));
+  }
   TRY_CUDA(cudaEventRecord(c->fork_ev, s));
   TRY_CUDA(cudaStreamWaitEvent(ms.side, c->fork_ev, 0));
+  const bool split = sponges_split(hash_cfg(c), (size_t)total);
+  if (split) TRY_CUDA(cudaStreamWaitEvent(ms.side2, c->fork_ev, 0));
   // GenMatrix and H(c) of every group in one launch (2 total sponges)
   {
     StageTimer tm_(c, "mix_front", ms.side);
-    k_mix_front<<<blocks_for(warp_round((size_t)total) + total, kHashBlock), kHashBlock, 0, ms.side>>>(
-        th, (int)ng, total, 0);
+    TRY_CUDA(launch_mix_front(hash_cfg(c), th, (int)ng, (size_t)total, gm, hp, ms.side, split ? ms.side2 : ms.side));
   }
   TRY_CUDA(cudaEventRecord(c->join_ev, ms.side));
+  if (split) TRY_CUDA(cudaEventRecord(c->join2_ev, ms.side2));
   // the per-set IND-CPA launches of a step run side by side on the context's
   // lanes (forked from s and joined back), so one set's last wave overlaps
   // the next set's launch
@@ -1809,14 +1760,15 @@ int mixed_enqueue(tmvp_ctx *c, size_t ng, const tmvp_dec_group *gr, uint8_t *ws,
   nsets = r1;
   {
     StageTimer tm_(c, "mix_g", s);
-    k_mix_g<<<nb, kHashBlock, 0, s>>>(th, (int)ng, total);
+    TRY_CUDA(launch_mix_g(hash_cfg(c), th, (int)ng, (size_t)total, gp, s));
   }
   TRY_CUDA(cudaStreamWaitEvent(s, c->join_ev, 0));  // GenMatrix
+  if (split) TRY_CUDA(cudaStreamWaitEvent(s, c->join2_ev, 0));
   int r2 = per_set(kReenc, sb, tre);
   if (r2 < 0) return r2;
   {
     StageTimer tm_(c, "mix_final", s);
-    k_mix_final<<<nb, kHashBlock, 0, s>>>(th, (int)ng, total);
+    TRY_CUDA(launch_mix_final(hash_cfg(c), th, (int)ng, (size_t)total, s));
   }
   c->launches += 3 + 2 * nsets;
   TRY_CUDA(cudaGetLastError());
@@ -1888,7 +1840,7 @@ int mixed_enqueue_chains(tmvp_ctx *c, size_t ng, const tmvp_dec_group *gr, int c
     cudaStream_t cs = c->lane[k * nl];
     TRY_CUDA(cudaStreamWaitEvent(cs, c->gm_ev, 0));
     int r = mixed_enqueue(c, part.size(), part.data(), wk, tab_ptrs[k], host_tabs[k], upload_tabs, cs,
-                          MixStreams{c->lane_side[k], k * nl, nl});
+                          MixStreams{c->lane_side[k], c->lane_side2[k], k * nl, nl});
     if (r) return r;
   }
   for (int k = 0; k < chains; k++) {

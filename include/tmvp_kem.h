@@ -220,24 +220,26 @@ int tmvp_ctx_set_dev_chunk(tmvp_ctx *ctx, size_t n);
  * timing (tmvp_ctx_set_timing) measures each kernel alone on the GPU.  Slower;
  * for measurement.  Results do not depend on it.  Default 0. */
 int tmvp_ctx_set_serial(tmvp_ctx *ctx, int on);
-/* Caps the Keccak front of decapsulation (GenMatrix + H(c), one launch beside
- * the decryption) at blocks_per_sm 64-thread blocks per SM, its threads then
- * striding over the sponges, so that decryption CTAs fit beside it on every
- * SM; 0 (the default) launches one thread per sponge.  0..64.  Results do
- * not depend on it. */
+/* Caps the Keccak front of decapsulation (GenMatrix + H(c), beside the
+ * decryption) at about blocks_per_sm 64-thread blocks (half as many of 128
+ * threads) resident per SM, so that decryption CTAs fit beside it on every SM;
+ * 0 (the default) leaves it to the library.  0..64.  Results do not depend on
+ * it. */
 int tmvp_ctx_set_front_cap(tmvp_ctx *ctx, int blocks_per_sm);
-/* The form of each Keccak launch (GenMatrix, GenSecret, H, G, the final
- * key).  Launches of at most warp_hash sponges run one warp per sponge, the
- * state spread over the warp's lanes (~2.1 us per permutation while the GPU
- * is far from full); larger ones of at most pair_hash sponges run two threads
- * per sponge, each holding half of every state lane (~3.3 us per permutation
- * up to ~10 K sponges); larger ones one thread per sponge (~4.7 us per
- * permutation, the best rate once the GPU is full).  Launches of short
- * sponges (G, the final key, the key-generation tail) count four times
- * against warp_hash and twice against pair_hash.  Defaults 1024 and 32768;
- * 0 turns a form off.  Results do not depend on them.  No counterpart in the reference, whose hash kernels run as one
- * block of one thread per instance
- * (TMVP-Saber/SABER-GPU/src/cuda_kernel.cu:116-127). */
+/* The form of each Keccak launch (GenMatrix, GenSecret, H, G, the final key):
+ * one warp per sponge, the state spread over the warp's lanes (~2.0 us per
+ * permutation while the GPU is far from full); two threads per sponge, each
+ * holding half of every state lane (~2.9 us per permutation up to ~10 K
+ * sponges); or one thread per sponge (~4.7 us per permutation, the best rate
+ * once the GPU is full).  By default the library chooses per role of a launch
+ * by its number of sponges.  Once either limit is set, launches of at most
+ * warp_hash sponges run one warp per sponge, larger ones of at most pair_hash
+ * sponges two threads, larger ones one thread; launches of short sponges (G,
+ * the final key, the key-generation tail) count four times against warp_hash
+ * and twice against pair_hash.  The other limit keeps its initial value (1024,
+ * 32768); 0 turns a form off.  Results do not depend on them.  No counterpart
+ * in the reference, whose hash kernels run as one block of one thread per
+ * instance (TMVP-Saber/SABER-GPU/src/cuda_kernel.cu:116-127). */
 int tmvp_ctx_set_warp_hash(tmvp_ctx *ctx, size_t max_sponges);
 int tmvp_ctx_set_pair_hash(tmvp_ctx *ctx, size_t max_sponges);
 
