@@ -65,6 +65,14 @@ int cpa_launch(int form, int op, const CpaArgs &a, void *stream);
 // is implied): ceil(n / per-CTA count) CTAs.
 int cpa_launch_decrypt_onekey(const CpaArgs &a, void *stream);
 
+// Re-encryption of b.n ciphertexts under one key as one matrix product
+// (cpa_onekey.cuh).  ops: onekey_operand_bytes of device memory, filled by
+// onekey_prep from the key's GenMatrix stream and packed b.  b.msg has stride
+// 64.
+size_t onekey_operand_bytes(const KemParams &P);
+int onekey_prep(const KemParams &P, const uint8_t *a_stream, const uint8_t *b_stream, uint8_t *ops, void *stream);
+int onekey_reenc(const CpaArgs &b, const uint8_t *ops, int sms, void *stream);
+
 // tcgen05 form only: one persistent launch over `ngroups` (<= kMixMaxGroups)
 // groups of instances, each with its own parameter set and buffers.  groups:
 // host copies; dev_tab: the same groups as a device table (mix_table_build

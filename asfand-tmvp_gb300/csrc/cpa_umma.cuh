@@ -72,6 +72,19 @@ __device__ __forceinline__ void umma_f8(uint32_t d_tmem, uint64_t adesc, uint64_
       : "memory");
 }
 
+// The same issued by the threads with `issue` set: one of a warp that computes
+// the operands together, so that the descriptors stay in uniform registers.
+__device__ __forceinline__ void umma_f8_if(bool issue, uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                           uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"((uint32_t)issue)
+      : "memory");
+}
+
 __device__ __forceinline__ void umma_commit(uint32_t mbar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar)
                : "memory");
@@ -143,6 +156,30 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t mbar, uint32_t parity
   for (uint32_t it = 0; it < (1u << 22); it++) {
     if (mbar_try_wait_sleep(mbar, parity, 20000u)) return true;
     if ((it & 15u) == 15u && global_ns() - t0 > 2000000000ull) return false;
+  }
+  return false;
+}
+
+// The same bound, polling without sleeping: for one thread whose wait is short
+// and on whose wake-up others depend.
+__device__ __forceinline__ bool mbar_spin_bounded(uint32_t mbar, uint32_t parity) {
+  auto test = [&] {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(ok)
+        : "r"(mbar), "r"(parity)
+        : "memory");
+    return ok != 0;
+  };
+  for (int i = 0; i < 64; i++)
+    if (test()) return true;
+  const uint64_t t0 = global_ns();
+  for (uint32_t it = 0; it < (1u << 28); it++) {
+    if (test()) return true;
+    if ((it & 1023u) == 1023u && global_ns() - t0 > 2000000000ull) return false;
   }
   return false;
 }

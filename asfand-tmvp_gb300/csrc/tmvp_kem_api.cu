@@ -464,6 +464,16 @@ DecScratch dec_scratch(const KemParams &P, size_t n, Arena &A) {
   return w;
 }
 
+// Whether the re-encryption of n ciphertexts under one key runs as one matrix
+// product (cpa_onekey.cuh), which pays for digit planes of the key and takes
+// its ciphertexts 128 at a time.  One-key decapsulation, matrix / per-instance
+// re-encryption (us): Saber 65536: 455 / 630, 16384: 151 / 197, 8192: 99 / 112,
+// 6000: 97 / 101, 4096: 87 / 84; FireSaber 6000: 147 / 145, 5000: 145 / 138;
+// LightSaber 4096: 61 / 64.
+// The planes (at most 444,416 bytes) go where the expanded A of the n instances
+// (1408 bytes or more each) would: no pass needs more workspace for them.
+inline bool onekey_matrix(size_t n) { return n >= 6144; }
+
 // Decapsulation of n instances in device memory (16-byte aligned): GenMatrix
 // and H(c) in one launch (2n sponges, so the integer pipe has warps enough)
 // on the high-priority side stream, concurrent with the decryption and G on
@@ -471,7 +481,7 @@ DecScratch dec_scratch(const KemParams &P, size_t n, Arena &A) {
 int dec_pipeline(tmvp_ctx *c, const KemParams &P, size_t n, uint8_t *ss, const uint8_t *ct,
                  const uint8_t *sk, int form, cudaStream_t s, const DecScratch &w, bool fork = true,
                  cudaStream_t side = nullptr, const uint8_t *a_cached = nullptr,
-                 cudaEvent_t a_ready = nullptr, bool key_shared = false) {
+                 cudaEvent_t a_ready = nullptr, bool key_shared = false, const uint8_t *key_ops = nullptr) {
   int r;
   if (!side) side = c->side;
   if (c->serial) {  // each stage alone on s (measurement: isolated stage durations)
@@ -493,10 +503,12 @@ int dec_pipeline(tmvp_ctx *c, const KemParams &P, size_t n, uint8_t *ss, const u
       if (side == c->lane_side[l]) side2 = c->lane_side2[l];
     TRY_CUDA(cudaStreamWaitEvent(side2, c->fork_ev, 0));
   }
+  const bool matrix = key_ops && onekey_matrix(n);
   {
     StageTimer tm_(c, "dec_front", side);
     TRY_CUDA(launch_dec_front(h, P, sk, ct, w.a_stream, w.hc, n, !a_cached, side, side2));
   }
+  if (matrix) TRY_CUDA(cudaMemsetAsync(w.fail, 0, n, side));
   TRY_CUDA(cudaEventRecord(c->join_ev, side));
   if (split) TRY_CUDA(cudaEventRecord(c->join2_ev, side2));
   c->launches++;
@@ -540,7 +552,14 @@ int dec_pipeline(tmvp_ctx *c, const KemParams &P, size_t n, uint8_t *ss, const u
   b.msg_stride = 64;
   b.ct = ct;
   b.fail = w.fail;
-  if ((r = run_cpa(c, form, kReenc, b, s))) return r;
+  if (matrix) {
+    StageTimer tm_(c, "cpa_reenc_onekey_fp8_tcgen05", s);
+    b.err = c->d_err;
+    c->launches++;
+    if (onekey_reenc(b, key_ops, c->nsm, s)) return TMVP_EDEVICE;
+  } else if ((r = run_cpa(c, form, kReenc, b, s))) {
+    return r;
+  }
   {
     StageTimer tm_(c, "final_key", s);
     TRY_CUDA(launch_final_key(hash_cfg(c), P, ct, w.hc, w.kr, w.fail, sk, key_shared ? 0 : (size_t)P.sk_bytes, ss, n, s));
@@ -1031,7 +1050,7 @@ int tmvp_kem_dec_batch_onekey(tmvp_ctx *c, tmvp_param_set set, size_t n, uint8_t
     for (int k = 0; k < NS; k++) slot_ct[k] = A.take(cn * P.ct_bytes);
     if (bss.host)
       for (int l = 0; l < NL; l++) ss_stage[l] = A.take(cn * 32);
-    uint8_t *a_one = A.take(P.gm_bytes);
+    uint8_t *a_one = A.take(P.gm_bytes), *ops = onekey_matrix(cn) ? w[0].a_stream : nullptr;  // (lanes share them)
     stage_assign(bsk, A);
     if ((r = upload(bsk, s))) return set_err(r);
     TRY_CUDA(cudaEventRecord(c->fork_ev, s));
@@ -1040,8 +1059,9 @@ int tmvp_kem_dec_batch_onekey(tmvp_ctx *c, tmvp_param_set set, size_t n, uint8_t
     {
       StageTimer tm_(c, "genmatrix", c->side);
       TRY_CUDA(launch_genmatrix(hash_cfg(c), P, bsk.dev + P.indcpa_sk_bytes, 0, a_one, 1, c->side));
+      if (ops && onekey_prep(P, a_one, bsk.dev + P.indcpa_sk_bytes, ops, c->side)) return set_err(TMVP_EDEVICE);
     }
-    c->launches++;
+    c->launches += ops ? 2 : 1;
     TRY_CUDA(cudaEventRecord(c->gm_ev, c->side));
     for (size_t off = 0, k = 0, m = 0; off < n; off += m, k++) {
       const size_t ck = k < (size_t)c->host_ramp ? std::max<size_t>(cn >> (c->host_ramp - k), 256) : cn;
@@ -1055,7 +1075,7 @@ int tmvp_kem_dec_batch_onekey(tmvp_ctx *c, tmvp_param_set set, size_t n, uint8_t
       TRY_CUDA(cudaStreamWaitEvent(ls, c->ev_loaded[sl][0], 0));
       uint8_t *ss_k = bss.host ? ss_stage[ln] : bss.dev + off * 32;
       if ((r = dec_pipeline(c, P, m, ss_k, slot_ct[sl], bsk.dev, form, ls, w[ln], true, c->lane_side[ln], a_one,
-                            c->gm_ev, true)))
+                            c->gm_ev, true, ops)))
         return set_err(r);
       TRY_CUDA(cudaEventRecord(c->ev_free[sl], ls));
       if (bss.host)
@@ -1079,6 +1099,7 @@ int tmvp_kem_dec_batch_onekey(tmvp_ctx *c, tmvp_param_set set, size_t n, uint8_t
   Arena A{c->ws};
   DecScratch w = dec_scratch(P, n, A);
   uint8_t *a_one = A.take(P.gm_bytes);
+  uint8_t *ops = shared && onekey_matrix(n) ? w.a_stream : nullptr;
   uint8_t *sk_rep = shared ? nullptr : A.take(n * P.sk_bytes), *a_rep = shared ? nullptr : A.take(n * P.gm_bytes);
   stage_assign(bss, A);
   stage_assign(bct, A);
@@ -1094,6 +1115,7 @@ int tmvp_kem_dec_batch_onekey(tmvp_ctx *c, tmvp_param_set set, size_t n, uint8_t
   {
     StageTimer tm_(c, "genmatrix", gs);
     TRY_CUDA(launch_genmatrix(hash_cfg(c), P, bsk.dev + P.indcpa_sk_bytes, 0, a_one, 1, gs));
+    if (ops && onekey_prep(P, a_one, bsk.dev + P.indcpa_sk_bytes, ops, gs)) return set_err(TMVP_EDEVICE);
     if (!shared)
       k_replicate16<<<grid, 256, 0, gs>>>(reinterpret_cast<uint4 *>(a_rep), reinterpret_cast<const uint4 *>(a_one),
                                           P.gm_bytes / 16, n);
@@ -1104,9 +1126,9 @@ int tmvp_kem_dec_batch_onekey(tmvp_ctx *c, tmvp_param_set set, size_t n, uint8_t
     k_replicate16<<<grid, 256, 0, s>>>(reinterpret_cast<uint4 *>(sk_rep), reinterpret_cast<const uint4 *>(bsk.dev),
                                        P.sk_bytes / 16, n);
   }
-  c->launches += shared ? 1 : 3;
+  c->launches += shared ? (ops ? 2 : 1) : 3;
   if ((r = dec_pipeline(c, P, n, bss.dev, bct.dev, shared ? bsk.dev : sk_rep, form, s, w, true, nullptr,
-                        shared ? a_one : a_rep, c->gm_ev, shared)))
+                        shared ? a_one : a_rep, c->gm_ev, shared, ops)))
     return set_err(r);
   if ((r = download(bss, s))) return set_err(r);
   return set_err(finish(c, s, bss.host));
