@@ -5,9 +5,9 @@
 // Per instance:
 //   1. the packed inputs arrive by TMA bulk copies (cp.async.bulk) issued by
 //      one thread, counted on an mbarrier;
-//   2. secrets (CBD or unpacked) straight into s_ext, radix-16 digit columns
-//      (r16_digits, raw e4m3 bytes worth digit * 2^-9) with K reversed, then
-//      the Hankel core matrices (cpa_umma.cuh);
+//   2. radix-16 digit columns (r16_digits, raw e4m3 bytes worth digit * 2^-9)
+//      with K reversed, and the secrets (CBD or unpacked) in registers, from
+//      there the Hankel core matrices (cpa_umma.cuh);
 //   3. one thread issues the 4 l tcgen05.mma (M = 128, N = 16 .. 64, K = 32;
 //      each even tile of the Hankel sequence serves four K steps through the
 //      negacyclic wrap) into tensor memory and commits them to an mbarrier;
@@ -74,16 +74,19 @@ constexpr int al16c(int x) { return (x + 15) & ~15; }
 // an instance; tensor memory is read by warps w and w + 4 (two M halves).
 constexpr int kI5Threads = 256;
 
-// Rows of the Hankel core matrices that one thread makes from one window of
-// s_ext: 6 rows take 4 128-bit loads and 14 byte permutes (2 rows at a time,
-// from one copy of s_ext, took 3 x 2 loads, 3 x 7 selects for the odd
-// windows and 3 x 6 permutes for Saber's three polynomials).
-constexpr int kHankelRun = 6;
+// Where a layout puts the packed GenMatrix and b streams, the sums that warps
+// exchange and the packed outputs: outside the Hankel core matrices (kFree: the
+// core matrices are written as soon as the secrets are read, and the next
+// instance's copies start beside the MMAs), or over them (kLate: they wait until
+// the streams are read).  kFree is the faster one at the same number of CTAs
+// per SM (LightSaber 65536, us: re-encryption 238 -> 227, key generation 258 ->
+// 238), but not at one less (Saber 276 -> 281, FireSaber 390 -> 436).
+enum InputPlace { kFree, kLate };
 
-// Shared-memory layout of one CTA (byte offsets).  The operand region ENG
-// holds the Hankel core matrices H (l x kHankelBytes5), the digit columns B
-// and s_ext; the packed GenMatrix / GenSecret / b streams and the packed
-// secret key are only read before H is written, so they land inside H.
+// Shared-memory layout of one CTA (byte offsets): the Hankel core matrices H
+// (l x HJ), the digit columns BM, the packed secrets (GenSecret stream, secret
+// key or matvec secrets), streams and epilogue buffers (InputPlace), ciphertext
+// and message.
 //
 // Digit columns of one j: K step t is 32 K rows (K reversed), two 16-byte K
 // chunks, in blocks of two steps: column 2n + (t & 1) of a block, PG groups of
@@ -93,8 +96,8 @@ constexpr int kHankelRun = 6;
 // and one a block later (0, 1 | -4, -5).
 // The strides put the 16-byte pieces that a store instruction writes at once
 // into different banks.
-template <int OP, int SET>
-struct LayoutC {
+template <int OP, int SET, InputPlace IP>
+struct LayoutAt {
   using C = SetC<SET>;
   using S = ShapeC<OP, SET>;
   static constexpr bool HAS_AS = OP == kEncrypt || OP == kReenc || OP == kKeygen;
@@ -109,19 +112,12 @@ struct LayoutC {
   static constexpr bool HAS_MV = OP == kMatvec;
   static constexpr int MV_A = C::L * C::L * 512, MV_S = C::L * 256;
   // Hankel core matrices per secret polynomial: tiles start at block w of 32
-  // rows (core 4w, w <= 6) and reach 15 row groups and two K chunks on; in
-  // whole runs of kHankelRun rows a thread
+  // rows (core 4w, w <= 6) and reach 15 row groups and two K chunks on
   static constexpr int CORES = 42;
-  static constexpr int PAIRS = CORES / kHankelRun;  // 8-thread groups per polynomial
-  static_assert(CORES % kHankelRun == 0 && C::L * PAIRS <= kI5Threads / 8, "one run per thread");
-  // s_ext of one j: 96 words (what the cores read), and the same one word on,
-  // EXC bytes after the first (4 of 8 16-byte units apart in the banks)
-  static constexpr int EXC = 448, EXJ = 2 * EXC;
-  static_assert(4 * (2 * (CORES - kHankelRun) + 16) <= 384, "the loads stay inside one copy");
-  static constexpr int HJ = CORES * 128;
-  static constexpr int LB = 160;
-  static constexpr int SB = S::NC4 == 16 ? 304 : 288;
-  static constexpr int QB = 16 * (S::NC4 == 16 ? 234 : (S::NC4 == 12 ? 164 : (S::NC4 == 8 ? 114 : 60)));  // one sequence, padded
+  static constexpr int CS = 144, HJ = CORES * CS;  // (a core is 128 bytes; the stride spreads equal rows of 8 cores over the banks)
+  static constexpr int LB = !HAS_AS || S::NC4 != 16 ? 160 : 128;
+  static constexpr int SB = S::NC4 != 16 ? 288 : (HAS_AS ? 272 : 304);
+  static constexpr int QB = 16 * (S::NC4 == 16 ? (HAS_AS ? 206 : 234) : (S::NC4 == 12 ? 164 : (S::NC4 == 8 ? 114 : 60)));  // one sequence, padded
   static_assert(QB >= 3 * S::PG * SB, "a sequence's three blocks");
   static constexpr int BJ = 2 * QB;  // digit columns of one j
   // byte offset of step t's columns within one j, and of their negated copy (t >= 4)
@@ -133,46 +129,58 @@ struct LayoutC {
   }
   // byte offset of digit column n from there
   __host__ __device__ static constexpr int col_off(int n) { return (n >> 2) * SB + (n & 3) * 32; }
-  static constexpr int ENG = 0;
-  static constexpr int H = ENG;
-  static constexpr int A = H;                                    // streams inside H
-  static constexpr int SS = HAS_AS ? al16c(A + C::GM + 16) : (HAS_MV ? al16c(A + MV_A) : A);
-  static constexpr int B = HAS_AS ? al16c(SS + C::GS + 16) : SS;
-  static constexpr int SKO = H;
+  // accumulator sums that another warp finishes: two 16-bit values a word, the last odd one by itself
+  static constexpr int XWORDS = S::R / 2, XBYTES = al16c(S::R * 512);
+  static constexpr int H = 0;
   static constexpr int BM = H + C::L * HJ;
-  static constexpr int EXT = BM + C::L * BJ;
-  static constexpr int ENG_END_OPS = EXT + C::L * EXJ;
-  static constexpr int ENG_BYTES = ENG_END_OPS;
+  static constexpr int SS = BM + C::L * BJ, SKO = SS;  // packed secrets
+  static constexpr int SS_BYTES = HAS_AS ? C::GS : (HAS_SK ? C::INDCPA_SK : MV_S);
+  static constexpr InputPlace PLACE = IP;
+  static constexpr int OUT_BYTES = OP == kEncrypt ? C::CT + 16
+                                   : (OP == kKeygen ? C::L * C::POLYCOMP + C::INDCPA_SK + 16 : 0);
+  static constexpr int A_BYTES = al16c(HAS_AS ? C::GM + 16 : (HAS_MV ? MV_A : 0));
+  static constexpr int STREAMS = al16c(A_BYTES + (HAS_B ? C::L * C::POLYCOMP + 16 : 0));
+  static constexpr int FREE0 = al16c(SS + SS_BYTES + 16);  // past the secrets
+  static constexpr int A = IP == kFree ? FREE0 : H;
+  static constexpr int B = A + A_BYTES;
+  static constexpr int XCH = A + STREAMS, OUT = XCH + XBYTES;
+  static_assert(IP != kLate || OUT + OUT_BYTES <= BM, "streams and epilogue buffers fit H");
   // the output ops' 16-bit values (R x 8 runs of 80 bytes), over the digit
   // columns (the next instance's inputs are landing in H)
   static constexpr int VALS = BM;
   static_assert(HAS_CT || HAS_MV || S::R * 640 <= C::L * BJ, "epilogue values fit the digit columns");
   // ciphertext and message, read until the end of an instance: two buffers of
   // CTB bytes, so that the next instance's copies land beside them
-  static constexpr int CTO = al16c(ENG + ENG_BYTES);
+  static constexpr int CTO = IP == kLate ? FREE0 : al16c(OUT + OUT_BYTES);
   static constexpr int MSG = HAS_CT ? al16c(CTO + NCT * CTS) : CTO;
   static constexpr int CTB = (HAS_B ? al16c(MSG + 32 + 16) : MSG) - CTO;
   static constexpr int SEC8 = CTO + 2 * CTB;
-  // Epilogue buffers inside H, past the inputs of the next instance that are
-  // landing there (the MMAs have read H; the next instance writes its core
-  // matrices after a barrier that follows the epilogue): accumulator sums that
-  // another warp finishes, and the packed outputs.
-  static constexpr int XWORDS = (S::R + 1) / 2;
-  static constexpr int XCH = HAS_AS ? al16c(B + (HAS_B ? C::L * C::POLYCOMP + 16 : 16))
-                                    : (HAS_SK ? al16c(SKO + C::INDCPA_SK + 16) : al16c(SS + MV_S + 16));
-  static constexpr int OUT = XCH + XWORDS * 1024;
-  static constexpr int OUT_BYTES = OP == kEncrypt ? C::CT + 16
-                                   : (OP == kKeygen ? C::L * C::POLYCOMP + C::INDCPA_SK + 16 : 0);
   // mbarriers in, mma, clc; TMEM base; the next instance; two CLC responses
-  static_assert(OUT + OUT_BYTES <= H + C::L * HJ, "the epilogue buffers fit H");
   static constexpr int BAR = al16c(SEC8 + (OP == kKeygen ? C::L * 256 : 0));
   static constexpr int TOTAL = BAR + 64;
+  static constexpr int CTAS = (228 * 1024) / (TOTAL + 1024);  // that shared memory admits
   static constexpr int IN_BYTES = (HAS_AS ? C::GM + C::GS : 0) + (HAS_B ? C::L * C::POLYCOMP + 32 : 0) +
                                   (HAS_CT ? C::CT : 0) + (HAS_SK ? C::INDCPA_SK : 0) + (HAS_MV ? MV_A + MV_S : 0);
-  static_assert(!HAS_AS || B + (HAS_B ? C::L * C::POLYCOMP + 16 : 0) <= BM, "streams fit inside H");
-  static_assert(!HAS_SK || C::INDCPA_SK + 16 <= C::L * HJ, "secret key fits inside H");
-  static_assert(!HAS_MV || SS + MV_S + 16 <= BM, "matvec inputs fit inside H");
 };
+
+// CTAs per SM that the registers admit without spilling more than a few words:
+// 8 of 32 registers (decryption), 6 of 40, and 5 of 48 where a thread loads 32
+// accumulator columns.
+template <int OP, int SET>
+constexpr int reg_ctas() {
+  return ShapeC<OP, SET>::NC4 == 16 ? 5 : (OP == kDecrypt ? 8 : 6);
+}
+
+// The layout of an operation: the first place that costs no resident CTA.
+template <int OP, int SET>
+constexpr InputPlace input_place() {
+  if (OP == kDecrypt || OP == kDecryptK) return kFree;  // (no streams)
+  constexpr int free = LayoutAt<OP, SET, kFree>::CTAS, late = LayoutAt<OP, SET, kLate>::CTAS,
+                cap = reg_ctas<OP, SET>();
+  return free >= (late < cap ? late : cap) ? kFree : kLate;
+}
+template <int OP, int SET>
+using LayoutC = LayoutAt<OP, SET, input_place<OP, SET>()>;
 
 // Eight W-bit little-endian fields from byte `byte0` (16 bytes of slack after
 // the stream), as four words of two 16-bit lanes.
@@ -259,28 +267,51 @@ __device__ __forceinline__ uint2 raw_digits8(const uint32_t (&X)[4], int d) {
   return make_uint2(a & mask, b & mask);
 }
 
-// The Hankel core matrices of the L polynomials (row x = 8m + i of core m,
-// s_ext[x .. x + 15], at byte 16x of H + j * HJ).  Eight threads (four byte
-// shifts sh, two parities) make the rows of kHankelRun consecutive cores;
-// thread (sh, par) the rows 4q + sh, q = 2m + par, windows of s_ext words
-// that start at q: from the copy of s_ext one word on for par = 1, so that
-// every window starts on a 16-byte boundary.
-template <class LO, int L>
-__device__ __forceinline__ void stage_hankel6(uint32_t H, uint32_t ext, int tid) {
-  const int item = tid >> 3;
-  if (item >= L * LO::PAIRS) return;
-  const int sh = tid & 3, par = (tid >> 2) & 1, j = item / LO::PAIRS, m0 = (item % LO::PAIRS) * kHankelRun;
-  const uint32_t sel = 0x3210u + 0x1111u * (uint32_t)sh;
-  const uint32_t e = ext + (uint32_t)(j * LO::EXJ + par * LO::EXC + 8 * m0);
-  constexpr int NP = 2 * kHankelRun + 2;  // permuted words
-  uint32_t w[NP + 2];
+// Words 2g .. 2g + 5 of one polynomial's s_ext (s_ext[d] = -s[d + 1] for
+// d < 255, s[d - 255] from there on) in lane g, from its coefficients 8g .. 8g + 7
+// (e0, e1: raw e4m3 bytes).
+__device__ __forceinline__ void secret_windows(uint32_t e0, uint32_t e1, int g, uint32_t (&w)[6]) {
+  constexpr uint32_t n = 0x80808080u;
+  const uint32_t nx = __shfl_sync(0xffffffffu, e0, (g + 1) & 31);
+  w[0] = __byte_perm(e0, e1, 0x4321) ^ n;
+  w[1] = __byte_perm(e1, nx, 0x4321) ^ (g == 31 ? 0x00808080u : n);  // s_ext[255] = s[0] keeps its sign
 #pragma unroll
-  for (int i = 0; i < NP + 2; i += 4) lds128(e + 4 * i, w[i], w[i + 1], w[i + 2], w[i + 3]);
+  for (int i = 1; i <= 2; i++) {  // (past word 63: s_ext[256 + d] = -s_ext[d])
+    const uint32_t f = g + i >= 32 ? n : 0u;
+    w[2 * i] = __shfl_sync(0xffffffffu, w[0], (g + i) & 31) ^ f;
+    w[2 * i + 1] = __shfl_sync(0xffffffffu, w[1], (g + i) & 31) ^ f;
+  }
+}
+
+// The Hankel core matrices of one polynomial, by a warp (row i of core m,
+// s_ext[8m + i .. 8m + i + 15], at byte CS m + 16i of h): lane g makes core g
+// from its windows, and lanes 0 .. 9 also core 32 + g, which is minus core g.
+// The windows by way of shared memory, eight threads to six cores, took 84 more
+// wavefronts of loads for an instance of Saber, on a port that the MMAs' operand
+// reads and these stores keep busy, one more barrier for the decryption, and
+// 0.9 KB of shared memory a polynomial.  65536 instances, us: Saber's decryption
+// 203 -> 169, re-encryption 281 -> 271, encryption 291 -> 285, key generation
+// 303 -> 302; FireSaber's re-encryption 461 -> 380 (four CTAs per SM, not
+// three), LightSaber's 236 -> 216.  (Cores 128 bytes apart, rows in a
+// lane-dependent order against bank conflicts: decryption 179, encryption 294.)
+template <class LO>
+__device__ __forceinline__ void stage_hankel(uint32_t h, const uint32_t (&w)[6], int g) {
+  const uint32_t core = h + (uint32_t)(LO::CS * g);
 #pragma unroll
-  for (int i = 0; i < NP; i++) w[i] = __byte_perm(w[i], w[i + 1], sel);
-  const uint32_t h = H + (uint32_t)(j * LO::HJ + 128 * m0 + 64 * par + 16 * sh);
+  for (int sh = 0; sh < 4; sh++) {
 #pragma unroll
-  for (int r = 0; r < kHankelRun; r++) sts128(h + 128 * r, w[2 * r], w[2 * r + 1], w[2 * r + 2], w[2 * r + 3]);
+    for (int par = 0; par < 2; par++) {
+      uint32_t o[4];
+#pragma unroll
+      for (int k = 0; k < 4; k++) o[k] = sh ? __funnelshift_r(w[par + k], w[par + k + 1], 8 * sh) : w[par + k];
+      const uint32_t at = core + (uint32_t)(64 * par + 16 * sh);
+      sts128(at, o[0], o[1], o[2], o[3]);
+      if (g < LO::CORES - 32) {
+        constexpr uint32_t n = 0x80808080u;
+        sts128(at + 32 * LO::CS, o[0] ^ n, o[1] ^ n, o[2] ^ n, o[3] ^ n);
+      }
+    }
+  }
 }
 
 // Digit columns of 32 coefficients of one W-bit packed polynomial: lane m
@@ -379,6 +410,21 @@ __device__ __forceinline__ uint32_t clc_answer(uint32_t resp) {
   return x;
 }
 
+// The CTA's barrier, whether the predicate held in all threads: the threads may
+// come to it from different branches.
+__device__ __forceinline__ bool bar_and(bool p) {
+  uint32_t r;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.b32 p, %1, 0;\n\t"
+      "bar.red.and.pred q, 0, p;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}\n"
+      : "=r"(r)
+      : "r"((uint32_t)p)
+      : "memory");
+  return r != 0;
+}
+
 // The input copies of instance inst into ciphertext / message buffer cb
 // (0 or CTB), counted on mbar (one thread).  kDecryptK: ciphertexts
 // inst * NCT .. of the one key.
@@ -449,8 +495,13 @@ __device__ __forceinline__ uint32_t combine5(const uint32_t (&f)[2 * ShapeC<OP, 
 // memory and barriers are set up once, and the next instance's input copies
 // run beside the epilogue of this one.  Without that, an empty instance (no
 // staging, no MMAs) took 0.207 of the decryption's 0.273 ms at 65536; with it
-// 0.090 of 0.246 (re-encryption 0.353 -> 0.342), and what bounds the kernel is
-// its MMAs (0.217 ms for the decryption's 24 alone).
+// 0.090 of 0.246 (re-encryption 0.353 -> 0.342).
+//
+// What bounds the kernel now: the shared-memory port and the instruction
+// slots, each about 60 % busy, in phases that only other CTAs overlap (65536
+// Saber, us, decryption / re-encryption: 203 / 281 before the core matrices came
+// from registers; without the MMAs 153 / 240, without the core matrices 154 /
+// 243, without the digits 185 / 209, inputs from L2 203 / 281).
 template <int OP, int SET, class AT>
 __device__ __forceinline__ void cpa5i_run(const AT &at, uint8_t *sm) {
   using C = SetC<SET>;
@@ -479,7 +530,6 @@ __device__ __forceinline__ void cpa5i_run(const AT &at, uint8_t *sm) {
   const uint32_t tmem = *reinterpret_cast<volatile uint32_t *>(tmem_slot);
   uint32_t *sec8w = reinterpret_cast<uint32_t *>(sm + LO::SEC8);
   uint8_t *H = sm + LO::H, *Bm = sm + LO::BM;
-  const uint32_t ext32 = smem_u32(sm + LO::EXT);
   unsigned gi = blockIdx.x;
   for (uint32_t it = 0;; it++) {
   // per-thread values are made afresh for every instance (not kept across the
@@ -498,87 +548,8 @@ __device__ __forceinline__ void cpa5i_run(const AT &at, uint8_t *sm) {
     clc_try_cancel(clc_resp + 16 * par, mbar_clc);
   }
   bool ready = mbar_wait_bounded(mbar_in, par);
-  bool ok = true;
   if (ready) {
-    // 1. secrets, straight into s_ext (s_ext[d] = -s[d + 1] for d < 255,
-    // s[d - 255] for 255 <= d; the first 96 words, twice).  Warp
-    // j < L makes polynomial j: lane g encodes the words 2g, 2g + 1
-    // (coefficients 8g..8g+7) and takes word 2g + 2 from the next lane
-    // (word 0 for lane 31).
-    // the secrets of j go to a warp that makes no digit columns where one is free
-    const int sj = S::R == 1 ? warp - L : (warp - S::R + 8) % 8;
-    if (sj >= 0 && sj < L) {
-      const int j = sj, g = lane;
-      uint32_t sb[2];
-      if (IS_DEC && !C::SABLE) {
-        // 13-bit two's complement (SABER pack.cu:53-84)
-        constexpr uint32_t m = ((1u << C::EQ) - 1u) * 0x10001u;
-        uint32_t X[4];
-        unpack8c<C::EQ>(sm + LO::SKO, (32 * j + g) * C::EQ, X);
-        uint32_t bad = 0;
-#pragma unroll
-        for (int i = 0; i < 4; i++) bad |= ((X[i] + 0x00800080u) & m) & 0xFF00FF00u;
-        ok = bad == 0u;
-        sb[0] = __byte_perm(X[0], X[1], 0x6420);
-        sb[1] = __byte_perm(X[2], X[3], 0x6420);
-      } else {
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-          const int w = 64 * j + 2 * g + h;
-          if (OP == kMatvec) {
-            sb[h] = lds32(smem_u32(sm + LO::SS) + 4 * w);  // four int8 coefficients
-          } else if (IS_DEC) {
-            // 2-bit two's complement (SABLE pack.cu:371-376): one byte = 4 coefficients
-            const uint32_t x = sm[LO::SKO + w];
-            const uint32_t spread = (x & 3u) | ((x & 0xcu) << 6) | ((x & 0x30u) << 12) | ((x & 0xc0u) << 18);
-            sb[h] = spread | (((spread >> 1) & 0x01010101u) * 0xfcu);
-          } else if (C::MU == 8) {
-            // CBD mu = 8 (SABER poly.cu:864-887)
-            const uint32_t x = lds32(smem_u32(sm + LO::SS) + 4 * w);
-            uint32_t n = x - ((x >> 1) & 0x55555555u);
-            n = (n & 0x33333333u) + ((n >> 2) & 0x33333333u);
-            sb[h] = __vsub4(n & 0x0f0f0f0fu, (n >> 4) & 0x0f0f0f0fu);
-          } else if (C::MU == 2) {
-            // CBD mu = 2 (SABLE fips202.cu:625-651)
-            const uint32_t x = sm[LO::SS + w];
-            const uint32_t spread = (x & 3u) | ((x & 0xcu) << 6) | ((x & 0x30u) << 12) | ((x & 0xc0u) << 18);
-            sb[h] = __vsub4(spread & 0x01010101u, (spread >> 1) & 0x01010101u);
-          } else {
-            // CBD mu = 6, 10: fields of mu bits, popcount halves
-            uint32_t r = 0;
-#pragma unroll
-            for (int b = 0; b < 4; b++) {
-              const uint32_t x = get_bits(sm + LO::SS, (4 * w + b) * C::MU, C::MU);
-              const int v = __popc(x & ((1u << (C::MU / 2)) - 1u)) - __popc(x >> (C::MU / 2));
-              r |= ((uint32_t)v & 0xffu) << (8 * b);
-            }
-            sb[h] = r;
-          }
-        }
-      }
-      // (CBD secrets are at most mu / 2 <= 5 in magnitude)
-      if (IS_DEC || OP == kMatvec) ok = ok && small4(sb[0]) && small4(sb[1]);
-      if (OP == kKeygen) {
-        sec8w[64 * j + 2 * g] = sb[0];
-        sec8w[64 * j + 2 * g + 1] = sb[1];
-      }
-      const uint32_t e0 = raw_secrets4(sb[0]), e1 = raw_secrets4(sb[1]);
-      const uint32_t nx = __shfl_sync(0xffffffffu, e0, (lane + 1) & 31);
-      const uint32_t p0 = __byte_perm(e0, e1, 0x4321), p1 = __byte_perm(e1, nx, 0x4321);
-      // word 63: s_ext[255] = s[0] keeps its sign; word 127: s_ext[511] = 0
-      const uint32_t n1 = p1 ^ (g == 31 ? 0x00808080u : 0x80808080u);
-      const uint32_t q1 = g == 31 ? __byte_perm(e1, 0u, 0x4321) : p1;
-      // word 2g + 2, from the next lane (word 64 = s_ext[256] on for lane 31)
-      const uint32_t np = __shfl_sync(0xffffffffu, p0, (lane + 1) & 31);
-      const uint32_t ex = ext32 + (uint32_t)(LO::EXJ * j + 8 * g);
-      sts64(ex, p0 ^ 0x80808080u, n1);
-      sts64(ex + LO::EXC, n1, g == 31 ? np : np ^ 0x80808080u);
-      if (g < 16) {
-        sts64(ex + 256, p0, q1);
-        sts64(ex + LO::EXC + 256, q1, np);
-      }
-    }
-    // 2. digit columns (K reversed, core-matrix order): lane g converts
+    // 1. digit columns (K reversed, core-matrix order): lane g converts
     // coefficients 8g..8g+7 (K rows k' = 8kq+7..8kq, kq = 31 - g) of one
     // polynomial per item.  Warp p < R makes polynomial p of every j (one
     // item per j); with R == 1 (decryption) warp j makes j.  The columns past
@@ -652,7 +623,79 @@ __device__ __forceinline__ void cpa5i_run(const AT &at, uint8_t *sm) {
       }
     }
   }
-  // s_ext complete, and the streams inside H read, before H is written
+  // 2. secrets: a polynomial to a warp that makes no digit columns (the last L
+  // warps, of which the one of b does for L = 4); lane g takes the words 2g,
+  // 2g + 1 (coefficients 8g..8g+7).  Core matrices over the streams wait in a
+  // barrier until those are read (in both branches, so that only these warps
+  // hold their windows across it).
+  const int sj = S::R == 1 ? warp - L : kI5Threads / 32 - 1 - warp;
+  if (sj >= 0 && sj < L) {
+    uint32_t win[6] = {};
+    if (ready) {
+      const int j = sj, g = lane;
+      uint32_t sb[2];
+      if (IS_DEC && !C::SABLE) {
+        // 13-bit two's complement (SABER pack.cu:53-84)
+        constexpr uint32_t m = ((1u << C::EQ) - 1u) * 0x10001u;
+        uint32_t X[4];
+        unpack8c<C::EQ>(sm + LO::SKO, (32 * j + g) * C::EQ, X);
+        uint32_t bad = 0;
+#pragma unroll
+        for (int i = 0; i < 4; i++) bad |= ((X[i] + 0x00800080u) & m) & 0xFF00FF00u;
+        if (bad != 0u && a.err) atomicOr(a.err, 1);
+        sb[0] = __byte_perm(X[0], X[1], 0x6420);
+        sb[1] = __byte_perm(X[2], X[3], 0x6420);
+      } else {
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          const int w = 64 * j + 2 * g + h;
+          if (OP == kMatvec) {
+            sb[h] = lds32(smem_u32(sm + LO::SS) + 4 * w);  // four int8 coefficients
+          } else if (IS_DEC) {
+            // 2-bit two's complement (SABLE pack.cu:371-376): one byte = 4 coefficients
+            const uint32_t x = sm[LO::SKO + w];
+            const uint32_t spread = (x & 3u) | ((x & 0xcu) << 6) | ((x & 0x30u) << 12) | ((x & 0xc0u) << 18);
+            sb[h] = spread | (((spread >> 1) & 0x01010101u) * 0xfcu);
+          } else if (C::MU == 8) {
+            // CBD mu = 8 (SABER poly.cu:864-887)
+            const uint32_t x = lds32(smem_u32(sm + LO::SS) + 4 * w);
+            uint32_t n = x - ((x >> 1) & 0x55555555u);
+            n = (n & 0x33333333u) + ((n >> 2) & 0x33333333u);
+            sb[h] = __vsub4(n & 0x0f0f0f0fu, (n >> 4) & 0x0f0f0f0fu);
+          } else if (C::MU == 2) {
+            // CBD mu = 2 (SABLE fips202.cu:625-651)
+            const uint32_t x = sm[LO::SS + w];
+            const uint32_t spread = (x & 3u) | ((x & 0xcu) << 6) | ((x & 0x30u) << 12) | ((x & 0xc0u) << 18);
+            sb[h] = __vsub4(spread & 0x01010101u, (spread >> 1) & 0x01010101u);
+          } else {
+            // CBD mu = 6, 10: fields of mu bits, popcount halves
+            uint32_t r = 0;
+#pragma unroll
+            for (int b = 0; b < 4; b++) {
+              const uint32_t x = get_bits(sm + LO::SS, (4 * w + b) * C::MU, C::MU);
+              const int v = __popc(x & ((1u << (C::MU / 2)) - 1u)) - __popc(x >> (C::MU / 2));
+              r |= ((uint32_t)v & 0xffu) << (8 * b);
+            }
+            sb[h] = r;
+          }
+        }
+      }
+      // (CBD secrets are at most mu / 2 <= 5 in magnitude)
+      if (IS_DEC || OP == kMatvec) {
+        if (!(small4(sb[0]) && small4(sb[1])) && a.err) atomicOr(a.err, 1);
+      }
+      if (OP == kKeygen) {
+        sec8w[64 * j + 2 * g] = sb[0];
+        sec8w[64 * j + 2 * g + 1] = sb[1];
+      }
+      secret_windows(raw_secrets4(sb[0]), raw_secrets4(sb[1]), g, win);
+    }
+    if (LO::PLACE != kFree) ready = bar_and(ready);
+    if (ready) stage_hankel<LO>(smem_u32(H) + (uint32_t)(sj * LO::HJ), win, lane);
+  } else if (LO::PLACE != kFree) {
+    ready = bar_and(ready);
+  }
+  fence_async_smem();  // generic-proxy writes -> visible to the tensor core
   ready = __syncthreads_and(ready) != 0;
   if (!ready) {  // the input copies did not complete in time: report, leave
     if (tid == 0 && a.err) atomicOr(a.err, 2);
@@ -662,15 +705,6 @@ __device__ __forceinline__ void cpa5i_run(const AT &at, uint8_t *sm) {
     }
     break;
   }
-  stage_hankel6<LO, L>(smem_u32(H), ext32, tid);
-  fence_async_smem();  // generic-proxy writes -> visible to the tensor core
-  if constexpr (IS_DEC || OP == kMatvec) {
-    ok = __syncthreads_and(ok) != 0;
-    if (!ok && tid == 0 && a.err) atomicOr(a.err, 1);
-  } else {
-    __syncthreads();
-  }
-
   // 3. the MMAs (one thread).  Coefficients and K steps come in blocks of 32:
   // coefficient block o takes step t through the 32 x 32 Hankel block
   // B = o + t (rows 32B + r of s_ext[. + e]), where block B + 8 = -block B
@@ -692,25 +726,27 @@ __device__ __forceinline__ void cpa5i_run(const AT &at, uint8_t *sm) {
   if (tid == 0) {
     tc_fence_after();  // the previous instance's accumulator loads come before these MMAs
     constexpr uint32_t idesc = umma_idesc_e4m3(NU);
-    const uint64_t ad0 = umma_desc(smem_u32(H), 256, 128);
+    const uint64_t ad0 = umma_desc(smem_u32(H), 2 * LO::CS, LO::CS);
     const uint64_t bd0 = umma_desc(smem_u32(Bm), LO::LB, LO::SB);
 #pragma unroll
     for (int j = 0; j < L; j++) {
       const uint64_t hj = ad0 + (uint64_t)((j * LO::HJ) >> 4), bj = bd0 + (uint64_t)((j * LO::BJ) >> 4);
 #pragma unroll
       for (int w = 0; w < 8; w += 2)
-        umma_f8(tmem, hj + (uint64_t)((4 * w * 128) >> 4),
+        umma_f8(tmem, hj + (uint64_t)((4 * w * LO::CS) >> 4),
                 bj + (uint64_t)((((w >> 1) & 1) * LO::QB + (w < 4 ? S::PG * LO::SB : 0)) >> 4), idesc, (j | w) != 0);
     }
     umma_commit(mbar_mma);
   }
   // 4. accumulators: one warp polls the MMA barrier and the CLC answer, the
-  // others wait in the CTA barrier.  The MMAs have read H and the other
-  // ciphertext buffer was last read before this instance's barriers, so the
-  // next instance's copies start here, beside the epilogue.
+  // others wait in the CTA barrier.  The next instance's copies start as soon
+  // as what they overwrite is read: beside the MMAs, or beside the epilogue
+  // where they land in H (the other ciphertext buffer was last read before this
+  // instance's barriers).
   bool done = true;
   if (warp == 0) {
-    done = mbar_wait_bounded(mbar_mma, par) && mbar_wait_bounded(mbar_clc, par);
+    if (LO::PLACE != kFree) done = mbar_wait_bounded(mbar_mma, par);
+    done = mbar_wait_bounded(mbar_clc, par) && done;
     done = __all_sync(0xffffffffu, done) != 0;
     if (tid == 0) {
       const uint32_t nx = done ? clc_answer(clc_resp + 16 * par) : ~0u;
@@ -721,6 +757,7 @@ __device__ __forceinline__ void cpa5i_run(const AT &at, uint8_t *sm) {
       }
       if (OP == kReenc && done) a.fail[inst] = 0;  // set below, after the barrier, by a warp that finds a difference
     }
+    if (LO::PLACE == kFree) done = mbar_wait_bounded(mbar_mma, par) && done;
   }
   done = __syncthreads_and(done) != 0;
   if (!done) {
@@ -730,6 +767,7 @@ __device__ __forceinline__ void cpa5i_run(const AT &at, uint8_t *sm) {
     if (warp == 0) {
       mbar_wait_bounded(mbar_mma, par);
       mbar_wait_bounded(mbar_clc, par);
+      if (*next_slot != ~0u) mbar_wait_bounded(mbar_in, par ^ 1u);
     }
     break;
   }
@@ -771,8 +809,7 @@ __device__ __forceinline__ void cpa5i_run(const AT &at, uint8_t *sm) {
     // odd steps first: block o' = q4 - 1 (hsel 0; block 7 negated for
     // q4 = 0) or q4 + 3, for the warp of that block; two 16-bit values a word
     uint32_t f[2 * S::NC4];
-    uint32_t odd[2 * LO::XWORDS];
-    odd[2 * LO::XWORDS - 1] = 0;
+    uint32_t odd[S::R];
     tmem_ld_cols(t0 + (uint32_t)(2 * S::NC4 * hsel), f);
     const int od = (warp + 7) & 7;  // the block the odd steps belong to
 #pragma unroll
@@ -784,6 +821,7 @@ __device__ __forceinline__ void cpa5i_run(const AT &at, uint8_t *sm) {
 #pragma unroll
     for (int i = 0; i < LO::XWORDS; i++)
       sts32(xch + (uint32_t)((i * 256 + 32 * od + lane) * 4), __byte_perm(odd[2 * i], odd[2 * i + 1], 0x5410));
+    if (S::R & 1) *reinterpret_cast<uint16_t *>(sm + LO::XCH + 1024 * LO::XWORDS + 2 * (32 * od + lane)) = (uint16_t)odd[S::R - 1];
 #pragma unroll
     for (int p = 0; p < S::R; p++) val[p] = combine5<OP, SET>(f, p, 0, ROUND);
     tc_fence_before();  // the loads above come before the next instance's MMAs (its barriers lie between)
@@ -792,8 +830,9 @@ __device__ __forceinline__ void cpa5i_run(const AT &at, uint8_t *sm) {
     for (int i = 0; i < LO::XWORDS; i++) {
       const uint32_t x = lds32(xch + (uint32_t)((i * 256 + tid) * 4));
       val[2 * i] += x;
-      if (2 * i + 1 < S::R) val[2 * i + 1] += x >> 16;
+      val[2 * i + 1] += x >> 16;
     }
+    if (S::R & 1) val[S::R - 1] += *reinterpret_cast<const uint16_t *>(sm + LO::XCH + 1024 * LO::XWORDS + 2 * tid);
   }
   if constexpr (OP == kEncrypt || OP == kKeygen) {
     // coefficient k of every output polynomial, rounded (b, b') or encoded
@@ -904,17 +943,14 @@ __device__ __forceinline__ void cpa5i_run(const AT &at, uint8_t *sm) {
   if (threadIdx.x < 32) tmem_dealloc(tmem, S::TMEM_COLS);
 }
 
-// CTAs per SM that shared memory (228 KB, 1 KB of it per CTA reserved) and
-// tensor memory (512 columns) allow, and at most what the registers allow
-// without spilling more than a few words: 8 of 32 registers (decryption, 212
-// against 216 us with 6 at 65536), 6 of 40, and 5 of 48 where a thread loads
-// 32 accumulator columns.  The speed comes from the CTAs that overlap each
-// other's phases.
+// CTAs per SM that shared memory (228 KB, 1 KB of it per CTA reserved), tensor
+// memory (512 columns) and registers allow.  The speed comes from the CTAs that
+// overlap each other's phases.
 template <int OP, int SET>
 constexpr int min_ctas() {
-  constexpr int by_smem = (228 * 1024) / (LayoutC<OP, SET>::TOTAL + 1024), by_tmem = 512 / ShapeC<OP, SET>::TMEM_COLS;
+  constexpr int by_smem = LayoutC<OP, SET>::CTAS, by_tmem = 512 / ShapeC<OP, SET>::TMEM_COLS;
   constexpr int m = by_smem < by_tmem ? by_smem : by_tmem;
-  constexpr int cap = ShapeC<OP, SET>::NC4 == 16 ? 5 : (OP == kDecrypt ? 8 : 6);
+  constexpr int cap = reg_ctas<OP, SET>();
   return m < cap ? m : cap;
 }
 
