@@ -22,6 +22,7 @@
 #include <cstdint>
 #include <type_traits>
 
+#include "chain.cuh"
 #include "cpa_persist.cuh"
 
 namespace tmvp {
@@ -486,6 +487,12 @@ __device__ __forceinline__ uint32_t combine5(const uint32_t (&f)[2 * ShapeC<OP, 
   return __float_as_uint(x) + 256u * __float_as_uint(col(2) + 48.0f);
 }
 
+// The decryptions are launched ordinarily (chain.cuh): they start a pass beside
+// the Keccak front on another stream, so nothing is gained there, and the two
+// instructions of the wait alone cost the decryption of 65536 Saber ciphertexts
+// 10 us (registers: it has 32).
+constexpr bool is_decryption(int op) { return op == kDecrypt || op == kDecryptK; }
+
 // The instances of a launch, from the CTA of kI5Threads threads that runs
 // blockIdx.x (sm: its dynamic shared memory).  at(gi) names the arguments and
 // the instance of CTA gi: a pair-like struct {const CpaArgs &a; unsigned inst}.
@@ -521,9 +528,11 @@ __device__ __forceinline__ void cpa5i_run(const AT &at, uint8_t *sm) {
     mbar_init(mbar_mma, 1);
     mbar_init(mbar_clc, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    if (!is_decryption(OP)) chain_wait();
     const auto w = at(blockIdx.x);
     cpa5i_load<OP, SET>(w.a, w.inst, smem_u32(sm), 0, mbar_in);
   }
+  if (!is_decryption(OP)) chain_wait();  // (all threads)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -1033,8 +1042,7 @@ inline int launch_cpa5ms(const CpaArgs *groups, int ng, cudaStream_t s) {
   if (e != cudaSuccess) return (int)e;
   int rc = cap_tmem_residency(fn, smem, S::TMEM_COLS);
   if (rc) return rc;
-  fn<<<T.total, kI5Threads, smem, s>>>(T);
-  return (int)cudaGetLastError();
+  return (int)launch_chained<!is_decryption(OP)>(fn, T.total, kI5Threads, smem, s, T);
 }
 
 // Groups of one parameter set (a mixed pass launches each set's groups by themselves).
@@ -1072,8 +1080,8 @@ inline int launch_cpa5i(const CpaArgs &a, cudaStream_t s) {
     if (nb <= cap) break;
     smem += 2048;
   }
-  fn<<<OP == kDecryptK ? (a.n + S::R - 1) / S::R : a.n, kI5Threads, smem, s>>>(a);
-  return (int)cudaGetLastError();
+  return (int)launch_chained<!is_decryption(OP)>(fn, OP == kDecryptK ? (a.n + S::R - 1) / S::R : a.n, kI5Threads,
+                                                 smem, s, a);
 }
 
 // Dispatch over the six parameter sets (matvec is not set-shaped).

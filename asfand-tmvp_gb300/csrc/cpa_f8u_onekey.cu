@@ -8,8 +8,7 @@ namespace {
 
 template <int SET>
 int prep(const uint8_t *a_stream, const uint8_t *b_stream, uint8_t *ops, cudaStream_t s) {
-  k_onekey_prep<SET><<<OneKeyC<SET>::PLANES, 256, 0, s>>>(a_stream, b_stream, ops);
-  return (int)cudaGetLastError();
+  return (int)launch_chained(k_onekey_prep<SET>, OneKeyC<SET>::PLANES, 256, 0, s, a_stream, b_stream, ops);
 }
 
 template <int SET>
@@ -19,8 +18,7 @@ int reenc(OneKeyArgs a, int sms, cudaStream_t s) {
   auto fn = k_onekey_reenc<SET>;
   const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, K::TOTAL);
   if (e != cudaSuccess) return (int)e;
-  fn<<<a.units < sms ? a.units : sms, kOkThreads, K::TOTAL, s>>>(a);
-  return (int)cudaGetLastError();
+  return (int)launch_chained(fn, a.units < sms ? a.units : sms, kOkThreads, K::TOTAL, s, a);
 }
 
 }  // namespace

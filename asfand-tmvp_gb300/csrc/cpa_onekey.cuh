@@ -91,6 +91,7 @@ __global__ void __launch_bounds__(256) k_onekey_prep(const uint8_t *a_stream, co
     d = b % K::PB;
   }
   const int k = threadIdx.x, W = p < L ? C::EQ : C::EP;
+  chain_wait();
   const uint8_t *src = p < L ? a_stream + 32 * (p * L + j) * C::EQ : b_stream + 32 * j * C::EP;
   // the W-bit coefficient k (byte reads inside the polynomial only)
   uint32_t x = 0;
@@ -182,6 +183,7 @@ __global__ void __launch_bounds__(kOkThreads, 1) k_onekey_reenc(const __grid_con
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *reinterpret_cast<volatile uint32_t *>(slot);
+  chain_wait();
   // units [u0, u1) of (block, output polynomial); `it` counts this CTA's blocks
   const int u0 = (int)((long long)a.units * blockIdx.x / gridDim.x),
             u1 = (int)((long long)a.units * (blockIdx.x + 1) / gridDim.x);

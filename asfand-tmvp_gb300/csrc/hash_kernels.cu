@@ -10,6 +10,7 @@
 
 #include <algorithm>
 
+#include "chain.cuh"
 #include "hash_engine.cuh"
 
 namespace tmvp {
@@ -187,6 +188,7 @@ struct MixFinal : MixBase {
 template <class R>
 __global__ void __launch_bounds__(kHashBlock) k_sponges(const __grid_constant__ SpongePlan S,
                                                         const __grid_constant__ R r) {
+  chain_wait();
   int k = 0;
   while (k + 1 < S.nseg && blockIdx.x >= S.seg[k + 1].block0) k++;
   const unsigned b = blockIdx.x - S.seg[k].block0, count = S.seg[k].count, first = S.seg[k].first;
@@ -224,8 +226,7 @@ cudaError_t launch_sponges(const SpongePlan &S, const R &r, cudaStream_t s) {
     const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S.smem);
     if (e != cudaSuccess) return e;
   }
-  fn<<<S.blocks, S.threads, S.smem, s>>>(S, r);
-  return cudaGetLastError();
+  return launch_chained(fn, S.blocks, S.threads, S.smem, s, S, r);
 }
 
 template <class R>
