@@ -282,6 +282,14 @@ bool sponges_split(const HashCfg &cfg, size_t n) {
 //    an SM that finishes early takes the next block instead of all being
 //    placed at the start: with one block per SM 16384 x (23 + 9) takes 135
 //    us; with two per SM 32768 345 -> 266 and 65536 530 -> 502 (one: 272, 517).
+//  * One role over several rounds: as many blocks resident per SM as rounds, so
+//    that none gets one more while a neighbour has one less (a grid's first
+//    152 blocks land on 148 SMs); the rest in a finer form then starts behind
+//    them.  65536 x 10 permutations 185 -> 166 us, x 8 154 -> 136, x 6 113 ->
+//    107, and a pass of two chains leaves room for the other one's kernels
+//    (decapsulation of 65536 Saber 1037 -> 1015, of 38912 659 -> 634).  Not
+//    with one round and a finer rest (20011 x 10: 70 -> 78) and not for a
+//    single permutation (25 -> 27).
 //  * Just above one round (up to 1.5) the longer role's thread-form blocks run
 //    alone at one per SM and the rest as a second launch beside them: as one
 //    launch, four SMs get two of those blocks (key generation of 20011: 386 us,
@@ -314,6 +322,11 @@ void plan_sponges(const HashCfg &cfg, const SpongeRole *roles, int nroles, Spong
     if (form == kHashWarp) warps += rest;
     add_seg(S[split && k == 1], r.id, kHashThread, 0, full);
     add_seg(S[split && (k == 1 || form != kHashThread)], r.id, form, full, rest);
+    if (nroles == 1 && r.perms >= 4) {
+      // blocks per SM when every SM has its share
+      const int q = (int)(full / (32 * W)) + (form == kHashThread && rest ? 1 : 0);
+      if (q <= 5 && (form == kHashThread || rest == 0 || q >= 2)) S[0].smem = smem_limit(q);
+    }
     if (nroles == 2 && k == 0 && (full || form == kHashThread)) S[0].smem = smem_limit(cfg.cap > 0 ? cfg.cap : (full && !split ? 2 : 1));
   }
 }
