@@ -184,29 +184,8 @@ template <int OP, int SET>
 using LayoutC = LayoutAt<OP, SET, input_place<OP, SET>()>;
 
 // Eight W-bit little-endian fields from byte `byte0` (16 bytes of slack after
-// the stream), as four words of two 16-bit lanes.
-template <int W>
-__device__ __forceinline__ void unpack8c(const uint8_t *base, int byte0, uint32_t (&X)[4]) {
-  const uint32_t wp = smem_u32(base) + (uint32_t)(byte0 & ~3);
-  const int sh = 8 * (byte0 & 3);
-  uint32_t q[5];
-#pragma unroll
-  for (int i = 0; i < 5; i++) q[i] = lds32(wp + 4 * i);
-  uint32_t a[4];
-#pragma unroll
-  for (int i = 0; i < 4; i++) a[i] = __funnelshift_r(q[i], q[i + 1], sh);
-  constexpr uint32_t m = (1u << W) - 1u;
-#pragma unroll
-  for (int k = 0; k < 8; k += 2) {
-    const int b0 = k * W, b1 = (k + 1) * W;
-    const uint32_t v0 = __funnelshift_r(a[b0 >> 5], a[(b0 >> 5) + 1 < 4 ? (b0 >> 5) + 1 : 3], b0 & 31) & m;
-    const uint32_t v1 = __funnelshift_r(a[b1 >> 5], a[(b1 >> 5) + 1 < 4 ? (b1 >> 5) + 1 : 3], b1 & 31) & m;
-    X[k >> 1] = __byte_perm(v0, v1, 0x5410);
-  }
-}
-
-// The same fields two at a time, without clearing the bits above them in
-// each 16-bit lane (raw_digits8 masks its digits).
+// the stream), as four words of two 16-bit lanes, two at a time and without
+// clearing the bits above them in each lane (whoever uses them masks).
 template <int W>
 __device__ __forceinline__ uint32_t field_pair(const uint32_t *w, int nw, int bit) {
   const int i = bit >> 5, sh = bit & 31;
@@ -583,20 +562,14 @@ __device__ __forceinline__ void cpa5i_run(const AT &at, uint8_t *sm) {
     if constexpr (OP == kMatvec) {
       // coefficients already in 16-bit lanes: digit d of the low 13 bits
       // (the result is needed mod 2^eq, eq <= 13)
-      if (warp < L) {
-        const int p = warp;
+      // over the warps that have no secrets
+      for (int t = warp; t < L * L && warp < NT / 32 - L; t += NT / 32 - L) {
+        const int p = t / L, j = t % L;
+        const int ij = a.mv_transpose ? (j * L + p) : (p * L + j);
+        uint32_t X[4];
+        lds128(smem_u32(sm + LO::A) + (uint32_t)(512 * ij + 16 * lane), X[0], X[1], X[2], X[3]);
 #pragma unroll
-        for (int j = 0; j < L; j++) {
-          const int ij = a.mv_transpose ? (j * L + p) : (p * L + j);
-          const uint32_t src = smem_u32(sm + LO::A) + (uint32_t)(512 * ij + 16 * lane);
-          uint32_t X[4];
-#pragma unroll
-          for (int i = 0; i < 4; i++) X[i] = lds32(src + 4 * i);
-#pragma unroll
-          for (int d = 0; d < S::DA; d++) {
-            put(j, p * S::DA + d, raw_digits8<S::WA>(X, d));
-          }
-        }
+        for (int d = 0; d < S::DA; d++) put(j, p * S::DA + d, raw_digits8<S::WA>(X, d));
       }
     } else if constexpr (DECK) {
       // warp r makes ciphertext r's b'_j for every j
@@ -610,18 +583,21 @@ __device__ __forceinline__ void cpa5i_run(const AT &at, uint8_t *sm) {
       if (warp < L) item(std::integral_constant<int, S::WB>{}, (int)cbuf + LO::CTO + 32 * warp * S::WB, 0, warp);
     } else {
       // public matrix A (RA x L polynomials), then b (encryption, re-encryption):
-      // four polynomials per warp, eight lanes each
-      constexpr int NA = S::RA * L, NB = (S::R - S::RA) * L;
+      // four polynomials per warp, eight lanes each; one that is left over (the
+      // ninth for L = 3) by a whole warp, in a third of the instructions
+      constexpr int NA = S::RA * L, NB = (S::R - S::RA) * L, NA8 = NA % 4 == 1 ? NA - 1 : NA;
       constexpr int WA_WARPS = (NA + 3) / 4, WB_WARPS = (NB + 3) / 4;
       static_assert(WA_WARPS + WB_WARPS <= 8, "digit polynomials fit the CTA's warps");
       const uint32_t bm32 = smem_u32(Bm);
-      if (warp < WA_WARPS) {
+      if (4 * warp < NA8) {
         const int t = 4 * warp + (lane >> 3);
-        if (t < NA) {
+        if (t < NA8) {
           const int p = t / L, j = t % L;
           const int ij = (OP == kKeygen) ? (j * L + p) : (p * L + j);
           stage_digits32<S::WA, LO>(sm, LO::A + 32 * ij * S::WA, bm32 + (uint32_t)(j * LO::BJ), p * S::DA, lane & 7);
         }
+      } else if (warp < WA_WARPS) {
+        item(std::integral_constant<int, S::WA>{}, LO::A + 32 * (L * L - 1) * S::WA, (S::RA - 1) * S::DA, L - 1);
       } else if (warp < WA_WARPS + WB_WARPS) {
         const int t = 4 * (warp - WA_WARPS) + (lane >> 3);
         if (t < NB) {
@@ -642,16 +618,14 @@ __device__ __forceinline__ void cpa5i_run(const AT &at, uint8_t *sm) {
     uint32_t win[6] = {};
     if (ready) {
       const int j = sj, g = lane;
-      uint32_t sb[2];
+      uint32_t sb[2], bad = 0;
       if (IS_DEC && !C::SABLE) {
-        // 13-bit two's complement (SABER pack.cu:53-84)
-        constexpr uint32_t m = ((1u << C::EQ) - 1u) * 0x10001u;
+        // 13-bit two's complement (SABER pack.cu:53-84); -8 .. 7 where bits 3 .. 12 agree
         uint32_t X[4];
-        unpack8c<C::EQ>(sm + LO::SKO, (32 * j + g) * C::EQ, X);
-        uint32_t bad = 0;
+        unpack8d<C::EQ>(sm + LO::SKO, (32 * j + g) * C::EQ, X);
 #pragma unroll
-        for (int i = 0; i < 4; i++) bad |= ((X[i] + 0x00800080u) & m) & 0xFF00FF00u;
-        if (bad != 0u && a.err) atomicOr(a.err, 1);
+        for (int i = 0; i < 4; i++) bad |= X[i] ^ (X[i] >> 1);
+        bad &= 0x0FF80FF8u;
         sb[0] = __byte_perm(X[0], X[1], 0x6420);
         sb[1] = __byte_perm(X[2], X[3], 0x6420);
       } else {
@@ -660,6 +634,7 @@ __device__ __forceinline__ void cpa5i_run(const AT &at, uint8_t *sm) {
           const int w = 64 * j + 2 * g + h;
           if (OP == kMatvec) {
             sb[h] = lds32(smem_u32(sm + LO::SS) + 4 * w);  // four int8 coefficients
+            bad |= (sb[h] ^ (sb[h] >> 1)) & 0x78787878u;
           } else if (IS_DEC) {
             // 2-bit two's complement (SABLE pack.cu:371-376): one byte = 4 coefficients
             const uint32_t x = sm[LO::SKO + w];
@@ -689,15 +664,16 @@ __device__ __forceinline__ void cpa5i_run(const AT &at, uint8_t *sm) {
           }
         }
       }
-      // (CBD secrets are at most mu / 2 <= 5 in magnitude)
-      if (IS_DEC || OP == kMatvec) {
-        if (!(small4(sb[0]) && small4(sb[1])) && a.err) atomicOr(a.err, 1);
-      }
       if (OP == kKeygen) {
         sec8w[64 * j + 2 * g] = sb[0];
         sec8w[64 * j + 2 * g + 1] = sb[1];
       }
-      secret_windows(raw_secrets4(sb[0]), raw_secrets4(sb[1]), g, win);
+      const uint32_t e0 = raw_secrets4(sb[0]), e1 = raw_secrets4(sb[1]);
+      // a magnitude of 8 is too large too (CBD secrets are at most mu / 2 <= 5, the 2-bit ones 2)
+      if ((IS_DEC && !C::SABLE) || OP == kMatvec) {
+        if ((bad | ((e0 | e1) & 0x08080808u)) != 0u && a.err) atomicOr(a.err, 1);
+      }
+      secret_windows(e0, e1, g, win);
     }
     if (LO::PLACE != kFree) ready = bar_and(ready);
     if (ready) stage_hankel<LO>(smem_u32(H) + (uint32_t)(sj * LO::HJ), win, lane);
@@ -870,7 +846,7 @@ __device__ __forceinline__ void cpa5i_run(const AT &at, uint8_t *sm) {
     const uint32_t t = (v - (cf[0] << (C::EP - C::ET))) & pmask;
     const uint32_t bits = __ballot_sync(0xffffffffu, ((t >> (C::EP - 1)) & 1u) != 0u);
     uint8_t *mo = a.m_out + (size_t)inst * a.m_out_stride;
-    if (lane < 4) mo[4 * (4 * hsel + q4) + lane] = (uint8_t)(bits >> (8 * lane));
+    if (lane == 0) reinterpret_cast<uint32_t *>(mo)[4 * hsel + q4] = bits;  // (rows of 32 or 64 bytes)
     if (a.copy_hpk && warp == 0) mo[32 + lane] = a.sk[(a.key_shared ? 0 : (size_t)inst * C::SK) + C::SK - 64 + lane];
   } else if constexpr (DECK) {
     // ciphertext r of the CTA: decode as above from its own columns and c_m
@@ -881,7 +857,7 @@ __device__ __forceinline__ void cpa5i_run(const AT &at, uint8_t *sm) {
       const uint32_t t = (v - (cf[r] << (C::EP - C::ET))) & pmask;
       const uint32_t bits = __ballot_sync(0xffffffffu, ((t >> (C::EP - 1)) & 1u) != 0u);
       uint8_t *mo = a.m_out + (inst0 + r) * a.m_out_stride;
-      if (lane < 4) mo[4 * (4 * hsel + q4) + lane] = (uint8_t)(bits >> (8 * lane));
+      if (lane == 0) reinterpret_cast<uint32_t *>(mo)[4 * hsel + q4] = bits;
       if (a.copy_hpk && warp == 0) mo[32 + lane] = a.sk[C::SK - 64 + lane];
     }
   } else if constexpr (OP == kReenc) {
