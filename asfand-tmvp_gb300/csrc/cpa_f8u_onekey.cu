@@ -21,6 +21,21 @@ int reenc(OneKeyArgs a, int sms, cudaStream_t s) {
   return (int)launch_chained(fn, a.units < sms ? a.units : sms, kOkThreads, K::TOTAL, s, a);
 }
 
+template <int SET>
+int decrypt(OneKeyDecArgs a, uint8_t *planes, int sms, cudaStream_t s) {
+  using K = OneKeyD<SET>;
+  cudaError_t e = launch_chained(k_onekey_sprep<SET>, K::PLANES, 256, 0, s, a.sk, planes, a.err);
+  if (e != cudaSuccess) return (int)e;
+  const int rounds = (a.n + kOkRows * sms - 1) / (kOkRows * sms);
+  a.rows = (a.n + sms * rounds - 1) / (sms * rounds);
+  a.blocks = (a.n + a.rows - 1) / a.rows;
+  a.planes = planes;
+  auto fn = k_onekey_decrypt<SET>;
+  if ((e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, K::TOTAL)) != cudaSuccess)
+    return (int)e;
+  return (int)launch_chained(fn, a.blocks < sms ? a.blocks : sms, kOkDecThreads, K::TOTAL, s, a);
+}
+
 }  // namespace
 
 #define TMVP_OK_SETS(X) \
@@ -57,6 +72,21 @@ int onekey_reenc(const CpaArgs &b, const uint8_t *ops, int sms, void *s) {
   a.n = b.n;
 #define TMVP_OK_REENC(S) reenc<S>(a, sms, (cudaStream_t)s)
   TMVP_OK_SETS(TMVP_OK_REENC)
+  return (int)cudaErrorInvalidValue;
+}
+
+size_t onekey_secret_bytes(const KemParams &P) { return (size_t)(2 * P.l * kOkHankel); }
+
+int onekey_decrypt(const CpaArgs &b, uint8_t *planes, int sms, void *s) {
+  const KemParams &P = b.P;
+  OneKeyDecArgs a{};
+  a.ct = b.ct;
+  a.sk = b.sk;
+  a.m_out = b.m_out;
+  a.err = b.err;
+  a.n = b.n;
+#define TMVP_OK_DEC(S) decrypt<S>(a, planes, sms, (cudaStream_t)s)
+  TMVP_OK_SETS(TMVP_OK_DEC)
   return (int)cudaErrorInvalidValue;
 }
 

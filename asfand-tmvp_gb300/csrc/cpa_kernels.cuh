@@ -72,6 +72,11 @@ int cpa_launch_decrypt_onekey(const CpaArgs &a, void *stream);
 size_t onekey_operand_bytes(const KemParams &P);
 int onekey_prep(const KemParams &P, const uint8_t *a_stream, const uint8_t *b_stream, uint8_t *ops, void *stream);
 int onekey_reenc(const CpaArgs &b, const uint8_t *ops, int sms, void *stream);
+// Decryption of b.n ciphertexts under the key at b.sk the same way, into rows of
+// 64 bytes at b.m_out (m' | H(pk)).  planes: onekey_secret_bytes of device memory,
+// filled here.
+size_t onekey_secret_bytes(const KemParams &P);
+int onekey_decrypt(const CpaArgs &b, uint8_t *planes, int sms, void *stream);
 
 // tcgen05 form only: one persistent launch over `ngroups` (<= kMixMaxGroups)
 // groups of instances, each with its own parameter set and buffers.  groups:

@@ -348,4 +348,236 @@ __global__ void __launch_bounds__(kOkThreads, 1) k_onekey_reenc(const __grid_con
   if (warp == kOkWorkers) tmem_dealloc(tmem, 512);
 }
 
+// ---------------------------------------------------------------------------
+// Decryption of many ciphertexts under one key, the same way: the key's secrets
+// are the Hankel side, resident in shared memory, and a row is one ciphertext's
+// b' in two balanced base-32 digit planes.  Digit 1 meets a copy of the secrets
+// scaled by 32, so that both planes add up in one accumulator: x * 2^-18 with
+// |x| <= 16 * 33 * 7 * 256 l < 2^24.
+//
+// What bounds it: the digits (about 6 instructions a coefficient and plane
+// pair) of 16 warps, which fill two buffers of one j each ahead of the MMAs
+// (48 of N = 256 for 128 Saber ciphertexts) and decode a block's accumulators
+// while the next block's first digits are multiplied.  The n ciphertexts are
+// spread evenly over whole rounds of one block per SM.  65536 Saber ciphertexts:
+// 47 us (five to a CTA of the per-instance kernel, which shares the staged secret
+// and the MMAs: 82).
+
+template <int SET>
+struct OneKeyD {
+  using C = SetC<SET>;
+  static constexpr int L = C::L, PLANES = 2 * L;
+  static constexpr int BR = 16 * kOkRows, PL = 16 * BR, BJ = 2 * PL;  // digit bytes: a 16-byte K chunk, a plane, a j
+  static constexpr int A = 0, B = 2 * BJ, BAR = B + PLANES * kOkHankel, TOTAL = BAR + 128;
+  static_assert(TOTAL <= 227 * 1024, "fits an SM");
+  static_assert(16 * 33 * 7 * 256 * L < (1 << 24), "exact in the f32 accumulators");
+};
+constexpr int kOkDecThreads = 32 * (kOkWorkers + 1);
+
+// Block (j, digit): the core matrices of the secret polynomial j times 32^digit.
+template <int SET>
+__global__ void __launch_bounds__(256) k_onekey_sprep(const uint8_t *sk, uint8_t *planes, int *err) {
+  using C = SetC<SET>;
+  __shared__ uint8_t ext[512];
+  const int k = threadIdx.x, j = blockIdx.x >> 1, d = blockIdx.x & 1;
+  constexpr int W = C::SABLE ? 2 : C::EQ;
+  chain_wait();
+  const uint8_t *src = sk + 32 * j * W;
+  uint32_t x = 0;
+  for (int q = (k * W) >> 3; q <= (k * W + W - 1) >> 3; q++) x |= (uint32_t)src[q] << (8 * (q - ((k * W) >> 3)));
+  int v = (int)((x >> ((k * W) & 7)) & ((1u << W) - 1u));
+  if (v >= 1 << (W - 1)) v -= 1 << W;
+  if (v < -7 || v > 7) {  // (as the per-instance kernel: reported, the result is not used)
+    if (err) atomicOr(err, 1);
+    v = 0;
+  }
+  const uint32_t e = e4m3_scaled(v, d);
+  ext[255 + k] = (uint8_t)e;
+  if (k > 0) ext[k - 1] = (uint8_t)(e ^ 0x80u);
+  __syncthreads();
+  uint8_t *out = planes + (size_t)blockIdx.x * kOkHankel;
+  for (int i = k; i < kOkHankel / 4; i += 256) {
+    const int byte = 4 * i, at = 8 * (byte >> 7) + ((byte >> 4) & 7) + (byte & 15);
+    reinterpret_cast<uint32_t *>(out)[i] =
+        (uint32_t)ext[at] | (uint32_t)ext[at + 1] << 8 | (uint32_t)ext[at + 2] << 16 | (uint32_t)ext[at + 3] << 24;
+  }
+}
+
+struct OneKeyDecArgs {
+  const uint8_t *planes;  // k_onekey_sprep
+  const uint8_t *ct;      // [n][ct_bytes]
+  const uint8_t *sk;      // the key: H(pk) is copied from it
+  uint8_t *m_out;         // [n][64]: m' | H(pk)
+  int *err;
+  int n, rows, blocks;    // ciphertexts; of a block (<= kOkRows); blocks
+};
+
+template <int SET>
+__global__ void __launch_bounds__(kOkDecThreads, 1) k_onekey_decrypt(const __grid_constant__ OneKeyDecArgs a) {
+  using C = SetC<SET>;
+  using K = OneKeyD<SET>;
+  constexpr int L = C::L, BR = K::BR, W = C::EP;
+  extern __shared__ __align__(128) uint8_t sm[];
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // (uniform)
+  const uint32_t s0 = smem_u32(sm), bar = s0 + K::BAR;
+  // barriers: digits full / empty, accumulators full / empty (two of each), planes
+  const uint32_t a_full = bar, a_empty = bar + 16, d_full = bar + 32, d_empty = bar + 48, b_full = bar + 64;
+  uint32_t *slot = reinterpret_cast<uint32_t *>(sm + K::BAR + 72);
+  if (warp == kOkWorkers) tmem_alloc(smem_u32(slot), 512);
+  if (tid == 0) {
+    for (int i = 0; i < 2; i++) {
+      mbar_init(a_full + 8 * i, 32 * kOkWorkers);
+      mbar_init(a_empty + 8 * i, 1);
+      mbar_init(d_full + 8 * i, 1);
+      mbar_init(d_empty + 8 * i, 32 * kOkWorkers);
+    }
+    mbar_init(b_full, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *reinterpret_cast<volatile uint32_t *>(slot);
+  chain_wait();
+  bool ok = true;
+  if (warp == kOkWorkers) {
+    // the planes, once, then the MMAs (the whole warp runs the loop, one lane issues)
+    const bool one = lane == 0;
+    if (one) {
+      mbar_expect_tx(b_full, K::PLANES * kOkHankel);
+      for (int q = 0; q < K::PLANES; q++)
+        bulk_g2s(s0 + K::B + q * kOkHankel, a.planes + (size_t)q * kOkHankel, kOkHankel, b_full);
+    }
+    __syncwarp();
+    ok = mbar_wait_bounded(b_full, 0);
+    if (!ok) mbar_wait_bounded(b_full, 0);  // (no copy outlives the CTA)
+    constexpr uint32_t idesc = umma_idesc_e4m3(256);
+    uint32_t item = 0, dn = 0;  // digit buffers and accumulators used so far
+    for (int blk = blockIdx.x; ok && blk < a.blocks; blk += gridDim.x, dn++) {
+      const uint32_t d = tmem + 256 * (dn & 1);
+      if (dn >= 2) ok = mbar_spin_bounded(d_empty + 8 * (dn & 1), ((dn >> 1) - 1) & 1);
+      for (int j = 0; ok && j < L; j++, item++) {
+        const uint32_t ab = item & 1;
+        ok = mbar_spin_bounded(a_full + 8 * ab, (item >> 1) & 1);
+        if (!ok) break;
+        tc_fence_after();
+#pragma unroll
+        for (int p = 0; p < 2; p++) {
+          const uint64_t ad = umma_desc(s0 + K::A + ab * K::BJ + p * K::PL, BR, 128);
+          const uint64_t bd = umma_desc(s0 + K::B + (2 * j + p) * kOkHankel, 256, 128);
+#pragma unroll
+          for (int t = 0; t < 8; t++)
+            umma_f8_if(one, d, ad + (uint64_t)((2 * t * BR) >> 4), bd + (uint64_t)((4 * t * 128) >> 4), idesc,
+                       (j | p | t) != 0);
+        }
+        if (one) umma_commit(a_empty + 8 * ab);
+      }
+      if (ok && one) umma_commit(d_full + 8 * (dn & 1));
+    }
+    if (!ok && one && a.err) atomicOr(a.err, 2);
+    // the last MMAs have completed when the workers have read their accumulators
+  } else {
+    uint32_t item = 0;
+    // Digits of b'_j of a block's ciphertexts into the next buffer: 8 ciphertexts
+    // x 4 chunks of 16 coefficients a warp task
+    auto stage = [&](int blk, int j) {
+      const uint32_t ab = item & 1;
+      ok = item < 2 || mbar_wait_bounded(a_empty + 8 * ab, ((item >> 1) - 1) & 1);
+      item++;
+      if (!ok) return;
+      const int base = blk * a.rows, nv = min(a.rows, a.n - base);
+      const uint32_t dst = s0 + K::A + ab * K::BJ;
+#pragma unroll 4
+      for (int u = warp; u < (kOkRows / 8) * 4; u += kOkWorkers) {
+        const int c = 8 * (u >> 2) + (lane & 7), g = 4 * (u & 3) + (lane >> 3);
+        if (c < nv) {
+          const int off = 2 * W * g;
+          const uint8_t *src = a.ct + (size_t)(base + c) * C::CT + j * C::POLYCOMP + (off & ~3);
+          uint32_t w[5];
+#pragma unroll
+          for (int i = 0; i < 5; i++) w[i] = __ldg(reinterpret_cast<const uint32_t *>(src) + i);
+          if (W & 1) {  // 18 bytes a chunk
+#pragma unroll
+            for (int i = 0; i < 5; i++) w[i] = __funnelshift_r(w[i], i < 4 ? w[i + 1] : 0u, 8 * (off & 2));
+          }
+          uint32_t lo[4], hi[4];
+#pragma unroll
+          for (int h = 0; h < 4; h++) {  // coefficients 4h .. 4h + 3, the last first
+            constexpr uint32_t m = ((1u << W) - 1u) * 0x10001u;
+            const uint32_t x0 = field_pair<W>(w, 5, 4 * W * h) & m, x1 = field_pair<W>(w, 5, 4 * W * h + 2 * W) & m;
+            lo[3 - h] = raw_sdigits4(__byte_perm(x0, x1, 0x0246));
+            hi[3 - h] = raw_sdigits4(__byte_perm((x0 + 0x00100010u) >> 5, (x1 + 0x00100010u) >> 5, 0x0246));
+          }
+          const uint32_t at = dst + (15 - g) * BR + 16 * c;
+          sts128(at, lo[0], lo[1], lo[2], lo[3]);
+          sts128(at + K::PL, hi[0], hi[1], hi[2], hi[3]);
+        }
+      }
+      fence_async_smem();
+      asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(a_full + 8 * ab) : "memory");
+    };
+    // this thread's ciphertext of a block, and its 64 coefficients
+    const int q4 = warp & 3, g = warp >> 2, c = 32 * q4 + lane;
+    const uint2 hpk = __ldg(reinterpret_cast<const uint2 *>(a.sk + C::SK - 64) + g);
+    uint32_t dn = 0;
+    auto decode = [&](int blk) {
+      const int base = blk * a.rows;
+      const bool valid = c < min(a.rows, a.n - base);
+      uint32_t w[2 * C::ET + 1];
+      w[2 * C::ET] = 0;
+      const uint8_t *src = a.ct + (size_t)(base + c) * C::CT + L * C::POLYCOMP + 8 * C::ET * g;
+#pragma unroll
+      for (int i = 0; i < C::ET; i++) {
+        uint2 v = make_uint2(0u, 0u);
+        if (valid) v = __ldg(reinterpret_cast<const uint2 *>(src) + i);
+        w[2 * i] = v.x;
+        w[2 * i + 1] = v.y;
+      }
+      ok = mbar_wait_bounded(d_full + 8 * (dn & 1), (dn >> 1) & 1);
+      if (!ok) return;
+      tc_fence_after();
+      const uint32_t tc = tmem + ((uint32_t)(32 * q4) << 16) + 256 * (dn & 1) + 64 * g;
+      uint32_t mw[2] = {0u, 0u};
+#pragma unroll
+      for (int k0 = 0; k0 < 64; k0 += 16) {
+        uint32_t f[16];
+        tmem_ld16(tc + k0, f);
+#pragma unroll
+        for (int i = 0; i < 16; i++) {
+          const int k = k0 + i, bit = C::ET * k, b5 = bit & 31;
+          // m'_k = ((x + h2 - (c_m,k << (ep - et))) mod p) >> (ep - 1)
+          const int x = __float2int_rn(__fmaf_rn(__uint_as_float(f[i]), 262144.0f, (float)C::H2));
+          const uint32_t cm =
+              b5 + C::ET <= 32 ? w[bit >> 5] >> b5 : __funnelshift_r(w[bit >> 5], w[(bit >> 5) + 1], b5);
+          const uint32_t v = (uint32_t)x - ((cm & ((1u << C::ET) - 1u)) << (C::EP - C::ET));
+          mw[k >> 5] |= ((v >> (C::EP - 1)) & 1u) << (k & 31);
+        }
+      }
+      tc_fence_before();
+      asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(d_empty + 8 * (dn & 1)) : "memory");
+      dn++;
+      if (valid) {
+        uint2 *mo = reinterpret_cast<uint2 *>(a.m_out + (size_t)(base + c) * 64);
+        mo[g] = make_uint2(mw[0], mw[1]);
+        mo[4 + g] = hpk;
+      }
+    };
+    // a block is decoded once two more buffers of digits are on their way
+    int last = -1;
+    for (int blk = blockIdx.x; ok && blk < a.blocks; blk += gridDim.x) {
+#pragma unroll 1
+      for (int j = 0; ok && j < L; j++) {
+        stage(blk, j);
+        if (ok && j == 1 && last >= 0) decode(last);
+      }
+      last = blk;
+    }
+    if (ok && last >= 0) decode(last);
+    if (!ok && a.err) atomicOr(a.err, 2);
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == kOkWorkers) tmem_dealloc(tmem, 512);
+}
+
 }  // namespace tmvp

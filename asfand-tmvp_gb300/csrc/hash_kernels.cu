@@ -294,6 +294,10 @@ bool sponges_split(const HashCfg &cfg, size_t n) {
 //    alone at one per SM and the rest as a second launch beside them: as one
 //    launch, four SMs get two of those blocks (key generation of 20011: 386 us,
 //    as two 324).
+//  * cfg.even: beside a kernel whose blocks take most of an SM each, blocks that
+//    fit anywhere pile up on the SMs it left or finished first; limited to an
+//    even share each, the one-key pass of 8192 takes 96 instead of 157 us, of
+//    20000 162 instead of 253.
 void plan_sponges(const HashCfg &cfg, const SpongeRole *roles, int nroles, SpongePlan (&S)[2]) {
   S[0] = SpongePlan{};
   S[1] = SpongePlan{};
@@ -322,10 +326,11 @@ void plan_sponges(const HashCfg &cfg, const SpongeRole *roles, int nroles, Spong
     if (form == kHashWarp) warps += rest;
     add_seg(S[split && k == 1], r.id, kHashThread, 0, full);
     add_seg(S[split && (k == 1 || form != kHashThread)], r.id, form, full, rest);
-    if (nroles == 1 && r.perms >= 4) {
+    if (nroles == 1) {
       // blocks per SM when every SM has its share
       const int q = (int)(full / (32 * W)) + (form == kHashThread && rest ? 1 : 0);
-      if (q <= 5 && (form == kHashThread || rest == 0 || q >= 2)) S[0].smem = smem_limit(q);
+      if (r.perms >= 4 && q <= 5 && (form == kHashThread || rest == 0 || q >= 2)) S[0].smem = smem_limit(q);
+      else if (cfg.even) S[0].smem = smem_limit((int)((S[0].blocks + cfg.sms - 1) / cfg.sms));
     }
     if (nroles == 2 && k == 0 && (full || form == kHashThread)) S[0].smem = smem_limit(cfg.cap > 0 ? cfg.cap : (full && !split ? 2 : 1));
   }

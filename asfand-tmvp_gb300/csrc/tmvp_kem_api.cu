@@ -470,9 +470,17 @@ DecScratch dec_scratch(const KemParams &P, size_t n, Arena &A) {
 // re-encryption (us): Saber 65536: 455 / 630, 16384: 151 / 197, 8192: 99 / 112,
 // 6000: 97 / 101, 4096: 87 / 84; FireSaber 6000: 147 / 145, 5000: 145 / 138;
 // LightSaber 4096: 61 / 64.
-// The planes (at most 444,416 bytes) go where the expanded A of the n instances
+// The planes (at most 444,416 and 63,488 bytes) go where the expanded A of the n instances
 // (1408 bytes or more each) would: no pass needs more workspace for them.
 inline bool onekey_matrix(size_t n) { return n >= 6144; }
+
+// Whether the decryption does too.  Its blocks take an SM each; the key's
+// GenMatrix, one chain of 10 to 40 permutations that bounds small passes, then
+// shares its SM with 16 busy warps.  Pass with the matrix / five or eight
+// ciphertexts a CTA (us): Saber 65536: 412 / 442, 16384: 137 / 148, 8192: 96 /
+// 104; LightSaber 8192: 77 / 78, 6144: 70 / 68; FireSaber 65536: 550 / 579,
+// 16384: 182 / 186, 12000: 163 / 158, 8192: 157 / 142.
+inline bool onekey_matrix_decrypt(const KemParams &P, size_t n) { return n >= (P.l < 4 ? 8192u : 16384u); }
 
 // Decapsulation of n instances in device memory (16-byte aligned): GenMatrix
 // and H(c) in one launch (2n sponges, so the integer pipe has warps enough)
@@ -492,7 +500,10 @@ int dec_pipeline(tmvp_ctx *c, const KemParams &P, size_t n, uint8_t *ss, const u
     TRY_CUDA(cudaEventRecord(c->fork_ev, s));
     TRY_CUDA(cudaStreamWaitEvent(side, c->fork_ev, 0));
   }
-  HashCfg h = hash_cfg(c);
+  const bool matrix = key_ops && onekey_matrix(n);
+  HashCfg h = hash_cfg(c), hg = h;
+  const bool matrix_dec = matrix && onekey_matrix_decrypt(P, n);
+  h.even = hg.even = matrix_dec;
   if (!a_cached && !c->serial) h.cap = (c->front_cap + 1) / 2;  // 64-thread blocks asked for, launched as 128
   // (GenMatrix given: the front is H(c) alone)
   const bool split = !a_cached && fork && sponges_split(h, n);
@@ -503,7 +514,6 @@ int dec_pipeline(tmvp_ctx *c, const KemParams &P, size_t n, uint8_t *ss, const u
       if (side == c->lane_side[l]) side2 = c->lane_side2[l];
     TRY_CUDA(cudaStreamWaitEvent(side2, c->fork_ev, 0));
   }
-  const bool matrix = key_ops && onekey_matrix(n);
   {
     StageTimer tm_(c, "dec_front", side);
     TRY_CUDA(launch_dec_front(h, P, sk, ct, w.a_stream, w.hc, n, !a_cached, side, side2));
@@ -522,18 +532,20 @@ int dec_pipeline(tmvp_ctx *c, const KemParams &P, size_t n, uint8_t *ss, const u
   a.copy_hpk = 1;
   a.key_shared = key_shared ? 1 : 0;
   if (key_shared && resolve_form(form) == kFp8Tcgen05) {
-    // one key: several ciphertexts per CTA share its staged secret and MMAs
+    // one key: one matrix product, or several ciphertexts per CTA that share its
+    // staged secret and MMAs
     StageTimer tm_(c, "cpa_decrypt_onekey_fp8_tcgen05", s);
     a.err = c->d_err;
-    const int e = cpa_launch_decrypt_onekey(a, s);
-    c->launches++;
+    const int e = matrix_dec ? onekey_decrypt(a, w.a_stream + up(onekey_operand_bytes(P)), c->nsm, s)
+                             : cpa_launch_decrypt_onekey(a, s);
+    c->launches += matrix_dec ? 2 : 1;
     if (e) return TMVP_EDEVICE;
   } else if ((r = run_cpa(c, form, kDecrypt, a, s))) {
     return r;
   }
   {
     StageTimer tm_(c, "dec_g", s);
-    TRY_CUDA(launch_dec_g(hash_cfg(c), P, w.mbuf, w.kr, w.s_stream, n, s));
+    TRY_CUDA(launch_dec_g(hg, P, w.mbuf, w.kr, w.s_stream, n, s));
   }
   c->launches++;
   TRY_CUDA(cudaStreamWaitEvent(s, c->join_ev, 0));  // join: GenMatrix

@@ -167,7 +167,8 @@ int tmvp_kem_dec_batch_a(tmvp_ctx *ctx, tmvp_param_set set, size_t n, uint8_t *s
  * of 39 Keccak-f per ciphertext), and with the tcgen05 form one CTA decrypts
  * 5 or 8 ciphertexts against the key's staged secret; from 6144 ciphertexts
  * (of a chunk) on, the re-encryption is one matrix product with the key's
- * digit planes, 128 ciphertexts a block.  Same bytes as
+ * digit planes, 128 ciphertexts a block, and from 8192 (l = 4: 16384) on so is
+ * the decryption.  Same bytes as
  * tmvp_kem_dec_batch with sk repeated n times.  The reference's saber_dec
  * and SABLE_dec also decapsulate their whole batch under one key
  * (TMVP-Saber/SABER-GPU/src/cuda_kernel.cu:320-321, TMVP_SABLE/src/

@@ -1,7 +1,9 @@
 """One-key decapsulation whose re-encryption is one matrix product (6144
-ciphertexts and more): both sides of that line, blocks of 128 ciphertexts with a
-remainder, runs of output polynomials that start inside a block, against the
-oracle, from device and from host buffers."""
+ciphertexts and more), and whose decryption is (8192; 16384 for l = 4): both
+sides of those lines, blocks of 128 ciphertexts with a remainder, runs of output
+polynomials that start inside a block, one to four blocks an SM, against the
+oracle, from device and from host buffers; and the secrets that the decryption
+accepts."""
 import os
 
 import numpy as np
@@ -14,7 +16,8 @@ THREADS = os.cpu_count() or 4
 
 @pytest.mark.parametrize("set_id,n", [(1, 6143), (1, 6144), (1, 6145), (0, 6271), (2, 6272), (3, 6273), (4, 6144 + 64),
                                       (5, 6144 + 65), (1, 152 * 128), (2, 152 * 128 + 1), (3, 152 * 64 - 1),
-                                      (0, 24577), (5, 20011)])
+                                      (0, 24577), (5, 20011), (0, 8191), (0, 8192), (3, 8193), (2, 16383), (2, 16384),
+                                      (5, 16385), (4, 152 * 256 + 1), (1, 152 * 384 + 5)])
 def test_onekey_matches_oracle(kem, oracle, set_id, n):
     import torch
     T, ctx = kem
@@ -33,3 +36,31 @@ def test_onekey_matches_oracle(kem, oracle, set_id, n):
     ctx.sync_status()
     assert np.array_equal(out.cpu().numpy(), want)
     assert np.array_equal(ctx.kem_dec_onekey(set_id, ct, sk[0]), want)
+
+
+@pytest.mark.parametrize("set_id,l", [(0, 2), (1, 3), (2, 4)])
+def test_onekey_secret_range(kem, oracle, set_id, l):
+    """-7 .. 7, as the per-instance decryption."""
+    T, ctx = kem
+    n = 16400
+    pk, sk = oracle.kem_keypair_batch(set_id, T.splitmix_bytes(9600, 96).reshape(1, 96), 1)
+    ct, _ = oracle.kem_enc_batch(set_id, np.repeat(pk, 16, axis=0), T.splitmix_bytes(9601, 512).reshape(16, 32), 1)
+    ct = np.tile(ct, (n // 16, 1))
+    rng = np.random.RandomState(5)
+    s = rng.randint(-7, 8, 256 * l)
+    s[::3] = 7
+    s[1::3] = -7
+
+    def pack(v):
+        return np.packbits((((v[:, None] & 0x1FFF) >> np.arange(13)) & 1).astype(np.uint8).reshape(-1), bitorder="little")
+
+    sk[0, :416 * l] = pack(s)
+    want, _ = oracle.kem_dec_batch(set_id, ct[:16], np.repeat(sk, 16, axis=0), THREADS)
+    assert np.array_equal(ctx.kem_dec_onekey(set_id, ct, sk[0]), np.tile(want, (n // 16, 1)))
+    for i, bad in enumerate((8, -8, 4095, -4096, 128)):
+        t = s.copy()
+        t[(97 * i + 3) % (256 * l)] = bad
+        sk[0, :416 * l] = pack(t)
+        with pytest.raises(T.TmvpError) as e:
+            ctx.kem_dec_onekey(set_id, ct, sk[0])
+        assert e.value.code == T.EINVAL
