@@ -56,14 +56,15 @@ SABER = 1
 CT_BYTES, SK_BYTES, PK_BYTES = 1088, 2304, 992
 # schoolbook-equivalent work of one negacyclic 256 x 256 product
 POLY_OPS = 2 * 256 * 256
-# SM cycles per tcgen05.mma kind::f8f6f4 with M = 128, N = 32, K = 32 when 4 CTAs per SM issue
-# back to back (measured on GB300 by the mma_rates workload); N = 256 takes 128
-MMA_CYCLES = 39.8
+# SM cycles per tcgen05.mma kind::f8f6f4 with M = 128, K = 32 when 4 CTAs per SM issue back to
+# back: 38.8 at N = 16, 39.8 at 32 and 48 at 64 (measured on GB300 by the mma_rates workload; N = 256
+# takes 128); about the 4 KB + 32 N bytes of its operands at 128 bytes a cycle, so 44 at N = 48
+MMA_CYCLES_N48 = 44.0
 MMA_CYCLES_N16 = 38.8
-# tcgen05.mma per Saber re-encryption: 3 secret polynomials x 8 Hankel windows,
-# each N = 32 over two K steps (the negacyclic wrap serves both M halves)
-REENC_MMAS = 24
-DEC_MMAS = 24
+# tcgen05.mma per Saber instance: 3 secret polynomials x 4 Hankel tiles, each against four K steps
+# (N = 4 x 12 digit columns for the re-encryption, 4 x 4 for the decryption)
+REENC_MMAS = 12
+DEC_MMAS = 12
 # the library's default host-buffer chunk and ramp (tmvp_ctx_set_host_chunk / _ramp)
 DEFAULT_HOST_CHUNK, DEFAULT_HOST_RAMP = 16384, 1
 
@@ -694,7 +695,7 @@ def _roofline_entries(stages, instances, hbm, bf16, peak_src, diag, nsm, sm_mhz)
             else:
                 rec.update({"peak": bf16, "frac": ach / bf16,
                             "peak_source": f"{peak_src} bf16 dense as a stand-in for e4m3"})
-            mmas, cyc, ncol = (REENC_MMAS, MMA_CYCLES, 32) if key == "cpa_reenc" else (DEC_MMAS, MMA_CYCLES_N16, 16)
+            mmas, cyc, ncol = (REENC_MMAS, MMA_CYCLES_N48, 48) if key == "cpa_reenc" else (DEC_MMAS, MMA_CYCLES_N16, 16)
             floor_s = per_launch * mmas * cyc / (nsm * sm_mhz * 1e6)
             rec["mma_instruction_floor_ms"] = floor_s * 1e3
             rec["frac_of_mma_floor"] = floor_s / avg_s
