@@ -24,6 +24,7 @@
 
 #include "chain.cuh"
 #include "cpa_persist.cuh"
+#include "hash_engine.cuh"
 
 namespace tmvp {
 
@@ -488,7 +489,10 @@ constexpr bool is_decryption(int op) { return op == kDecrypt || op == kDecryptK;
 // Saber, us, decryption / re-encryption: 203 / 281 before the core matrices came
 // from registers; without the MMAs 153 / 240, without the core matrices 154 /
 // 243, without the digits 185 / 209, inputs from L2 203 / 281).
-template <int OP, int SET, class AT>
+//
+// TAIL: warp 0 finishes the instance (CpaArgs::tail) while the others go on to
+// the next one's first barrier.
+template <int OP, int SET, bool TAIL = false, class AT>
 __device__ __forceinline__ void cpa5i_run(const AT &at, uint8_t *sm) {
   using C = SetC<SET>;
   using S = ShapeC<OP, SET>;
@@ -874,7 +878,17 @@ __device__ __forceinline__ void cpa5i_run(const AT &at, uint8_t *sm) {
       else diffm = ((v - (mk << (C::EP - 1))) >> (C::EP - C::ET)) ^ cf[L];
     }
     diff = (diff & pmask) | (diffm & ((1u << C::ET) - 1u));
-    if (__any_sync(0xffffffffu, diff != 0u) && lane == 0) a.fail[inst] = 1;
+    if constexpr (TAIL) {
+      const bool bad = __syncthreads_or(diff != 0u) != 0;
+      if (warp == 0) {
+        const WarpSponge e{lane, true, warp_keccak_lane(lane)};
+        const uint8_t *z = a.sk + (a.key_shared ? 0 : (size_t)inst * C::SK) + C::SK - 32;
+        const auto kk = e.sel4(e.load(a.kr + (size_t)inst * 64, 4), e.load(z, 4), bad);
+        e.store(a.ss + (size_t)inst * 32, e.template sha3_256<8>(e.cat4(kk, e.load(a.hc + (size_t)inst * 32, 4))), 4);
+      }
+    } else {
+      if (__any_sync(0xffffffffu, diff != 0u) && lane == 0) a.fail[inst] = 1;
+    }
   } else if constexpr (OP == kMatvec) {
     // coefficient k of every output polynomial, mod 2^eq
     const uint32_t m = (1u << a.mv_eq) - 1u;
@@ -895,6 +909,11 @@ __device__ __forceinline__ void cpa5i_run(const AT &at, uint8_t *sm) {
     }
     __syncthreads();
     copy16(a.ct_out + (size_t)inst * C::CT, sm + LO::OUT, C::CT);
+    if (TAIL && warp == 0) {
+      const WarpSponge e{lane, true, warp_keccak_lane(lane)};
+      const auto h = e.sha3_256_mem(sm + LO::OUT, C::CT);
+      e.store(a.ss + (size_t)inst * 32, e.template sha3_256<8>(e.cat4(e.load(a.kr + (size_t)inst * 64, 4), h)), 4);
+    }
   } else if (OP == kKeygen) {
     constexpr int bbytes = L * C::POLYCOMP;
     uint8_t *outb = sm + LO::OUT;
@@ -923,6 +942,14 @@ __device__ __forceinline__ void cpa5i_run(const AT &at, uint8_t *sm) {
     copy16(pko, outb, bbytes);
     copy16(sko + C::INDCPA_SK, outb, bbytes);
     copy16(sko, outb + bbytes, C::INDCPA_SK);
+    if constexpr (TAIL) {
+      __syncthreads();  // pk is complete in global memory
+      if (warp == 0) {
+        const WarpSponge e{lane, true, warp_keccak_lane(lane)};
+        const auto h = e.sha3_256_mem(pko, C::PK);
+        e.store(sko + C::SK - 64, e.cat4(h, e.load(a.coins + (size_t)inst * 96 + 64, 4)), 8);
+      }
+    }
   }
   if (next == ~0u) break;
   gi = next;
@@ -953,6 +980,13 @@ template <int OP, int SET>
 __global__ void __launch_bounds__(kI5Threads, min_ctas<OP, SET>()) k_cpa5i(const __grid_constant__ CpaArgs a) {
   extern __shared__ __align__(16) uint8_t sm[];
   cpa5i_run<OP, SET>([&](unsigned gi) { return CpaAt{a, gi}; }, sm);
+}
+
+// The same with the instance's last Keccak stage in it (CpaArgs::tail).
+template <int OP, int SET>
+__global__ void __launch_bounds__(kI5Threads, 2) k_cpa5t(const __grid_constant__ CpaArgs a) {
+  extern __shared__ __align__(16) uint8_t sm[];
+  cpa5i_run<OP, SET, true>([&](unsigned gi) { return CpaAt{a, gi}; }, sm);
 }
 
 // Mixed launch whose groups all have parameter set SET (the per-set launches
@@ -1046,6 +1080,9 @@ inline int launch_cpa5i(const CpaArgs &a, cudaStream_t s) {
   using LO = LayoutC<OP, SET>;
   using S = ShapeC<OP, SET>;
   auto fn = k_cpa5i<OP, SET>;
+  if constexpr (OP == kReenc || OP == kEncrypt || OP == kKeygen) {
+    if (a.tail) fn = k_cpa5t<OP, SET>;
+  }
   int smem = LO::TOTAL;
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
   if (e != cudaSuccess) return (int)e;

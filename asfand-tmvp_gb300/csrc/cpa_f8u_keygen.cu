@@ -9,7 +9,7 @@
 namespace tmvp {
 int cpa_launch_f8u_keygen(const CpaArgs &a, cudaStream_t s) {
   const int mode = persist_ctas_per_sm(kKeygen, a.P.set);
-  if (mode < 0) return launch_cpa5i_set<kKeygen>(a, s);  // one CTA per instance
+  if (mode < 0 || a.tail) return launch_cpa5i_set<kKeygen>(a, s);  // one CTA per instance
   return launch_persist<kKeygen>(&a, 1, nullptr, s, mode);
 }
 int cpa_launch_mixed_keygen(const CpaArgs *g, int ng, const MixTable *dev_tab, cudaStream_t s, int ctas_per_sm) {

@@ -55,6 +55,13 @@ struct CpaArgs {
   // tcgen05 per-instance kernel only: sk (decryption) and a_stream
   // (re-encryption) hold one key for every instance (stride 0)
   int key_shared;
+  // tcgen05 per-instance kernel only (small batches): a warp of the instance's
+  // CTA goes on with its last Keccak stage.  kReenc: K = H((fail ? z : kr) || hc)
+  // (z from sk, one key if key_shared); kEncrypt: K = H(kr || H(c)); kKeygen:
+  // H(pk) || z (coins + i * 96 + 64) into sk.
+  int tail;
+  const uint8_t *kr, *hc, *coins;
+  uint8_t *ss;
 };
 
 // Launch over a.n instances on `stream`.  Returns a CUDA error code (0 on
