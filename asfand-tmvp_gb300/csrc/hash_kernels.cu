@@ -278,6 +278,10 @@ bool sponges_split(const HashCfg &cfg, size_t n) {
 //    two threads a sponge 67 us up to 16, one thread 109 us up to 32: the
 //    forms' lines.  Past whole rounds of 32, the rest goes the same way beside
 //    them: 20011 sponges in 122 us instead of 206.
+//    A one-role launch that shares the GPU (G, H(c) alone) leaves the warp form,
+//    which issues five times the instructions, at 1.5: decapsulation of 1000
+//    Saber 83 -> 77 us, of 1600 107 -> 91, of 1200 FireSaber 144 -> 134, of 1600
+//    with cached A 70 -> 54.
 //  * Two roles side by side: longest first, and few blocks resident, so that
 //    an SM that finishes early takes the next block instead of all being
 //    placed at the start: with one block per SM 16384 x (23 + 9) takes 135
@@ -321,7 +325,8 @@ void plan_sponges(const HashCfg &cfg, const SpongeRole *roles, int nroles, Spong
     const SpongeRole &r = roles[order[k]];
     const size_t full = r.n / (32 * W) * (32 * W), rest = r.n - full;
     int form = kHashThread;
-    if (warps + rest <= (full ? 9 * W / 4 : 11 * W / 4)) form = kHashWarp;
+    const size_t line = full ? 9 * W / 4 : (cfg.beside && nroles == 1 ? 3 * W / 2 : 11 * W / 4);
+    if (warps + rest <= line) form = kHashWarp;
     else if (rest <= 16 * W) form = kHashPair;
     if (form == kHashWarp) warps += rest;
     add_seg(S[split && k == 1], r.id, kHashThread, 0, full);

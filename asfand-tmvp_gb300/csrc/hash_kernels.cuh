@@ -40,6 +40,7 @@ struct HashCfg {
   bool limits = false;
   size_t warp_max = kWarpHashDefault, pair_max = kPairHashDefault;
   int cap = 0;
+  bool beside = false;  // the launch shares the GPU with others of its pass
   bool even = false;  // one role: its blocks limited to an even share per SM in every form
 };
 

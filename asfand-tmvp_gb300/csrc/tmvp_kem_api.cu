@@ -512,7 +512,9 @@ int dec_pipeline(tmvp_ctx *c, const KemParams &P, size_t n, uint8_t *ss, const u
     TRY_CUDA(cudaStreamWaitEvent(side, c->fork_ev, 0));
   }
   const bool matrix = key_ops && onekey_matrix(n);
-  HashCfg h = hash_cfg(c), hg = h;
+  HashCfg h = hash_cfg(c);
+  h.beside = true;
+  HashCfg hg = h;
   const bool matrix_dec = matrix && onekey_matrix_decrypt(P, n);
   h.even = hg.even = matrix_dec;
   if (!a_cached && !c->serial) h.cap = (c->front_cap + 1) / 2;  // 64-thread blocks asked for, launched as 128
@@ -1818,7 +1820,9 @@ int mixed_enqueue(tmvp_ctx *c, size_t ng, const tmvp_dec_group *gr, uint8_t *ws,
   nsets = r1;
   {
     StageTimer tm_(c, "mix_g", s);
-    TRY_CUDA(launch_mix_g(hash_cfg(c), th, (int)ng, (size_t)total, gp, s));
+    HashCfg hg = hash_cfg(c);
+    hg.beside = true;
+    TRY_CUDA(launch_mix_g(hg, th, (int)ng, (size_t)total, gp, s));
   }
   TRY_CUDA(cudaStreamWaitEvent(s, c->join_ev, 0));  // GenMatrix
   if (split) TRY_CUDA(cudaStreamWaitEvent(s, c->join2_ev, 0));

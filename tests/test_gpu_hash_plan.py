@@ -36,3 +36,26 @@ def test_kem_matches_oracle(kem, oracle, n):
     torch.cuda.synchronize()
     assert np.array_equal(out.cpu().numpy(), want)
     assert np.array_equal(ctx.kem_dec(set_id, ct, sk), want)
+
+
+@pytest.mark.parametrize("n", [3 * PARTS // 2, 3 * PARTS // 2 + 1, 11 * PARTS // 4 + 1])
+def test_cached_decapsulation_matches_oracle(kem, oracle, n):
+    """H(c) and G as launches of one role beside others: both sides of the line
+    where they leave the warp form."""
+    import torch
+    T, ctx = kem
+    set_id = T.FIRESABER if n % 2 else T.SABER
+    opk, osk = oracle.kem_keypair_batch(set_id, T.splitmix_bytes(8300 + n, n * 96).reshape(n, 96), THREADS)
+    ct, _ = oracle.kem_enc_batch(set_id, opk, T.splitmix_bytes(8400 + n, n * 32).reshape(n, 32), THREADS)
+    ct[::3, 5] ^= 0x41
+    want, _ = oracle.kem_dec_batch(set_id, ct, osk, THREADS)
+    dpk, dsk, dct = (torch.from_numpy(x).cuda() for x in (opk, osk, ct))
+    a = torch.empty((n, T.genmatrix_bytes(set_id)), dtype=torch.uint8, device="cuda")
+    out = torch.empty((n, 32), dtype=torch.uint8, device="cuda")
+    ctx.genmatrix_ptr(set_id, n, a, dpk)
+    ctx.kem_dec_a_ptr(set_id, n, out, dct, dsk, a)
+    torch.cuda.synchronize()
+    assert np.array_equal(out.cpu().numpy(), want)
+    ctx.kem_dec_ptr(set_id, n, out, dct, dsk)
+    torch.cuda.synchronize()
+    assert np.array_equal(out.cpu().numpy(), want)
