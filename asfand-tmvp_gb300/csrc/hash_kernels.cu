@@ -281,7 +281,9 @@ bool sponges_split(const HashCfg &cfg, size_t n) {
 //    A one-role launch that shares the GPU (G, H(c) alone) leaves the warp form,
 //    which issues five times the instructions, at 1.5: decapsulation of 1000
 //    Saber 83 -> 77 us, of 1600 107 -> 91, of 1200 FireSaber 144 -> 134, of 1600
-//    with cached A 70 -> 54.
+//    with cached A 70 -> 54.  The shorter role of a front beside the decryption
+//    does so at 2 in all: decapsulation of 800 Saber 87 -> 78 us, FireSaber 125
+//    -> 113, LightSaber 54 -> 46.
 //  * Two roles side by side: longest first, and few blocks resident, so that
 //    an SM that finishes early takes the next block instead of all being
 //    placed at the start: with one block per SM 16384 x (23 + 9) takes 135
@@ -325,7 +327,8 @@ void plan_sponges(const HashCfg &cfg, const SpongeRole *roles, int nroles, Spong
     const SpongeRole &r = roles[order[k]];
     const size_t full = r.n / (32 * W) * (32 * W), rest = r.n - full;
     int form = kHashThread;
-    const size_t line = full ? 9 * W / 4 : (cfg.beside && nroles == 1 ? 3 * W / 2 : 11 * W / 4);
+    const bool slack = cfg.beside && k == 1 && 5 * r.perms <= 3 * roles[order[0]].perms;  // ends first in either form
+    const size_t line = full ? 9 * W / 4 : (slack ? 2 * W : (cfg.beside && nroles == 1 ? 3 * W / 2 : 11 * W / 4));
     if (warps + rest <= line) form = kHashWarp;
     else if (rest <= 16 * W) form = kHashPair;
     if (form == kHashWarp) warps += rest;

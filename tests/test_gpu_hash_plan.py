@@ -38,10 +38,10 @@ def test_kem_matches_oracle(kem, oracle, n):
     assert np.array_equal(ctx.kem_dec(set_id, ct, sk), want)
 
 
-@pytest.mark.parametrize("n", [3 * PARTS // 2, 3 * PARTS // 2 + 1, 11 * PARTS // 4 + 1])
+@pytest.mark.parametrize("n", [PARTS, PARTS + 1, 3 * PARTS // 2, 3 * PARTS // 2 + 1, 11 * PARTS // 4 + 1])
 def test_cached_decapsulation_matches_oracle(kem, oracle, n):
-    """H(c) and G as launches of one role beside others: both sides of the line
-    where they leave the warp form."""
+    """H(c) and G beside others, with GenMatrix and as launches of their own: both
+    sides of the lines where they leave the warp form."""
     import torch
     T, ctx = kem
     set_id = T.FIRESABER if n % 2 else T.SABER
