@@ -134,9 +134,13 @@ __device__ __forceinline__ void keccak_absorb_words(uint64_t (&A)[25], const uin
   while (nw >= RATE_W) {
 #pragma unroll
     for (int i = 0; i < RATE_W; i++) A[i] ^= in[i];
-    keccak_f1600(A);
     in += RATE_W;
     nw -= RATE_W;
+    if (nw > 0) {  // the next block's lines, while this one is permuted (front of 32768 Saber 271 -> 266 us)
+      asm volatile("prefetch.L1 [%0];" ::"l"(in));
+      asm volatile("prefetch.L1 [%0];" ::"l"(in + (nw < RATE_W ? nw : RATE_W) - 1));
+    }
+    keccak_f1600(A);
   }
   // tail of nw < RATE_W whole words, then the domain byte in word nw
 #pragma unroll
