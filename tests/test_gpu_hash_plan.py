@@ -1,7 +1,8 @@
 """How a Keccak launch's sponges are spread (plan_sponges): one warp, two
 threads or one thread per sponge by count, whole rounds of 32 sponges per SM
 sub-partition with the remainder in a finer form, and two launches side by side
-just above one round.  Batches at both sides of every line, against the oracle."""
+just above one round; below it the shorter of two roles partly in two threads a
+sponge.  Batches at both sides of every line, against the oracle."""
 import os
 
 import numpy as np
@@ -13,7 +14,7 @@ THREADS = os.cpu_count() or 4
 PARTS = 4 * 152  # sub-partitions
 
 
-@pytest.mark.parametrize("n", [11 * PARTS // 8, 11 * PARTS // 8 + 1, 11 * PARTS // 4 + 1, 16 * PARTS, 16 * PARTS + 1,
+@pytest.mark.parametrize("n", [9800, 14001, 15000, 16384, 11 * PARTS // 8, 11 * PARTS // 8 + 1, 11 * PARTS // 4 + 1, 16 * PARTS, 16 * PARTS + 1,
                                32 * PARTS - 1, 32 * PARTS, 32 * PARTS + 9 * PARTS // 8 + 1, 32 * PARTS + 9 * PARTS // 4 + 1,
                                48 * PARTS - 1, 48 * PARTS, 64 * PARTS + 3])
 def test_kem_matches_oracle(kem, oracle, n):
