@@ -223,7 +223,9 @@ cudaError_t launch_sponges(const SpongePlan &S, const R &r, cudaStream_t s) {
   if (S.blocks == 0) return cudaSuccess;
   auto fn = k_sponges<R>;
   if (S.smem > 48 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S.smem);
+    // always the largest limit: the attribute is the function's, so a smaller one set by
+    // another thread's context would refuse a launch of this one
+    const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kSpongeSmemMax);
     if (e != cudaSuccess) return e;
   }
   return launch_chained(fn, S.blocks, S.threads, S.smem, s, S, r);
@@ -261,7 +263,9 @@ static void add_seg(SpongePlan &S, int role, int form, size_t first, size_t coun
 
 // Shared memory that leaves room for at most `blocks` blocks per SM (228 KB,
 // 1 KB of it per block reserved).
-static unsigned smem_limit(int blocks) { return blocks <= 1 ? 117000u : (unsigned)(227 * 1024 / (blocks + 1)); }
+static unsigned smem_limit(int blocks) {
+  return blocks <= 1 ? (unsigned)kSpongeSmemMax : (unsigned)(227 * 1024 / (blocks + 1));
+}
 
 // Two thread-form roles below one round, n1 sponges of p1 permutations and n2 of
 // p2 <= p1, one block resident per SM: how many of the n2 run in the thread form.

@@ -61,6 +61,7 @@ struct SpongeRole {
   int id = 0;  // the stage's name for the role
 };
 constexpr unsigned kHashBlock = 128;
+constexpr int kSpongeSmemMax = 117000;  // the most shared memory a plan asks for (one block per SM)
 // One or two roles over the GPU: S[0] and S[1] (empty unless sponges_split),
 // two launches that run side by side.
 void plan_sponges(const HashCfg &cfg, const SpongeRole *roles, int nroles, SpongePlan (&S)[2]);
