@@ -7,7 +7,9 @@
 // all words in one thread, their 32-bit halves in two, or word k in lane k.
 // Every thread of a warp calls an engine's functions together (the pair and
 // warp forms exchange by shuffles); `live` is false in threads that only
-// repeat another sponge's work, and they store nothing.
+// repeat another sponge's work, and they store nothing.  The 16 sponges of a
+// pair-form warp may have different lengths (a mixed pass's groups): all its
+// threads permute as often as the longest of them needs.
 #pragma once
 #include <cstddef>
 #include <cstdint>
@@ -169,17 +171,16 @@ struct PairSponge {
     uint32_t w[25];
     absorb_seed(w, a);
     uint32_t *o32 = reinterpret_cast<uint32_t *>(out) + me;
-    int nw = nbytes >> 3;
-    while (nw > 0) {
+    const int nw = nbytes >> 3;
+    const int most = __reduce_max_sync(0xFFFFFFFFu, nw);  // (a warp may hold sponges of several parameter sets)
+    for (int at = 0; at < most; at += 21) {
       pair_keccak_f1600(w, me);
-      const int k = nw < 21 ? nw : 21;
       if (live) {
 #pragma unroll
         for (int q = 0; q < 21; q++)
-          if (q < k) o32[2 * q] = w[q];
+          if (q < nw - at) o32[2 * q] = w[q];
       }
       o32 += 2 * 21;
-      nw -= k;
     }
   }
   __device__ __forceinline__ Msg shake128_first(const Msg &a) const {

@@ -106,7 +106,8 @@ __device__ __forceinline__ void pair_sha3_lanes(int me, const uint32_t *m, int n
 
 // SHA3-256 of nbytes (a multiple of 8) at in: this thread's halves of the
 // four digest words.  The words of a block are loaded before the permutation
-// of the one before it.
+// of the one before it.  nbytes may differ between the pairs of a warp: each
+// takes its digest after its own last block and goes on to the longest one's.
 __device__ __forceinline__ void pair_sha3_256_mem(int me, const uint8_t *in, int nbytes, uint32_t (&h)[4]) {
   constexpr int RATE_W = 17;
   const uint32_t *in32 = reinterpret_cast<const uint32_t *>(in) + me;
@@ -114,22 +115,23 @@ __device__ __forceinline__ void pair_sha3_256_mem(int me, const uint8_t *in, int
   uint32_t w[25], nx[RATE_W];
   pair_zero(w);
   int nw = nbytes >> 3;
+  const int most = __reduce_max_sync(0xFFFFFFFFu, nw);
 #pragma unroll
   for (int i = 0; i < RATE_W; i++) nx[i] = i < nw ? in32[2 * i] : 0u;
-  for (;;) {
-    const bool last = nw < RATE_W;
+  for (int at = 0; at <= most; at += RATE_W) {  // (a message of whole blocks has a last one of padding)
 #pragma unroll
     for (int i = 0; i < RATE_W; i++) w[i] ^= i == nw ? dom : nx[i];
+    const bool last = nw >= 0 && nw < RATE_W;
     if (last) w[RATE_W - 1] ^= pair_half(0x8000000000000000ull, me);
     in32 += 2 * RATE_W;
     nw -= RATE_W;
 #pragma unroll
     for (int i = 0; i < RATE_W; i++) nx[i] = i < nw ? in32[2 * i] : 0u;
     pair_keccak_f1600(w, me);
-    if (last) break;
-  }
 #pragma unroll
-  for (int i = 0; i < 4; i++) h[i] = w[i];
+    for (int i = 0; i < 4; i++)
+      if (last) h[i] = w[i];
+  }
 }
 
 }  // namespace tmvp
