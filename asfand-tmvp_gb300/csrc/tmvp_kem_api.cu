@@ -1094,6 +1094,9 @@ int tmvp_kem_dec_batch_onekey(tmvp_ctx *c, tmvp_param_set set, size_t n, uint8_t
     TRY_CUDA(cudaEventRecord(c->fork_ev, s));
     for (int l = 0; l < NL; l++) TRY_CUDA(cudaStreamWaitEvent(c->lane[l], c->fork_ev, 0));
     TRY_CUDA(cudaStreamWaitEvent(c->side, c->fork_ev, 0));
+    // (the copies too: an earlier call may still use the workspace, and the inputs
+    // may be still on their way on the caller's stream)
+    TRY_CUDA(cudaStreamWaitEvent(c->copy[0], c->fork_ev, 0));
     {
       StageTimer tm_(c, "genmatrix", c->side);
       TRY_CUDA(launch_genmatrix(hash_cfg(c), P, bsk.dev + P.indcpa_sk_bytes, 0, a_one, 1, c->side));
@@ -1226,6 +1229,9 @@ int tmvp_kem_dec_batch(tmvp_ctx *c, tmvp_param_set set, size_t n, uint8_t *ss, c
       for (int l = 0; l < NL; l++) ss_stage[l] = A.take(cn * 32);
     TRY_CUDA(cudaEventRecord(c->fork_ev, s));
     for (int l = 0; l < tmvp_ctx::kLanes; l++) TRY_CUDA(cudaStreamWaitEvent(c->lane[l], c->fork_ev, 0));
+    // (the copies too: an earlier call may still use the workspace, and the inputs
+    // may be still on their way on the caller's stream)
+    TRY_CUDA(cudaStreamWaitEvent(c->copy[0], c->fork_ev, 0));
     if (a_full) {
       TRY_CUDA(cudaStreamWaitEvent(c->side, c->fork_ev, 0));
       {
