@@ -307,7 +307,7 @@ __global__ void __launch_bounds__(kOkThreads, 1) k_onekey_reenc(const __grid_con
           m[0] = v.x;
           m[1] = v.y;
         }
-        ok = mbar_wait_bounded(d_full + 8 * (dn & 1), (dn >> 1) & 1);
+        ok = mbar_wait_warp(d_full + 8 * (dn & 1), (dn >> 1) & 1);
         if (!ok) return;
         tc_fence_after();
         // one secret buffer: the block's MMAs are over now
@@ -482,7 +482,7 @@ __global__ void __launch_bounds__(kOkDecThreads, 1) k_onekey_decrypt(const __gri
     // x 4 chunks of 16 coefficients a warp task
     auto stage = [&](int blk, int j) {
       const uint32_t ab = item & 1;
-      ok = item < 2 || mbar_wait_bounded(a_empty + 8 * ab, ((item >> 1) - 1) & 1);
+      ok = item < 2 || mbar_wait_warp(a_empty + 8 * ab, ((item >> 1) - 1) & 1);
       item++;
       if (!ok) return;
       const int base = blk * a.rows, nv = min(a.rows, a.n - base);
@@ -533,7 +533,7 @@ __global__ void __launch_bounds__(kOkDecThreads, 1) k_onekey_decrypt(const __gri
         w[2 * i] = v.x;
         w[2 * i + 1] = v.y;
       }
-      ok = mbar_wait_bounded(d_full + 8 * (dn & 1), (dn >> 1) & 1);
+      ok = mbar_wait_warp(d_full + 8 * (dn & 1), (dn >> 1) & 1);
       if (!ok) return;
       tc_fence_after();
       const uint32_t tc = tmem + ((uint32_t)(32 * q4) << 16) + 256 * (dn & 1) + 64 * g;

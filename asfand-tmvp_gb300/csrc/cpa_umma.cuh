@@ -160,6 +160,13 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t mbar, uint32_t parity
   return false;
 }
 
+// The same by a whole warp, true in all its lanes or in none: lanes reach the
+// bound at different polls, and what follows the wait (shuffles, tensor-memory
+// loads) needs all of them.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t mbar, uint32_t parity) {
+  return __all_sync(0xffffffffu, mbar_wait_bounded(mbar, parity)) != 0;
+}
+
 // The same bound, polling without sleeping: for one thread whose wait is short
 // and on whose wake-up others depend.
 __device__ __forceinline__ bool mbar_spin_bounded(uint32_t mbar, uint32_t parity) {
