@@ -37,4 +37,16 @@ inline cudaError_t launch_chained(void (*fn)(P...), unsigned blocks, unsigned th
   return cudaLaunchKernelEx(&cfg, fn, args...);
 }
 
+// Lets launches of fn ask for any dynamic shared memory that a block can have.
+// The limit belongs to the kernel, for all host threads: one set to each launch's
+// own size could refuse a larger launch that another thread is making.
+template <class... P>
+inline cudaError_t allow_shared_memory(void (*fn)(P...)) {
+  constexpr int kBlockMax = 227 * 1024;
+  cudaFuncAttributes at{};
+  const cudaError_t e = cudaFuncGetAttributes(&at, fn);
+  if (e != cudaSuccess) return e;
+  return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kBlockMax - (int)at.sharedSizeBytes);
+}
+
 }  // namespace tmvp

@@ -18,6 +18,7 @@
 #include <cstddef>
 #include <cstdint>
 
+#include "chain.cuh"
 #include "cpa_engine.cuh"
 #include "cpa_kernels.cuh"
 #include "cpa_tc.cuh"
@@ -421,8 +422,7 @@ inline int launch_one(const CpaArgs &a, cudaStream_t s) {
   } else {
     using C = CpaCfg<FORM, OP, L, Q>;
     const CpaLayout lo = cpa_layout<FORM, OP, L, Q>(a.P);
-    cudaError_t e = cudaFuncSetAttribute(k_cpa<FORM, OP, L, Q>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, lo.total);
+    const cudaError_t e = allow_shared_memory(k_cpa<FORM, OP, L, Q>);
     if (e != cudaSuccess) return (int)e;
     k_cpa<FORM, OP, L, Q><<<a.n, C::NT, lo.total, s>>>(a);
     return (int)cudaGetLastError();

@@ -713,7 +713,7 @@ inline int launch_persist(const CpaArgs *groups, int ng, const MixTable *dev_tab
   }
   const PLayout lo = persist_layout<OP>(groups, ng);
   auto fn = k_cpa5p<OP>;
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, lo.total);
+  cudaError_t e = allow_shared_memory(fn);
   if (e != cudaSuccess) return (int)e;
   e = cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
   if (e != cudaSuccess) return (int)e;

@@ -15,6 +15,7 @@
 #pragma once
 #include <cstdint>
 
+#include "chain.cuh"
 #include "cpa_kernels.cuh"
 #include "cpa_tc.cuh"
 
@@ -407,7 +408,7 @@ inline int launch_tc(const CpaArgs &a, cudaStream_t s) {
   int smem = lo.total;
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
   if (e != cudaSuccess) return (int)e;
-  e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  e = allow_shared_memory(fn);
   if (e != cudaSuccess) return (int)e;
   fn<<<a.n, 128, smem, s>>>(a, lo);
   return (int)cudaGetLastError();
