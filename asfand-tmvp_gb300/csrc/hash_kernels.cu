@@ -182,16 +182,14 @@ struct MixFinal : MixBase {
 // one warp in a launch that has only the warp form (few sponges then spread
 // over all SMs: four on one SM share its shuffle unit, 51.2 against 49.2 us
 // for 17 LightSaber encapsulations).
-// The segment, form and role depend on blockIdx alone.  Past the end of a
+// The segment, form and role depend on the block alone.  Past the end of a
 // segment the pair and warp forms repeat its last sponge (their shuffles need
 // every thread) and store nothing.
 template <class R>
-__global__ void __launch_bounds__(kHashBlock) k_sponges(const __grid_constant__ SpongePlan S,
-                                                        const __grid_constant__ R r) {
-  chain_wait();
+__device__ __forceinline__ void sponge_block(const SpongePlan &S, const R &r, const unsigned block) {
   int k = 0;
-  while (k + 1 < S.nseg && blockIdx.x >= S.seg[k + 1].block0) k++;
-  const unsigned b = blockIdx.x - S.seg[k].block0, count = S.seg[k].count, first = S.seg[k].first;
+  while (k + 1 < S.nseg && block >= S.seg[k + 1].block0) k++;
+  const unsigned b = block - S.seg[k].block0, count = S.seg[k].count, first = S.seg[k].first;
   const int role = S.seg[k].role;
   switch (S.seg[k].form) {
     case kHashThread: {
@@ -212,6 +210,22 @@ __global__ void __launch_bounds__(kHashBlock) k_sponges(const __grid_constant__ 
       r.run(WarpSponge{lane, live, warp_keccak_lane(lane)}, role, first + (live ? i : count - 1));
     }
   }
+}
+
+template <class R>
+__global__ void __launch_bounds__(kHashBlock) k_sponges(const __grid_constant__ SpongePlan S,
+                                                        const __grid_constant__ R r) {
+  chain_wait();
+  sponge_block(S, r, blockIdx.x);
+}
+
+// The same by fewer blocks than the plan has, each taking every gridDim.x-th of
+// them: a capped front holds neither threads nor shared memory beyond its blocks.
+template <class R>
+__global__ void __launch_bounds__(kHashBlock) k_sponges_strided(const __grid_constant__ SpongePlan S,
+                                                                const __grid_constant__ R r) {
+  chain_wait();
+  for (unsigned b = blockIdx.x; b < S.blocks; b += gridDim.x) sponge_block(S, r, b);
 }
 
 unsigned per_block(int form) {
@@ -341,7 +355,6 @@ void plan_sponges(const HashCfg &cfg, const SpongeRole *roles, int nroles, Spong
                      : (short_sponges ? 2 * total : total) <= cfg.pair_max ? kHashPair
                                                                            : kHashThread;
     for (int k = 0; k < nroles; k++) add_seg(S[0], roles[order[k]].id, form, 0, roles[order[k]].n);
-    if (cfg.cap > 0) S[0].smem = smem_limit(cfg.cap);
     return;
   }
   const size_t W = 4 * (size_t)cfg.sms;  // sub-partitions
@@ -358,7 +371,7 @@ void plan_sponges(const HashCfg &cfg, const SpongeRole *roles, int nroles, Spong
     if (form == kHashWarp) warps += rest;
     add_seg(S[split && k == 1], r.id, kHashThread, 0, full);
     size_t fit = rest;
-    if (k == 1 && form == kHashThread && !full && roles[order[0]].n < 32 * W)
+    if (k == 1 && form == kHashThread && !full && cfg.cap == 0 && roles[order[0]].n < 32 * W)
       fit = thread_part(cfg.sms, roles[order[0]].n, roles[order[0]].perms, rest, r.perms);
     add_seg(S[split && (k == 1 || form != kHashThread)], r.id, form, full, fit);
     add_seg(S[split && k == 1], r.id, kHashPair, full + fit, rest - fit);
@@ -368,13 +381,21 @@ void plan_sponges(const HashCfg &cfg, const SpongeRole *roles, int nroles, Spong
       if (r.perms >= 4 && q <= 5 && (form == kHashThread || rest == 0 || q >= 2)) S[0].smem = smem_limit(q);
       else if (cfg.even) S[0].smem = smem_limit((int)((S[0].blocks + cfg.sms - 1) / cfg.sms));
     }
-    if (nroles == 2 && k == 0 && (full || form == kHashThread)) S[0].smem = smem_limit(cfg.cap > 0 ? cfg.cap : (full && !split ? 2 : 1));
+    if (nroles == 2 && k == 0 && (cfg.cap == 0 || split) && (full || form == kHashThread))
+      S[0].smem = smem_limit(full && !split ? 2 : 1);
   }
 }
 
 cudaError_t launch_dec_front(const HashCfg &cfg, const KemParams &P, const uint8_t *sk, const uint8_t *ct,
                              uint8_t *a_stream, uint8_t *hc, size_t n, bool with_gm, cudaStream_t s, cudaStream_t s2) {
   const SpongeRole roles[2] = {{n, gm_perms(P), 0}, {n, sha3_256_perms(P.ct_bytes), 1}};
+  if (cfg.cap > 0 && with_gm && !sponges_split(cfg, n)) {  // one launch, no limit but the cap on its blocks
+    SpongePlan S[2];
+    plan_sponges(cfg, roles, 2, S);
+    const unsigned most = (unsigned)(cfg.cap * cfg.sms);
+    if (S[0].seg[0].form == kHashThread && S[0].blocks > most)
+      return launch_chained(k_sponges_strided<DecFront>, most, kHashBlock, 0, s, S[0], DecFront{P, sk, ct, a_stream, hc});
+  }
   return launch_sponges(cfg, with_gm ? roles : roles + 1, with_gm ? 2 : 1, DecFront{P, sk, ct, a_stream, hc}, s, s2);
 }
 

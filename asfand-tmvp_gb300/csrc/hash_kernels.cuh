@@ -33,7 +33,11 @@ enum HashForm { kHashThread, kHashWarp, kHashPair };
 // _pair_hash), a launch of at most warp_max sponges runs one warp per sponge,
 // else of at most pair_max two threads per sponge, else one thread (short
 // sponges counting four times against the first and twice against the second).
-// cap: most 128-thread blocks per SM of a decapsulation front (0: the planner's).
+// cap: most 128-thread blocks per SM of a decapsulation front whose sponges take
+// one thread each; they stride over the plan's blocks, without the planner's own
+// limits (0: those).  A split front is not capped: its first launch has one block
+// per SM already (decapsulation of 20000 Saber: 362 us, capped at any of 2 to 8 in
+// one launch 384 to 451).
 constexpr size_t kWarpHashDefault = 1024, kPairHashDefault = 32768;
 struct HashCfg {
   int sms;

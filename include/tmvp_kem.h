@@ -223,11 +223,13 @@ int tmvp_ctx_set_dev_chunk(tmvp_ctx *ctx, size_t n);
  * timing (tmvp_ctx_set_timing) measures each kernel alone on the GPU.  Slower;
  * for measurement.  Results do not depend on it.  Default 0. */
 int tmvp_ctx_set_serial(tmvp_ctx *ctx, int on);
-/* Caps the Keccak front of decapsulation (GenMatrix + H(c), beside the
- * decryption) at about blocks_per_sm 64-thread blocks (half as many of 128
- * threads) resident per SM, so that decryption CTAs fit beside it on every SM;
- * 0 (the default) leaves it to the library.  0..64.  Results do not depend on
- * it. */
+/* Caps the Keccak front of decapsulation (GenMatrix + H(c), one launch beside
+ * the decryption) at blocks_per_sm 64-thread blocks per SM (launched as half as
+ * many of 128, rounded up), which then stride over the sponges, so that
+ * decryption CTAs fit beside it on every SM.  Not capped: fronts small enough
+ * to spread a sponge over several threads, and those of 128 to 192 instances per
+ * SM, which keep one 128-thread block per SM anyway.  0 (the default) leaves it to
+ * the library.  0..64.  Results do not depend on it. */
 int tmvp_ctx_set_front_cap(tmvp_ctx *ctx, int blocks_per_sm);
 /* The form of each Keccak launch (GenMatrix, GenSecret, H, G, the final key):
  * one warp per sponge, the state spread over the warp's lanes (~2.0 us per
