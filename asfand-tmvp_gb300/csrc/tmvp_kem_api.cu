@@ -75,9 +75,10 @@ struct tmvp_ctx {
   size_t dev_chunk = 32768;                        // chunk of device-input decapsulation (0: none)
   bool serial = false;                             // every stage on the caller's stream, one at a time
   int front_cap = 0;                               // Keccak-front blocks per SM (0: one thread per sponge)
-  bool hash_limits = false;                        // the caller set one of the next two (else plan_sponges chooses)
   size_t warp_hash = kWarpHashDefault;             // Keccak launches of <= this many sponges: a warp per sponge
   size_t pair_hash = kPairHashDefault;             // else of <= this many: two threads per sponge
+  // one of the two away from its default (else plan_sponges chooses)
+  bool hash_limits() const { return warp_hash != kWarpHashDefault || pair_hash != kPairHashDefault; }
   // set by the caller (tmvp_ctx_set_*): then the autotuner's per-batch choice does not apply
   bool host_chunk_set = false, host_ramp_set = false, dev_chunk_set = false, front_cap_set = false;
   int nsm = 0;                                     // SMs of the device
@@ -322,7 +323,7 @@ int run_cpa(tmvp_ctx *c, int form, int op, CpaArgs &a, cudaStream_t s) {
 // What the Keccak launches of a context may use (plan_sponges).
 inline HashCfg hash_cfg(const tmvp_ctx *c) {
   HashCfg h{c->nsm};
-  h.limits = c->hash_limits;
+  h.limits = c->hash_limits();
   h.warp_max = c->warp_hash;
   h.pair_max = c->pair_hash;
   return h;
@@ -472,7 +473,7 @@ DecScratch dec_scratch(const KemParams &P, size_t n, Arena &A) {
 // 152: 69.9 / 68.9, 450: 78 / 96; LightSaber 17: encapsulation 42.5 / 41.3, key
 // generation 36.7 / 35.3; 300: 44.7 / 49.8, 38.3 / 36.3.
 inline bool fused_tail(const tmvp_ctx *c, int form, size_t n, size_t per_sm) {
-  return resolve_form(form) == kFp8Tcgen05 && !c->hash_limits && !c->serial && n <= per_sm * (size_t)c->nsm;
+  return resolve_form(form) == kFp8Tcgen05 && !c->hash_limits() && !c->serial && n <= per_sm * (size_t)c->nsm;
 }
 
 // Whether the re-encryption of n ciphertexts under one key runs as one matrix
@@ -801,7 +802,6 @@ int tmvp_ctx_set_warp_hash(tmvp_ctx *c, size_t max_sponges) {
   if (!c) return set_err(TMVP_EINVAL);
   std::lock_guard<std::mutex> lk(c->mu);
   c->warp_hash = max_sponges;
-  c->hash_limits = true;
   return set_err(TMVP_OK);
 }
 
@@ -809,7 +809,6 @@ int tmvp_ctx_set_pair_hash(tmvp_ctx *c, size_t max_sponges) {
   if (!c) return set_err(TMVP_EINVAL);
   std::lock_guard<std::mutex> lk(c->mu);
   c->pair_hash = max_sponges;
-  c->hash_limits = true;
   return set_err(TMVP_OK);
 }
 

@@ -237,14 +237,14 @@ int tmvp_ctx_set_front_cap(tmvp_ctx *ctx, int blocks_per_sm);
  * holding half of every state lane (~2.9 us per permutation up to ~10 K
  * sponges); or one thread per sponge (~4.7 us per permutation, the best rate
  * once the GPU is full).  By default the library chooses per role of a launch
- * by its number of sponges.  Once either limit is set, launches of at most
+ * by its number of sponges, and so it does again when both limits have their
+ * initial values (1024, 32768).  With another value in either, launches of at most
  * warp_hash sponges run one warp per sponge, larger ones of at most pair_hash
  * sponges two threads, larger ones one thread; launches of short sponges (G,
  * the final key, the key-generation tail) count four times against warp_hash
- * and twice against pair_hash.  The other limit keeps its initial value (1024,
- * 32768); 0 turns a form off.  Results do not depend on them.  No counterpart
- * in the reference, whose hash kernels run as one block of one thread per
- * instance (TMVP-Saber/SABER-GPU/src/cuda_kernel.cu:116-127). */
+ * and twice against pair_hash.  0 turns a form off.  Results do not depend on
+ * them.  No counterpart in the reference, whose hash kernels run as one block of
+ * one thread per instance (TMVP-Saber/SABER-GPU/src/cuda_kernel.cu:116-127). */
 int tmvp_ctx_set_warp_hash(tmvp_ctx *ctx, size_t max_sponges);
 int tmvp_ctx_set_pair_hash(tmvp_ctx *ctx, size_t max_sponges);
 
