@@ -350,7 +350,7 @@ void plan_sponges(const HashCfg &cfg, const SpongeRole *roles, int nroles, Spong
   if (cfg.limits) {
     size_t total = 0;
     for (int r = 0; r < nroles; r++) total += roles[r].n;
-    const bool short_sponges = nroles == 1 && roles[0].perms <= 10;
+    const bool short_sponges = roles[0].brief;
     const int form = (short_sponges ? 4 * total : total) <= cfg.warp_max   ? kHashWarp
                      : (short_sponges ? 2 * total : total) <= cfg.pair_max ? kHashPair
                                                                            : kHashThread;
@@ -401,14 +401,14 @@ cudaError_t launch_dec_front(const HashCfg &cfg, const KemParams &P, const uint8
 
 cudaError_t launch_dec_g(const HashCfg &cfg, const KemParams &P, const uint8_t *mbuf, uint8_t *kr, uint8_t *s_stream,
                          size_t n, cudaStream_t s) {
-  const SpongeRole role{n, 1 + gs_perms(P)};
+  const SpongeRole role{n, 1 + gs_perms(P), 0, true};
   return launch_sponges(cfg, &role, 1, DecG{P, mbuf, kr, s_stream}, s, s);
 }
 
 cudaError_t launch_final_key(const HashCfg &cfg, const KemParams &P, const uint8_t *ct, const uint8_t *hc,
                              const uint8_t *kr, const uint8_t *fail, const uint8_t *sk, size_t sk_stride, uint8_t *ss,
                              size_t n, cudaStream_t s) {
-  const SpongeRole role{n, 1 + (hc ? 0 : sha3_256_perms(P.ct_bytes))};
+  const SpongeRole role{n, 1 + (hc ? 0 : sha3_256_perms(P.ct_bytes)), 0, true};
   return launch_sponges(cfg, &role, 1, FinalKey{P, ct, hc, kr, fail, sk, sk_stride, ss}, s, s);
 }
 
@@ -434,7 +434,7 @@ cudaError_t launch_shake_jobs(const HashCfg &cfg, const ShakeJob &j0, const Shak
 
 cudaError_t launch_kp_final(const HashCfg &cfg, const KemParams &P, const uint8_t *pk, uint8_t *sk,
                             const uint8_t *coins, size_t n, cudaStream_t s) {
-  const SpongeRole role{n, sha3_256_perms(P.pk_bytes)};
+  const SpongeRole role{n, sha3_256_perms(P.pk_bytes), 0, true};
   return launch_sponges(cfg, &role, 1, KpFinal{P, pk, sk, coins}, s, s);
 }
 
@@ -448,7 +448,7 @@ cudaError_t launch_mix_front(const HashCfg &cfg, const HashGroup *T, int ng, siz
 }
 
 cudaError_t launch_mix_g(const HashCfg &cfg, const HashGroup *T, int ng, size_t total, int perms, cudaStream_t s) {
-  const SpongeRole role{total, perms};
+  const SpongeRole role{total, perms, 0, true};
   MixG r;
   r.T = T;
   r.ng = ng;
@@ -456,7 +456,7 @@ cudaError_t launch_mix_g(const HashCfg &cfg, const HashGroup *T, int ng, size_t 
 }
 
 cudaError_t launch_mix_final(const HashCfg &cfg, const HashGroup *T, int ng, size_t total, cudaStream_t s) {
-  const SpongeRole role{total, 1};
+  const SpongeRole role{total, 1, 0, true};
   MixFinal r;
   r.T = T;
   r.ng = ng;

@@ -63,6 +63,7 @@ struct SpongeRole {
   size_t n;
   int perms;   // Keccak-f per sponge
   int id = 0;  // the stage's name for the role
+  bool brief = false;  // G, the final key, the key-generation tail: counted several times against the caller's limits
 };
 constexpr unsigned kHashBlock = 128;
 constexpr int kSpongeSmemMax = 117000;  // the most shared memory a plan asks for (one block per SM)

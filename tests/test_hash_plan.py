@@ -28,7 +28,8 @@ class Plan(ctypes.Structure):
 
 
 class Role(ctypes.Structure):
-    _fields_ = [("n", ctypes.c_size_t), ("perms", ctypes.c_int), ("id", ctypes.c_int)]
+    _fields_ = [("n", ctypes.c_size_t), ("perms", ctypes.c_int), ("id", ctypes.c_int),
+                ("brief", ctypes.c_bool)]
 
 
 @pytest.fixture(scope="module")
@@ -40,8 +41,9 @@ def plan():
     fn.restype = None
 
     def call(perms, n, **cfg):
+        brief = cfg.pop("brief", False)
         c = Cfg(sms=SMS, warp_max=cfg.pop("warp_max", 1024), pair_max=cfg.pop("pair_max", 32768), **cfg)
-        roles = (Role * len(perms))(*[Role(n, p, i) for i, p in enumerate(perms)])
+        roles = (Role * len(perms))(*[Role(n, p, i, brief) for i, p in enumerate(perms)])
         out = (Plan * 2)()
         fn(ctypes.byref(c), roles, len(perms), out)
         return out
@@ -57,3 +59,15 @@ def test_a_capped_front_holds_no_shared_memory(plan, name, n):
     main, second = plan(SETS[name], n, beside=True, cap=4)
     assert main.seg[0].form == THREAD and main.blocks > 0
     assert main.smem == 0 and second.blocks == 0
+
+
+@pytest.mark.parametrize("perms,brief,times", [((9,), False, (1, 1)), ((40,), False, (1, 1)), ((23, 9), False, (2, 2)),
+                                               ((6,), True, (4, 2)), ((1,), True, (4, 2))])
+def test_the_callers_limits_count_each_sponge_once(plan, perms, brief, times):
+    """... but those of G, the final key and the key-generation tail four times
+    against the warp limit and twice against the pair limit, whatever their length."""
+    for form, limit, k in ((WARP, 1024, times[0]), (PAIR, 32768, times[1])):
+        at, above = limit // k, limit // k + 1
+        cfg = dict(limits=True, pair_max=32768 if form == PAIR else 0)
+        assert plan(perms, at, brief=brief, **cfg)[0].seg[0].form == form
+        assert plan(perms, above, brief=brief, **cfg)[0].seg[0].form == THREAD
