@@ -302,7 +302,7 @@ static size_t thread_part(int sms, size_t n1, int p1, size_t n2, int p2) {
 }
 
 bool sponges_split(const HashCfg &cfg, size_t n) {
-  return !cfg.limits && n >= (size_t)128 * cfg.sms && n < (size_t)192 * cfg.sms;
+  return !cfg.limits && !cfg.one && n >= (size_t)128 * cfg.sms && n < (size_t)192 * cfg.sms;
 }
 
 // Why the lines lie where they do (152 SMs, 608 sub-partitions; a sponge of 23

@@ -46,6 +46,7 @@ struct HashCfg {
   int cap = 0;
   bool beside = false;  // the launch shares the GPU with others of its pass
   bool even = false;  // one role: its blocks limited to an even share per SM in every form
+  bool one = false;  // never two launches (sponges_split)
 };
 
 // A launch's sponges: role r's sponges [first, first + count) in `form`, from

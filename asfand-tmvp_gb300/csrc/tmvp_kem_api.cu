@@ -326,18 +326,29 @@ inline HashCfg hash_cfg(const tmvp_ctx *c) {
   h.limits = c->hash_limits();
   h.warp_max = c->warp_hash;
   h.pair_max = c->pair_hash;
+  h.one = c->serial;
   return h;
 }
 
+bool is_capturing(cudaStream_t s) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &st) != cudaSuccess) cudaGetLastError();  // (the launches will say so)
+  return st != cudaStreamCaptureStatusNone;
+}
+
 // A two-role Keccak launch on s, its second launch (if n splits it) on a lane
-// forked from s and joined back.
+// forked from s and joined back.  One launch where s is being captured: the lane
+// would belong to the capture until the caller ends it, and no other call of the
+// context could use it.
 template <class F>
 int forked(tmvp_ctx *c, size_t n, cudaStream_t s, F launch) {
-  if (c->serial || !sponges_split(hash_cfg(c), n)) return cuda_err(launch(s));
+  HashCfg h = hash_cfg(c);
+  if (sponges_split(h, n) && is_capturing(s)) h.one = true;
+  if (!sponges_split(h, n)) return cuda_err(launch(h, s));
   cudaStream_t s2 = c->lane[0];
   TRY_CUDA(cudaEventRecord(c->fork2_ev, s));
   TRY_CUDA(cudaStreamWaitEvent(s2, c->fork2_ev, 0));
-  TRY(cuda_err(launch(s2)));
+  TRY(cuda_err(launch(h, s2)));
   TRY_CUDA(cudaEventRecord(c->join2_ev, s2));
   TRY_CUDA(cudaStreamWaitEvent(s, c->join2_ev, 0));
   return TMVP_OK;
@@ -902,7 +913,7 @@ int tmvp_kem_keypair_batch(tmvp_ctx *c, tmvp_param_set set, size_t n, uint8_t *p
   ShakeJob j1{bco.dev, 96, 32, s_stream, (size_t)P.gs_bytes, P.gs_bytes, 0, nullptr, 0, 0};
   {
     StageTimer tm_(c, "shake_jobs", s);
-    if ((r = forked(c, n, s, [&](cudaStream_t s2) { return launch_shake_jobs(hash_cfg(c), j0, j1, n, s, s2); })))
+    if ((r = forked(c, n, s, [&](const HashCfg &h, cudaStream_t s2) { return launch_shake_jobs(h, j0, j1, n, s, s2); })))
       return set_err(r);
   }
   c->launches++;
@@ -957,10 +968,10 @@ int enc_batch(tmvp_ctx *c, tmvp_param_set set, size_t n, uint8_t *ct, uint8_t *s
   if ((r = upload(bpk, s)) || (r = upload(bco, s))) return set_err(r);
   {
     StageTimer tm_(c, "enc_front", s);
-    auto launch = [&](cudaStream_t s2) {
-      return launch_enc_front(hash_cfg(c), P, bpk.dev, bco.dev, mbuf, kr, s_stream, a_stream, n, !a_cached, s, s2);
+    auto launch = [&](const HashCfg &h, cudaStream_t s2) {
+      return launch_enc_front(h, P, bpk.dev, bco.dev, mbuf, kr, s_stream, a_stream, n, !a_cached, s, s2);
     };
-    if ((r = a_cached ? cuda_err(launch(s)) : forked(c, n, s, launch))) return set_err(r);
+    if ((r = a_cached ? cuda_err(launch(hash_cfg(c), s)) : forked(c, n, s, launch))) return set_err(r);
   }
   c->launches++;
   CpaArgs a{};
@@ -1349,7 +1360,7 @@ int tmvp_indcpa_keypair_batch(tmvp_ctx *c, tmvp_param_set set, size_t n, uint8_t
   ShakeJob j1{bse.dev, 64, 32, s_stream, (size_t)P.gs_bytes, P.gs_bytes, 0, nullptr, 0, 0};
   {
     StageTimer tm_(c, "shake_jobs", s);
-    if ((r = forked(c, n, s, [&](cudaStream_t s2) { return launch_shake_jobs(hash_cfg(c), j0, j1, n, s, s2); })))
+    if ((r = forked(c, n, s, [&](const HashCfg &h, cudaStream_t s2) { return launch_shake_jobs(h, j0, j1, n, s, s2); })))
       return set_err(r);
   }
   c->launches++;
@@ -1397,7 +1408,7 @@ int tmvp_indcpa_enc_batch(tmvp_ctx *c, tmvp_param_set set, size_t n, uint8_t *ct
               (size_t)P.gm_bytes, P.gm_bytes, 0, nullptr, 0, 0};
   {
     StageTimer tm_(c, "shake_jobs", s);
-    if ((r = forked(c, n, s, [&](cudaStream_t s2) { return launch_shake_jobs(hash_cfg(c), j0, j1, n, s, s2); })))
+    if ((r = forked(c, n, s, [&](const HashCfg &h, cudaStream_t s2) { return launch_shake_jobs(h, j0, j1, n, s, s2); })))
       return set_err(r);
   }
   c->launches++;

@@ -14,7 +14,7 @@ SETS = {"lightsaber": (10, 6), "saber": (23, 9), "firesaber": (40, 11), "lightsa
 class Cfg(ctypes.Structure):
     _fields_ = [("sms", ctypes.c_int), ("limits", ctypes.c_bool), ("warp_max", ctypes.c_size_t),
                 ("pair_max", ctypes.c_size_t), ("cap", ctypes.c_int), ("beside", ctypes.c_bool),
-                ("even", ctypes.c_bool)]
+                ("even", ctypes.c_bool), ("one", ctypes.c_bool)]
 
 
 class Seg(ctypes.Structure):
