@@ -25,6 +25,7 @@
 #include <functional>
 #include <map>
 #include <mutex>
+#include <optional>
 #include <string>
 #include <utility>
 #include <vector>
@@ -336,19 +337,27 @@ bool is_capturing(cudaStream_t s) {
   return st != cudaStreamCaptureStatusNone;
 }
 
-// A two-role Keccak launch on s, its second launch (if n splits it) on a lane
+// A two-role Keccak stage on s, its second launch (if n splits it) on a lane
 // forked from s and joined back.  One launch where s is being captured: the lane
 // would belong to the capture until the caller ends it, and no other call of the
 // context could use it.
 template <class F>
-int forked(tmvp_ctx *c, size_t n, cudaStream_t s, F launch) {
+int forked(tmvp_ctx *c, const char *stage, size_t n, cudaStream_t s, F launch) {
   HashCfg h = hash_cfg(c);
   if (sponges_split(h, n) && is_capturing(s)) h.one = true;
-  if (!sponges_split(h, n)) return cuda_err(launch(h, s));
+  if (!sponges_split(h, n)) {
+    StageTimer tm_(c, stage, s);
+    c->launches++;
+    return cuda_err(launch(h, s));
+  }
   cudaStream_t s2 = c->lane[0];
   TRY_CUDA(cudaEventRecord(c->fork2_ev, s));
   TRY_CUDA(cudaStreamWaitEvent(s2, c->fork2_ev, 0));
-  TRY(cuda_err(launch(h, s2)));
+  {
+    StageTimer tm_(c, stage, s), tm2_(c, stage, s2);
+    TRY(cuda_err(launch(h, s2)));
+  }
+  c->launches += 2;
   TRY_CUDA(cudaEventRecord(c->join2_ev, s2));
   TRY_CUDA(cudaStreamWaitEvent(s, c->join2_ev, 0));
   return TMVP_OK;
@@ -541,12 +550,14 @@ int dec_pipeline(tmvp_ctx *c, const KemParams &P, size_t n, uint8_t *ss, const u
   }
   {
     StageTimer tm_(c, "dec_front", side);
+    std::optional<StageTimer> tm2_;
+    if (split) tm2_.emplace(c, "dec_front", side2);
     TRY_CUDA(launch_dec_front(h, P, sk, ct, w.a_stream, w.hc, n, !a_cached, side, side2));
   }
   if (matrix) TRY_CUDA(cudaMemsetAsync(w.fail, 0, n, side));
   TRY_CUDA(cudaEventRecord(c->join_ev, side));
   if (split) TRY_CUDA(cudaEventRecord(c->join2_ev, side2));
-  c->launches++;
+  c->launches += split ? 2 : 1;
   CpaArgs a{};
   a.P = P;
   a.n = (int)n;
@@ -911,12 +922,9 @@ int tmvp_kem_keypair_batch(tmvp_ctx *c, tmvp_param_set set, size_t n, uint8_t *p
   ShakeJob j0{bco.dev, 96, 0, a_stream, (size_t)P.gm_bytes, P.gm_bytes, 1, bpk.dev,
               (size_t)P.pk_bytes, (size_t)P.l * P.polycompbytes};
   ShakeJob j1{bco.dev, 96, 32, s_stream, (size_t)P.gs_bytes, P.gs_bytes, 0, nullptr, 0, 0};
-  {
-    StageTimer tm_(c, "shake_jobs", s);
-    if ((r = forked(c, n, s, [&](const HashCfg &h, cudaStream_t s2) { return launch_shake_jobs(h, j0, j1, n, s, s2); })))
-      return set_err(r);
-  }
-  c->launches++;
+  if ((r = forked(c, "shake_jobs", n, s,
+                  [&](const HashCfg &h, cudaStream_t s2) { return launch_shake_jobs(h, j0, j1, n, s, s2); })))
+    return set_err(r);
   CpaArgs a{};
   a.P = P;
   a.n = (int)n;
@@ -966,14 +974,16 @@ int enc_batch(tmvp_ctx *c, tmvp_param_set set, size_t n, uint8_t *ct, uint8_t *s
   stage_assign(bpk, A);
   stage_assign(bco, A);
   if ((r = upload(bpk, s)) || (r = upload(bco, s))) return set_err(r);
-  {
+  auto front = [&](const HashCfg &h, cudaStream_t s2) {
+    return launch_enc_front(h, P, bpk.dev, bco.dev, mbuf, kr, s_stream, a_stream, n, !a_cached, s, s2);
+  };
+  if (a_cached) {  // (one role)
     StageTimer tm_(c, "enc_front", s);
-    auto launch = [&](const HashCfg &h, cudaStream_t s2) {
-      return launch_enc_front(h, P, bpk.dev, bco.dev, mbuf, kr, s_stream, a_stream, n, !a_cached, s, s2);
-    };
-    if ((r = a_cached ? cuda_err(launch(hash_cfg(c), s)) : forked(c, n, s, launch))) return set_err(r);
+    if ((r = cuda_err(front(hash_cfg(c), s)))) return set_err(r);
+    c->launches++;
+  } else if ((r = forked(c, "enc_front", n, s, front))) {
+    return set_err(r);
   }
-  c->launches++;
   CpaArgs a{};
   a.P = P;
   a.n = (int)n;
@@ -1358,12 +1368,9 @@ int tmvp_indcpa_keypair_batch(tmvp_ctx *c, tmvp_param_set set, size_t n, uint8_t
   ShakeJob j0{bse.dev, 64, 0, a_stream, (size_t)P.gm_bytes, P.gm_bytes, 1, bpk.dev,
               (size_t)P.pk_bytes, (size_t)P.l * P.polycompbytes};
   ShakeJob j1{bse.dev, 64, 32, s_stream, (size_t)P.gs_bytes, P.gs_bytes, 0, nullptr, 0, 0};
-  {
-    StageTimer tm_(c, "shake_jobs", s);
-    if ((r = forked(c, n, s, [&](const HashCfg &h, cudaStream_t s2) { return launch_shake_jobs(h, j0, j1, n, s, s2); })))
-      return set_err(r);
-  }
-  c->launches++;
+  if ((r = forked(c, "shake_jobs", n, s,
+                  [&](const HashCfg &h, cudaStream_t s2) { return launch_shake_jobs(h, j0, j1, n, s, s2); })))
+    return set_err(r);
   CpaArgs a{};
   a.P = P;
   a.n = (int)n;
@@ -1406,12 +1413,9 @@ int tmvp_indcpa_enc_batch(tmvp_ctx *c, tmvp_param_set set, size_t n, uint8_t *ct
   ShakeJob j0{bns.dev, 32, 0, s_stream, (size_t)P.gs_bytes, P.gs_bytes, 0, nullptr, 0, 0};
   ShakeJob j1{bpk.dev, (size_t)P.pk_bytes, (size_t)P.l * P.polycompbytes, a_stream,
               (size_t)P.gm_bytes, P.gm_bytes, 0, nullptr, 0, 0};
-  {
-    StageTimer tm_(c, "shake_jobs", s);
-    if ((r = forked(c, n, s, [&](const HashCfg &h, cudaStream_t s2) { return launch_shake_jobs(h, j0, j1, n, s, s2); })))
-      return set_err(r);
-  }
-  c->launches++;
+  if ((r = forked(c, "shake_jobs", n, s,
+                  [&](const HashCfg &h, cudaStream_t s2) { return launch_shake_jobs(h, j0, j1, n, s, s2); })))
+    return set_err(r);
   CpaArgs a{};
   a.P = P;
   a.n = (int)n;
@@ -1802,6 +1806,8 @@ int mixed_enqueue(tmvp_ctx *c, size_t ng, const tmvp_dec_group *gr, uint8_t *ws,
   // GenMatrix and H(c) of every group in one launch (2 total sponges)
   {
     StageTimer tm_(c, "mix_front", ms.side);
+    std::optional<StageTimer> tm2_;
+    if (split) tm2_.emplace(c, "mix_front", ms.side2);
     TRY_CUDA(launch_mix_front(hash_cfg(c), th, (int)ng, (size_t)total, gm, hp, ms.side, split ? ms.side2 : ms.side));
   }
   TRY_CUDA(cudaEventRecord(c->join_ev, ms.side));
@@ -1848,7 +1854,7 @@ int mixed_enqueue(tmvp_ctx *c, size_t ng, const tmvp_dec_group *gr, uint8_t *ws,
     StageTimer tm_(c, "mix_final", s);
     TRY_CUDA(launch_mix_final(hash_cfg(c), th, (int)ng, (size_t)total, s));
   }
-  c->launches += 3 + 2 * nsets;
+  if (total) c->launches += 3 + split + 2 * nsets;
   TRY_CUDA(cudaGetLastError());
   return TMVP_OK;
 }
