@@ -38,3 +38,46 @@ def test_groups_end_inside_a_warp(kem, oracle, total):
     ctx.sync_status()
     for (set_id, out, _, _), w in zip(groups, want):
         assert np.array_equal(out.cpu().numpy(), w), set_id
+
+
+def _pass_and_batches(T, ctx, groups, seed):
+    """A mixed pass over (set, count) groups, made on the GPU, and each group as a batch."""
+    import torch
+    made, ref = [], T.Context(0)
+    for i, (set_id, n) in enumerate(groups):
+        z = T.sizes(set_id)
+        new = lambda w: torch.zeros((n, w), dtype=torch.uint8, device="cuda")
+        pk, sk, ct, ss, out, want = (new(w) for w in (z.pk_bytes, z.sk_bytes, z.ct_bytes, 32, 32, 32))
+        ref.kem_keypair_ptr(set_id, n, pk, sk, torch.from_numpy(T.splitmix_bytes(seed + 2 * i, n * 96)).cuda())
+        ref.kem_enc_ptr(set_id, n, ct, ss, pk, torch.from_numpy(T.splitmix_bytes(seed + 2 * i + 1, n * 32)).cuda())
+        ct[::3, 9] ^= 0x08
+        ref.kem_dec_ptr(set_id, n, want, ct, sk)
+        ref.sync_status()
+        made.append((set_id, out, ct, sk, want))
+    torch.cuda.synchronize()
+    ctx.kem_dec_mixed([m[:4] for m in made])
+    ctx.sync_status()
+    for set_id, out, _, _, want in made:
+        assert torch.equal(out, want), set_id
+    ref.close()
+
+
+@pytest.mark.parametrize("total", [32 * PARTS + 5000, 48 * PARTS + 3, 2 * 32 * PARTS + 9001, 4 * 32 * PARTS + 777])
+def test_large_passes_match_batches(kem, total):
+    """A split front, a round and a rest, and two chains of each."""
+    T, ctx = kem
+    rest = total - sum(n for _, n in SMALL)
+    big = [(s, rest // 6 + (3, -1, 5, -7, 2, 0)[s]) for s in range(5)]
+    big.append((5, rest - sum(n for _, n in big)))
+    _pass_and_batches(T, ctx, SMALL + big, 12000)
+
+
+@pytest.mark.parametrize("warp,pair", [(1 << 40, 0), (0, 1 << 40), (0, 0), (500, 3000)])
+def test_passes_under_the_callers_limits(kem, warp, pair):
+    T, _ = kem
+    ctx = T.Context(0)
+    ctx.set_warp_hash(warp)
+    ctx.set_pair_hash(pair)
+    for big in ([], [(1, 701), (4, 1203), (0, 998)]):
+        _pass_and_batches(T, ctx, SMALL + big, 12100)
+    ctx.close()

@@ -6,6 +6,7 @@ import pytest
 SMS = 152
 THREAD, WARP, PAIR = 0, 1, 2
 PER_BLOCK = {THREAD: 128, WARP: 4, PAIR: 64}
+W = 4 * SMS  # sub-partitions
 # GenMatrix and H(c) permutations of the six sets, in the library's order
 SETS = {"lightsaber": (10, 6), "saber": (23, 9), "firesaber": (40, 11), "lightsable": (9, 5), "sable": (19, 8),
         "firesable": (34, 11)}
@@ -59,6 +60,39 @@ def test_a_capped_front_holds_no_shared_memory(plan, name, n):
     main, second = plan(SETS[name], n, beside=True, cap=4)
     assert main.seg[0].form == THREAD and main.blocks > 0
     assert main.smem == 0 and second.blocks == 0
+
+
+# permutations of every two-role stage: decapsulation front, encapsulation front, key generation
+GS, HPK = (4, 5, 5, 1, 2, 2), (5, 8, 10, 5, 7, 10)
+STAGES = ([(gm, h) for gm, h in SETS.values()] +
+          [(gm, 2 + hp + gs) for (gm, _), gs, hp in zip(SETS.values(), GS, HPK)] +
+          [(gm + 1, gs) for (gm, _), gs in zip(SETS.values(), GS)])
+LINES = [W, 3 * W // 2, 2 * W, 9 * W // 4, 11 * W // 4, 11 * W // 8, 9 * W // 8, 16 * W, 24 * W, 32 * W, 48 * W]
+COUNTS = sorted({1, 2, 31, 33} | {n + d for n in LINES for d in (-1, 0, 1)} |
+                {r * 32 * W + d for r in (1, 2, 3, 5, 6) for d in (-1, 0, 1, 700, 16 * W + 1, 20 * W, 17 * W)} |
+                {9800, 12500, 14001, 16384, 20011, 65536, 1 << 20})
+
+
+@pytest.mark.parametrize("perms", sorted(set(STAGES)) + [(1,), (3,), (10,), (40,)])
+@pytest.mark.parametrize("cfg", [{}, {"beside": True}, {"beside": True, "even": True}, {"beside": True, "cap": 3},
+                                 {"one": True}, {"limits": True, "warp_max": 0}, {"limits": True, "pair_max": 0}])
+def test_a_plan_takes_every_sponge_once(plan, perms, cfg):
+    for n in COUNTS:
+        both = plan(perms, n, **cfg)
+        split = len(perms) == 2 and not cfg.get("limits") and not cfg.get("one") and 128 * SMS <= n < 192 * SMS
+        assert (both[1].blocks > 0) == split
+        taken = [[] for _ in perms]
+        for p in both:
+            blocks = 0
+            for s in p.seg[:p.nseg]:
+                assert s.block0 == blocks and s.count > 0
+                blocks += -(-s.count // PER_BLOCK[s.form])
+                taken[s.role].append((s.first, s.first + s.count))
+            assert p.blocks == blocks and p.smem <= 117000 and p.nseg <= 8
+        for t in taken:
+            t.sort()
+            assert t[0][0] == 0 and t[-1][1] == n
+            assert all(a[1] == b[0] for a, b in zip(t, t[1:]))
 
 
 @pytest.mark.parametrize("perms,brief,times", [((9,), False, (1, 1)), ((40,), False, (1, 1)), ((23, 9), False, (2, 2)),
