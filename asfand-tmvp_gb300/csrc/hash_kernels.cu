@@ -316,6 +316,10 @@ bool sponges_split(const HashCfg &cfg, size_t n) {
 //    two threads a sponge 67 us up to 16, one thread 109 us up to 32: the
 //    forms' lines.  Past whole rounds of 32, the rest goes the same way beside
 //    them: 20011 sponges in 122 us instead of 206.
+//    Beside one round of a single role the warp form pays below one sponge a
+//    sub-partition, beside two up to two: GenMatrix of 19456 + 600 Saber keys 145
+//    us (rest in pairs 167), + 700 240 (167), of 38912 + 1216 258 (265), + 1300 291
+//    (264), of three rounds + 1300 363 (362).
 //    A one-role launch that shares the GPU (G, H(c) alone) leaves the warp form,
 //    which issues five times the instructions, at 1.5: decapsulation of 1000
 //    Saber 83 -> 77 us, of 1600 107 -> 91, of 1200 FireSaber 144 -> 134, of 1600
@@ -365,7 +369,9 @@ void plan_sponges(const HashCfg &cfg, const SpongeRole *roles, int nroles, Spong
     const size_t full = r.n / (32 * W) * (32 * W), rest = r.n - full;
     int form = kHashThread;
     const bool slack = cfg.beside && k == 1 && 5 * r.perms <= 3 * roles[order[0]].perms;  // ends first in either form
-    const size_t line = full ? 9 * W / 4 : (slack ? 2 * W : (cfg.beside && nroles == 1 ? 3 * W / 2 : 11 * W / 4));
+    const size_t rounds = full / (32 * W);
+    const size_t above = nroles == 2 || rounds > 2 ? 9 * W / 4 : (rounds == 2 ? 2 * W : W - 1);
+    const size_t line = full ? above : (slack ? 2 * W : (cfg.beside && nroles == 1 ? 3 * W / 2 : 11 * W / 4));
     if (warps + rest <= line) form = kHashWarp;
     else if (rest <= 16 * W) form = kHashPair;
     if (form == kHashWarp) warps += rest;
@@ -377,7 +383,7 @@ void plan_sponges(const HashCfg &cfg, const SpongeRole *roles, int nroles, Spong
     add_seg(S[split && k == 1], r.id, kHashPair, full + fit, rest - fit);
     if (nroles == 1) {
       // blocks per SM when every SM has its share
-      const int q = (int)(full / (32 * W)) + (form == kHashThread && rest ? 1 : 0);
+      const int q = (int)rounds + (form == kHashThread && rest ? 1 : 0);
       if (r.perms >= 4 && q <= 5 && (form == kHashThread || rest == 0 || q >= 2)) S[0].smem = smem_limit(q);
       else if (cfg.even) S[0].smem = smem_limit((int)((S[0].blocks + cfg.sms - 1) / cfg.sms));
     }

@@ -105,3 +105,13 @@ def test_the_callers_limits_count_each_sponge_once(plan, perms, brief, times):
         cfg = dict(limits=True, pair_max=32768 if form == PAIR else 0)
         assert plan(perms, at, brief=brief, **cfg)[0].seg[0].form == form
         assert plan(perms, above, brief=brief, **cfg)[0].seg[0].form == THREAD
+
+
+@pytest.mark.parametrize("perms", [9, 23, 40])
+@pytest.mark.parametrize("rounds,most", [(1, W - 1), (2, 2 * W), (3, 9 * W // 4)])
+def test_the_rest_of_one_role_leaves_the_warp_form_early(plan, perms, rounds, most):
+    """Beside one or two rounds more sponges than that take longer in the warp
+    form than in pairs, and longer than no plan at all."""
+    for rest, form in ((most, WARP), (most + 1, PAIR)):
+        p = plan((perms,), rounds * 32 * W + rest)[0]
+        assert [s.form for s in p.seg[:p.nseg]] == [THREAD, form]
