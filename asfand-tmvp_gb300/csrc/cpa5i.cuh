@@ -539,7 +539,7 @@ __device__ __forceinline__ void cpa5i_run(const AT &at, uint8_t *sm) {
     mbar_expect_tx(mbar_clc, 16);
     clc_try_cancel(clc_resp + 16 * par, mbar_clc);
   }
-  bool ready = mbar_wait_warp(mbar_in, par);
+  bool ready = __all_sync(0xffffffffu, mbar_wait_bounded(mbar_in, par)) != 0;  // (a warp's lanes agree: shuffles follow)
   if (ready) {
     // 1. digit columns (K reversed, core-matrix order): lane g converts
     // coefficients 8g..8g+7 (K rows k' = 8kq+7..8kq, kq = 31 - g) of one
