@@ -6,7 +6,7 @@
 //   out[ciphertext][(p, n)] = sum_(j, k) s_j[ciphertext][k] M[(j, k)][(p, n)]
 // with M the negacyclic Toeplitz matrices of the public polynomials.  The
 // per-instance kernel (cpa5i.cuh) spends 12 MMAs of N = 48, its Hankel and
-// digit stagings and its phase barriers on each ciphertext (268 us for 65536
+// digit stagings and its phase barriers on each ciphertext (262 us for 65536
 // Saber ones); here 264 MMAs of N = 256 serve 128 ciphertexts.
 //
 //   * A (M side): the CBD secrets of 128 ciphertexts as raw e4m3 bytes (worth

@@ -75,7 +75,7 @@ struct tmvp_ctx {
   int host_ramp = 1;                               // first chunks host_chunk >> ramp, >> ramp-1, ...
   size_t dev_chunk = 32768;                        // chunk of device-input decapsulation (0: none)
   bool serial = false;                             // every stage on the caller's stream, one at a time
-  int front_cap = 0;                               // Keccak-front blocks per SM (0: one thread per sponge)
+  int front_cap = 0;                               // Keccak-front blocks of 64 threads per SM (0: the planner's)
   size_t warp_hash = kWarpHashDefault;             // Keccak launches of <= this many sponges: a warp per sponge
   size_t pair_hash = kPairHashDefault;             // else of <= this many: two threads per sponge
   // one of the two away from its default (else plan_sponges chooses)
@@ -1213,11 +1213,12 @@ int tmvp_kem_dec_batch(tmvp_ctx *c, tmvp_param_set set, size_t n, uint8_t *ss, c
     // host inputs: chunk k's copies (one copy stream, five input slots) run
     // ahead of the kernels, and chunk k's chain runs on lane k mod 4 (as in
     // dec_lanes, each lane with its own scratch and Keccak-front stream), so
-    // consecutive chunks' chains overlap.  The kernels are slower than the
-    // host link, so the call lasts about (first chunk's copy) + (the kernels
-    // of the whole batch): the first host_ramp chunks are host_chunk >>
-    // host_ramp, >> host_ramp - 1, ..., which starts the kernels early while
-    // later chunks stay large enough to fill the GPU.
+    // consecutive chunks' chains overlap.  The host link (62 K Saber instances
+    // per ms) and the kernels (65 K) are about equally fast, so the call lasts
+    // about the copies, the first chunk's before any kernel, and the last
+    // chunk's chain: the first host_ramp chunks are host_chunk >> host_ramp,
+    // >> host_ramp - 1, ..., which starts the kernels early while later chunks
+    // stay large enough to fill the GPU.
     constexpr int NL = tmvp_ctx::kLanes, NS = tmvp_ctx::kSlots;
     const size_t cn = c->host_chunk;
     const size_t inb = up(cn * P.ct_bytes) + up(cn * P.sk_bytes);

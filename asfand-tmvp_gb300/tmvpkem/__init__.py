@@ -418,11 +418,12 @@ class Context:
         _check(lib().tmvp_ctx_set_serial(self.h, int(bool(on))), "tmvp_ctx_set_serial")
 
     def set_front_cap(self, blocks_per_sm: int):
-        """Keccak-front blocks per SM in decapsulation (0 = one thread per sponge)."""
+        """Keccak-front blocks of 64 threads per SM in decapsulation (0: the library chooses)."""
         _check(lib().tmvp_ctx_set_front_cap(self.h, blocks_per_sm), "tmvp_ctx_set_front_cap")
 
     def set_warp_hash(self, max_sponges: int):
-        """Keccak launches of at most max_sponges sponges run one warp per sponge (0: never)."""
+        """Keccak launches of at most max_sponges sponges run one warp per sponge (0: never).
+        With 1024 here and 32768 in set_pair_hash, the initial values, the library chooses."""
         _check(lib().tmvp_ctx_set_warp_hash(self.h, max_sponges), "tmvp_ctx_set_warp_hash")
 
     def set_pair_hash(self, max_sponges: int):

@@ -57,9 +57,9 @@ CT_BYTES, SK_BYTES, PK_BYTES = 1088, 2304, 992
 # schoolbook-equivalent work of one negacyclic 256 x 256 product
 POLY_OPS = 2 * 256 * 256
 # SM cycles per tcgen05.mma kind::f8f6f4 with M = 128, K = 32 when 4 CTAs per SM issue back to
-# back: 38.8 at N = 16, 39.8 at 32 and 48 at 64 (measured on GB300 by the mma_rates workload; N = 256
-# takes 128); about the 4 KB + 32 N bytes of its operands at 128 bytes a cycle, so 44 at N = 48
-MMA_CYCLES_N48 = 44.0
+# back, measured on GB300: 38.8 at N = 16, 39.8 at 32, 47.8 at 64, 127.8 at 256 (the mma_rates
+# workload), and 43.8 at 48 (the same diagnostic with 64 tensor-memory columns for N = 48)
+MMA_CYCLES_N48 = 43.8
 MMA_CYCLES_N16 = 38.8
 # tcgen05.mma per Saber instance: 3 secret polynomials x 4 Hankel tiles, each against four K steps
 # (N = 4 x 12 digit columns for the re-encryption, 4 x 4 for the decryption)

@@ -398,11 +398,12 @@ int tmvp_diag_keccak_rate(tmvp_ctx *ctx, int perms, double *out);
  *
  * Up to 64 groups (at most 2^30 instances in all), each with its own
  * parameter set (any of the six) and its own device buffers (16-byte aligned,
- * this context's GPU), decapsulate in one pass: every stage is ONE launch over
- * all groups -- GenMatrix, H(c), G and the final key as Keccak kernels, the two
- * IND-CPA steps on the tcgen05 tensor cores (one CTA per instance, or the
- * persistent pipelined kernel where the autotuner chose it for every set in
- * the pass).  tmvp_mixed_plan_create
+ * this context's GPU), decapsulate in one pass: the Keccak stages (GenMatrix with
+ * H(c), G, the final key) are launches over all groups, the two IND-CPA steps on
+ * the tcgen05 tensor cores one launch per parameter set present (one CTA per
+ * instance, or the persistent pipelined kernel where the autotuner chose it for
+ * that set).  Passes above the device chunk run as two such chains.
+ * tmvp_mixed_plan_create
  * captures the pass for fixed buffers into a CUDA graph (the plan owns its
  * workspace); tmvp_mixed_plan_launch replays it, so the caller refills the
  * ciphertext / key buffers and relaunches.  Asynchronous on `stream`; use
