@@ -49,3 +49,33 @@ def test_other_calls_during_a_capture(kem, oracle):
     wct, wss = oracle.kem_enc_batch(S, wpk, ec, threads)
     for got, want in ((pk, wpk), (sk, wsk), (ct, wct), (ss, wss)):
         assert np.array_equal(got.cpu().numpy(), want)
+
+
+def test_captured_decapsulation_and_mixed_plan(kem):
+    """Decapsulation and a mixed plan of such a batch keep their two launches in a graph."""
+    import torch
+    T, _ = kem
+    S = T.LIGHTSABER
+    z = T.sizes(S)
+    new = lambda w: torch.zeros((N, w), dtype=torch.uint8, device="cuda")
+    pk, sk, ct, ss, out, mix = (new(w) for w in (z.pk_bytes, z.sk_bytes, z.ct_bytes, 32, 32, 32))
+    ctx = T.Context(0)
+    ctx.kem_keypair_ptr(S, N, pk, sk, torch.from_numpy(T.splitmix_bytes(9955, N * 96)).cuda())
+    ctx.kem_enc_ptr(S, N, ct, ss, pk, torch.from_numpy(T.splitmix_bytes(9956, N * 32)).cuda())
+    ctx.kem_dec_ptr(S, N, out, ct, sk)
+    ctx.sync_status()
+    out.zero_()
+    torch.cuda.synchronize()
+    st = torch.cuda.Stream()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=st):
+        ctx.kem_dec_ptr(S, N, out, ct, sk, stream=st.cuda_stream)
+    plan = T.MixedPlan(ctx, [(S, mix[:N // 2], ct[:N // 2], sk[:N // 2]), (S, mix[N // 2:], ct[N // 2:], sk[N // 2:])])
+    for _ in range(2):
+        g.replay()
+        plan.launch()
+    ctx.sync_status()
+    torch.cuda.synchronize()
+    assert torch.equal(out, ss) and torch.equal(mix, ss)
+    plan.close()
+    ctx.close()
